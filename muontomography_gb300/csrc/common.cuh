@@ -343,35 +343,36 @@ void launch_em_voxel(const VoxelPassArgs<Real, OutT>& a, const VoxDesc* const* l
                      const int* resident_blocks, uint32_t streamed, int num_sms, const ClassFan* fan,
                      cudaStream_t s);
 // Bricked voxel order for the muon passes' lambda gathers and the per-voxel
-// sums: 4x4x4 bricks of 64 consecutive entries, each brick made of eight
-// 2x2x2 micro-blocks of 8 entries (one 32-byte sector in FP32), so the
-// consecutive voxels of a muon's path, which differ by one step on one
-// axis, fall into the same sector about half the time instead of lying a
-// grid row or plane apart.
+// sums: 4x4x8 bricks of 128 consecutive entries, made of 2x2x8 lines of 32
+// entries (128 bytes in FP32, one L2 request), each of four 2x1x4 sectors of 8
+// (32 bytes).  Muons are steep: a path of 221 voxels on a 128-layer grid takes
+// 128 steps in z and 93 in x and y, so sectors and lines are longest in z.  A
+// warp instruction over 32 consecutive pairs of a path then touches 10.2 lines
+// and 15.9 sectors; with 4x4x2 lines of 2x2x2 sectors it was 12.8 and 16.5
+// (counted by ncu on the reductions of the 256 x 256 x 128 grid).
 struct BrickDims {
     uint32_t nx, ny, nz, nbx, nby, nbz;
 };
 __host__ __device__ inline BrickDims brick_dims(const muto_grid& g) {
-    return BrickDims{g.nx, g.ny, g.nz, (g.nx + 3) / 4, (g.ny + 3) / 4, (g.nz + 3) / 4};
+    return BrickDims{g.nx, g.ny, g.nz, (g.nx + 3) / 4, (g.ny + 3) / 4, (g.nz + 7) / 8};
 }
 __host__ __device__ inline uint64_t brick_volume(const BrickDims& b) {
-    return static_cast<uint64_t>(b.nbx) * b.nby * b.nbz * 64;
+    return static_cast<uint64_t>(b.nbx) * b.nby * b.nbz * 128;
 }
 __host__ __device__ inline uint32_t brick_xyz(uint32_t x, uint32_t y, uint32_t z, const BrickDims& b) {
-    const uint32_t in = (((z >> 1) & 1u) << 5) | (((y >> 1) & 1u) << 4) | (((x >> 1) & 1u) << 3) | ((z & 1u) << 2) |
-                        ((y & 1u) << 1) | (x & 1u);
-    return (((z >> 2) * b.nby + (y >> 2)) * b.nbx + (x >> 2)) * 64u + in;
+    const uint32_t in = (x & 1u) | ((z & 3u) << 1) | ((y & 1u) << 3) | ((z & 4u) << 2) | ((x & 2u) << 4) | ((y & 2u) << 5);
+    return (((z >> 3) * b.nby + (y >> 2)) * b.nbx + (x >> 2)) * 128u + in;
 }
 __host__ __device__ inline uint32_t brick_of(uint32_t j, const BrickDims& b) {
     const uint32_t x = j % b.nx, t = j / b.nx, y = t % b.ny, z = t / b.ny;
     return brick_xyz(x, y, z, b);
 }
 __host__ __device__ inline uint32_t unbrick(uint32_t jb, const BrickDims& b) {
-    const uint32_t in = jb & 63u, blk = jb >> 6;
+    const uint32_t in = jb & 127u, blk = jb >> 7;
     const uint32_t bx = blk % b.nbx, t = blk / b.nbx, by = t % b.nby, bz = t / b.nby;
-    const uint32_t x = bx * 4 + (((in >> 3) & 1u) << 1) + (in & 1u);
-    const uint32_t y = by * 4 + (((in >> 4) & 1u) << 1) + ((in >> 1) & 1u);
-    const uint32_t z = bz * 4 + (((in >> 5) & 1u) << 1) + ((in >> 2) & 1u);
+    const uint32_t x = bx * 4 + ((in & 1u) | ((in >> 4) & 2u));
+    const uint32_t y = by * 4 + (((in >> 3) & 1u) | ((in >> 5) & 2u));
+    const uint32_t z = bz * 8 + (((in >> 1) & 3u) | ((in >> 2) & 4u));
     return x + b.nx * (y + b.ny * z);
 }
 // voxel indices to bricked ones in place (indices >= V are left alone)
