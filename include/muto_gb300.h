@@ -77,7 +77,8 @@ typedef struct muto_status {
     int32_t tile_pairs;         /* pairs per tile (TMA variant), pairs per muon held in registers
                                    (fused stored-list pass), pairs staged per batch (staged pass),
                                    pairs in flight per lane (split form's scatter); 0 otherwise */
-    int32_t tile_muons;         /* muons per tile (TMA variant), muons per CTA batch (fused pass),
+    int32_t tile_muons;         /* muons per tile (TMA variant), muons per CTA batch (fused pass) or
+                                   per warp (its mixed "auto" form),
                                    chunks of muons whose muon pass and scatter overlap (split form;
                                    0: not overlapped) */
     int32_t path_lists;         /* how the pairs are kept: 1 muon-major lists and their voxel-major copy,
@@ -131,9 +132,11 @@ typedef struct muto_handle muto_handle;
  * (update_with_mean true, mean_percentile 100), else "voxel_major";
  * "muon_major" and "recompute" require the mean update),
  * "fused_variant" ("auto": the mean update's pass over muon-major lists
- * takes the lanes per muon and pairs held per lane by timing the variants
- * that suit the scan's mean path and the split form (the muon pass, then a
- * second pass over the lists adding the terms) at prepare; "4x8", "8x4",
+ * is, in the mixed form, the one-pass kernel without block barriers, its
+ * lanes per muon by the scan's mean path; in fp64 it takes the lanes per
+ * muon and pairs held per lane by timing the variants that suit the mean
+ * path and the split form (the muon pass, then a second pass over the lists
+ * adding the terms) at prepare; "4x8", "8x4",
  * "8x8", "8x16", "16x8", "16x16", "split", "split8" (its scatter with 8
  * pairs in flight per lane), "split8_overlap" (the same, the scatter of one
  * chunk of muons running beside the muon pass of the next) or "staged"

@@ -11,6 +11,9 @@
 // needed: every muon adds its g_ij to G_j with a reduction to global memory
 // (G is L2-resident), and a small voxel kernel finishes the update.
 //
+// One-pass form of the mixed precision (k_em_once, below): what "auto" runs
+// there.  The forms that follow serve FP64 and the forced variants.
+//
 // Stored-list pass (k_em_fused_lists).  A CTA takes 32 consecutive muons at a
 // time, GROUP lanes per muon.  Each lane loads its share of the muon's pairs
 // (voxel index, L, T) once, keeps the first RC of them in registers, and
@@ -29,8 +32,7 @@
 // per lane) writes every muon's coefficients; a second pass streams the lists
 // again and only adds g_ij to G_j, 4 or 8 pairs in flight per lane.  Twice
 // the list traffic from HBM, but neither pass waits at a block barrier; the
-// autotuner times it beside the one-pass variants, and on the largest scans
-// it is the one picked.
+// autotuner times it beside the one-pass variants (FP64).
 //
 // Recompute pass (k_em_fused_walk).  The same sums without stored lists: a
 // thread per muon (one muon each, so that a warp's lanes walk in step; the
@@ -774,7 +776,293 @@ __global__ void __launch_bounds__(256) k_em_scatter(FusedArgs<Real> a, const typ
     }
 }
 
+// ---------------------------------------------------------------------------
+// One-pass form of the mixed precision: a muon per lane group, no barrier.
+// ---------------------------------------------------------------------------
+// k_em_fused_lists holds a batch of muons at two block barriers so that one
+// warp can do their FP64 2x2 algebra together.  Here every group of lanes goes
+// through its own muon alone -- load the pairs, gather lambda, sum, 2x2, add
+// g_ij -- with the 2x2 algebra in double-floats on every lane of the group
+// (about 100 FP32 instructions; the same algebra in FP64 would hold the SM's
+// FP64 pipe, two lanes wide, for 960 cycles a muon).  The lists leave HBM once
+// for all but the pairs beyond the RC held per lane.
+//
+// Bound by the L1-to-L2 request path: 256x256x128 voxels, 2 M muons (212 M
+// pairs), 841 us: request path 69 % busy, L2 72 %, DRAM 55 %, issue 49 %; the
+// reductions' 0.50 sectors a pair are most of it.  With 20 M muons (2.1 G
+// pairs) a pass takes 8.6 ms, against 5.0 + 8.0 ms in the two-pass form (muon
+// pass and scatter).  Tried and slower: the next muon's pairs loaded ahead into
+// registers (16 instead of 24 warps on an SM), lists through shared memory by
+// cp.async or by bulk copies (their reads queue behind the reductions),
+// L2 prefetch of the next muon, muons in spatial order (reductions collide).
+constexpr int kOnceThreads = 128;
+
+// A double-float: the unevaluated sum of two floats, about 48 bits.
+struct Df {
+    float h, l;
+};
+__device__ __forceinline__ Df df_sum(float a, float b) {  // Knuth's exact sum
+    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+    return Df{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ Df df_prod(float a, float b) {  // exact product
+    const float p = __fmul_rn(a, b);
+    return Df{p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ Df df_muladd(float a, float b, Df c) {  // a b + c
+    const Df p = df_prod(a, b), s = df_sum(p.h, c.h);
+    return Df{s.h, __fadd_rn(s.l, __fadd_rn(p.l, c.l))};
+}
+// a x - b y to about a float's rounding, however much cancels (Kahan's
+// difference of products, with the low parts of a and b)
+__device__ __forceinline__ float df_cross(Df a, float x, Df b, float y) {
+    const float w = __fmul_rn(b.h, y), e = __fmaf_rn(-b.h, y, w), f = __fmaf_rn(a.h, x, -w);
+    return __fadd_rn(f, __fmaf_rn(a.l, x, __fmaf_rn(-b.l, y, e)));
+}
+__device__ __forceinline__ float rcp_approx(float x) {  // to 1 ulp; refined where it is used
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+struct DfE {  // the hit-error terms of Sigma
+    Df e00, e01, e11;
+};
+
+// A muon's g_ij as a function of a pair's length L and tail midpoint U:
+//   g = 1/2 pr^2 L [ (u_x . (1, U))^2 + (u_y . (1, U))^2 - 2 f11 (U - S01/S00)^2 - 2/S00
+//                    + (u_x1^2 + u_y1^2 - 2 f11) L^2 / 12 ],
+// u = Sigma^-1 (S, D) per plane, f11 = (Sigma^-1)_11: pr^2 (1/2 xyS - tr(Sigma^-1 W))
+// with both forms completed to squares, so that only their difference cancels
+// (k0 W00 + k1 W01 + k2 W11 cancels within each of them, by 1 / (1 - rho^2)).
+struct OnceCoef {
+    float ax, bx, ay, by, f, u0, h, w, c;
+};
+
+// The coefficients of a muon from its sums: Sigma and its determinant in
+// double-floats, Sigma^-1 (S, D) by exact differences of products.  The sums
+// come in as floats, so this leaves the coefficients' own rounding as the
+// largest error.  False where it would not (a determinant that nearly cancels,
+// is near the singular threshold or out of range), and for a NaN: the caller
+// then takes the FP64 algebra.
+__device__ __forceinline__ bool once_coefficients(float c0, float c1, float c2, float pr2, const float4& v,
+                                                  const DfE& e, OnceCoef& o, unsigned& singular) {
+    const Df s00 = df_muladd(pr2, c0, e.e00), s01 = df_muladd(pr2, c1, e.e01), s11 = df_muladd(pr2, c2, e.e11);
+    const Df a = df_prod(s00.h, s11.h), b = df_prod(s01.h, s01.h), d = df_sum(a.h, -b.h);
+    const float low = __fmaf_rn(s00.h, s11.l, __fmaf_rn(s00.l, s11.h, __fmaf_rn(-2.f * s01.h, s01.l, a.l - b.l)));
+    const float dl = __fadd_rn(d.l, low);
+    const float ad = fabsf(d.h);
+    if (!(ad > 2.0e-12f && ad > 1.0e-4f * a.h && a.h < 1.0e30f && s00.h > 1.0e-20f)) return false;
+    const float q = rcp_approx(d.h), r = fmaf(q, fmaf(-dl, q, fmaf(-d.h, q, 1.0f)), q);
+    const float p = rcp_approx(s00.h), rs = fmaf(p, fmaf(-s00.l, p, fmaf(-s00.h, p, 1.0f)), p);
+    // Sigma^-1 (S, D) = (s11 S - s01 D, s00 D - s01 S) / det
+    o.ax = r * df_cross(s11, v.x, s01, v.y);
+    o.bx = r * df_cross(s00, v.y, s01, v.x);
+    o.ay = r * df_cross(s11, v.z, s01, v.w);
+    o.by = r * df_cross(s00, v.w, s01, v.z);
+    o.u0 = s01.h * rs;
+    o.h = 2.0f * rs;
+    o.f = 2.0f * s00.h * r;
+    o.w = (fmaf(o.bx, o.bx, o.by * o.by) - o.f) * (1.0f / 12.0f);
+    o.c = 0.5f * pr2;
+    if (d.h <= 0.f) ++singular;  // inverse used, cost 0 (:461-464)
+    return true;
+}
+__device__ __forceinline__ float once_g(const OnceCoef& o, float L, float T) {
+    const float u = fmaf(0.5f, L, T);
+    const float x = fmaf(o.bx, u, o.ax), y = fmaf(o.by, u, o.ay), d = u - o.u0;
+    return o.c * L * fmaf(x, x, fmaf(y, y, fmaf(-o.f * d, d, fmaf(o.w * L, L, -o.h))));
+}
+
+// the pair's two factors beside its length: U = T + L/2 and q = U^2 + L^2/12, with
+// W00 = L, W01 = L U, W11 = L q
+__device__ __forceinline__ void pair_factors(float L, float T, float& u, float& q) {
+    u = fmaf(0.5f, L, T);
+    q = fmaf(u, u, L * L * (1.0f / 12.0f));
+}
+
+template <int GROUP, int RC, int MB>
+__global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a, DfE e, float4* __restrict__ sums) {
+    constexpr int kPer = 32 / GROUP;  // muons of a warp at once
+    constexpr int U = 4;              // loads in flight per lane for the pairs beyond the held ones
+    const int lane = threadIdx.x & 31, sub = lane / GROUP, glane = lane % GROUP;
+    const uint32_t V = a.V;
+    const uint64_t keep = l2_keep_policy();
+    const uint32_t step = ((gridDim.x * blockDim.x) >> 5) * kPer;
+    unsigned singular = 0;
+    uint32_t m = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kPer + sub;
+    uint64_t pb = 0;
+    uint32_t n = 0;
+    if (m < a.N) {
+        pb = a.off[m];
+        n = static_cast<uint32_t>(a.off[m + 1] - pb);
+    }
+    for (uint32_t mw = m - sub; mw < a.N; mw += step) {
+        uint32_t cj[RC];
+        float cL[RC], cT[RC], cl[RC];
+        {
+            const uint32_t* vp = a.vidx + pb + glane;
+            const float* lp = a.L + pb + glane;
+            const float* tp = a.T + pb + glane;
+#pragma unroll
+            for (int r = 0; r < RC; ++r) {
+                cj[r] = 0xffffffffu;
+                cL[r] = cT[r] = 0.f;
+                if (glane + r * GROUP < n) {
+                    cj[r] = __ldcs(vp + r * GROUP);
+                    cL[r] = __ldcs(lp + r * GROUP);
+                    cT[r] = __ldcs(tp + r * GROUP);
+                }
+            }
+        }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        float pr2 = 0.f;
+        if (m < a.N) {
+            v = __ldcs(a.sd + m);
+            pr2 = __ldcs(a.pr2 + m);
+        }
+        const uint32_t mn = m + step;
+        uint64_t pbn = 0, pen = 0;
+        if (mn < a.N && mn > m) {
+            pbn = a.off[mn];
+            pen = a.off[mn + 1];
+        }
+#pragma unroll
+        for (int r = 0; r < RC; ++r) {
+            cl[r] = 0.f;
+            if (cj[r] < V) cl[r] = ld_keep(a.lam + cj[r], keep);
+        }
+        float c0 = 0.f, c1 = 0.f, c2 = 0.f;
+        auto add = [&](float l, float L, float T) {
+            float u, q;
+            pair_factors(L, T, u, q);
+            const float lL = l * L;
+            c0 += lL;
+            c1 = fmaf(lL, u, c1);
+            c2 = fmaf(lL, q, c2);
+        };
+#pragma unroll
+        for (int r = 0; r < RC; ++r) add(cl[r], cL[r], cT[r]);
+        // pairs beyond the held ones: read again below, from L1 or L2
+        for (uint32_t k0 = glane + GROUP * RC; k0 < n; k0 += GROUP * U) {
+            uint32_t jj[U];
+            float ll[U], tt[U], lv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                jj[u] = 0xffffffffu;
+                ll[u] = tt[u] = 0.f;
+                if (k0 + u * GROUP < n) {
+                    jj[u] = __ldg(a.vidx + pb + k0 + u * GROUP);
+                    ll[u] = __ldg(a.L + pb + k0 + u * GROUP);
+                    tt[u] = __ldg(a.T + pb + k0 + u * GROUP);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                lv[u] = 0.f;
+                if (jj[u] < V) lv[u] = ld_keep(a.lam + jj[u], keep);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) add(lv[u], ll[u], tt[u]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = GROUP / 2; o > 0; o >>= 1) {
+            c0 += __shfl_xor_sync(kFull, c0, o);
+            c1 += __shfl_xor_sync(kFull, c1, o);
+            c2 += __shfl_xor_sync(kFull, c2, o);
+        }
+        OnceCoef o{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        unsigned sing = 0;
+        if (m < a.N && !once_coefficients(c0, c1, c2, pr2, v, e, o, sing)) {
+            // rare: the terms added here from the lists, and nothing below
+            float k0, k1, k2;
+            unsigned long long s64 = 0;
+            double cost = 0.0;
+            muon_coefficients<float>(c0, c1, c2, pr2, v, a.E00, a.E01, a.E11, false, k0, k1, k2, cost, s64);
+            sing = static_cast<unsigned>(s64);
+            for (uint32_t k = glane; k < n; k += GROUP) {
+                const uint32_t j = a.vidx[pb + k];
+                if (j < V) red_add(a.G + j, g_term(k0, k1, k2, a.L[pb + k], a.T[pb + k]), keep);
+            }
+            n = 0;
+#pragma unroll
+            for (int r = 0; r < RC; ++r) cj[r] = 0xffffffffu;
+        }
+        if (glane == 0) {
+            singular += sing;
+            if (sums && m < a.N) sums[m] = make_float4(c0, c1, c2, 0.f);
+        }
+        auto put = [&](uint32_t j, float L, float T) {
+            if (j < V) red_add(a.G + j, once_g(o, L, T), keep);
+        };
+        for (uint32_t k0p = glane + GROUP * RC; k0p < n; k0p += GROUP * U) {
+            uint32_t jj[U];
+            float ll[U], tt[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                jj[u] = 0xffffffffu;
+                ll[u] = tt[u] = 0.f;
+                if (k0p + u * GROUP < n) {
+                    jj[u] = __ldcs(a.vidx + pb + k0p + u * GROUP);
+                    ll[u] = __ldcs(a.L + pb + k0p + u * GROUP);
+                    tt[u] = __ldcs(a.T + pb + k0p + u * GROUP);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) put(jj[u], ll[u], tt[u]);
+        }
+#pragma unroll
+        for (int r = 0; r < RC; ++r) put(cj[r], cL[r], cT[r]);
+        m = mn;
+        pb = pbn;
+        n = static_cast<uint32_t>(pen - pbn);
+        if (mw + step < mw) break;  // the next muons are past 2^32
+    }
+    singular = __reduce_add_sync(kFull, singular);
+    if (lane == 0 && singular) atomicAdd(&a.ctr->singular, static_cast<unsigned long long>(singular));
+}
+
+// The cost of every muon (src/MutoMLSD.cpp:465-468) from the sums that
+// k_em_once left, in FP64, a muon per lane.
+__global__ void __launch_bounds__(256) k_once_cost(FusedArgs<float> a, const float4* __restrict__ sums) {
+    const uint64_t m = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    double cost = 0.0;
+    unsigned long long singular = 0;  // counted by k_em_once
+    if (m < a.N) {
+        const float4 c = sums[m], v = a.sd[m];
+        float k0, k1, k2;
+        muon_coefficients<float>(c.x, c.y, c.z, a.pr2[m], v, a.E00, a.E01, a.E11, true, k0, k1, k2, cost, singular);
+    }
+    flush_counters<256>(cost, 0ull, 1, a.ctr);
+}
+
 }  // namespace
+
+namespace {
+Df df_of(double x) {
+    const float h = static_cast<float>(x);
+    return Df{h, static_cast<float>(x - static_cast<double>(h))};
+}
+template <int GROUP, int RC, int MB>
+void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t s) {
+    const DfE e{df_of(a.E00), df_of(a.E01), df_of(a.E11)};
+    const uint64_t need = (static_cast<uint64_t>(a.N) * GROUP + kOnceThreads - 1) / kOnceThreads;
+    const uint64_t most = static_cast<uint64_t>(MB) * num_sms;
+    k_em_once<GROUP, RC, MB><<<static_cast<unsigned>(need < most ? need : most), kOnceThreads, 0, s>>>(a, e, sums);
+    count_launches(1);
+}
+}  // namespace
+
+void launch_em_once(const FusedArgs<float>& a, int group, float4* sums, int num_sms, cudaStream_t s) {
+    if (a.N == 0) return;
+    // blocks per SM: what the registers allow
+    if (group <= 16) run_once<16, kOnceHeld, 6>(a, sums, num_sms, s);
+    else run_once<32, kOnceHeld, 7>(a, sums, num_sms, s);
+    if (sums) {
+        k_once_cost<<<static_cast<unsigned>((static_cast<uint64_t>(a.N) + 255) / 256), 256, 0, s>>>(a, sums);
+        count_launches(1);
+    }
+}
 
 // (GROUP, RC) of each stored-list variant; the last is the staged one (GROUP
 // lanes per muon, its batch's pairs in shared memory)

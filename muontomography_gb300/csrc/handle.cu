@@ -165,6 +165,8 @@ struct Params {
 
 // how an EM / MAP handle keeps its pair lists
 enum Lists { kListsVoxelMajor = 1, kListsMuonMajor = 2, kListsRecompute = 3 };
+// fused_variant beyond the forced ones: the mixed form's one-pass kernel (launch_em_once)
+constexpr int kFusedOnce = kFusedVariants + 8;
 
 // variant of the one-shot (PoCA) handle: 0 PoCA, 1 PoCut, 2 SLR, 3 SLRIter
 Params parse_params(Method m, const std::string& text, int variant = 0) {
@@ -413,6 +415,7 @@ struct muto_handle {
     DevMem gsum;                      // muon-major / recompute: per-voxel sums of g_ij (bricked like lam_b)
     DevMem ltot;                      // recompute: in-grid path length per kept muon
     int fused_variant = 1, fused_blocks = 0;  // stored-list fused pass: variant and persistent grid
+    int once_group = 32;                         // lanes per muon of the one-pass mixed form
     int scatter_group = 32, scatter_blocks = 0;  // split form's scatter pass (fused_variant == kFusedVariants)
     int scatter_depth = 4;                       // its pairs in flight per lane
     // the split form overlapped: muon pass and scatter on chunks of the muons,
@@ -1368,6 +1371,12 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
     a.compute_cost = cost ? 1 : 0;
     a.prefetch = P.fused_prefetch ? 1 : 0;
     a.ctr = h->ctr();
+    if constexpr (std::is_same<Real, float>::value) {
+        if (h->lists == kListsMuonMajor && h->fused_variant == kFusedOnce) {
+            launch("em_fused", [&] { launch_em_once(a, h->once_group, cost ? h->kvec.as<float4>() : nullptr, h->num_sms, s); });
+            return;
+        }
+    }
     if (h->lists == kListsMuonMajor && h->fused_variant == kFusedVariants) {
         // split form: the muon pass writes every muon's coefficients, the scatter adds g_ij
         const MuonPassArgs<Real> m = muon_args<Real>(h, lam, cost);
@@ -1442,14 +1451,27 @@ std::map<TuneShape, int> g_fused_choice;  // the tuner's pick per scan shape (gu
 
 template <typename Real>
 void autotune_fused(muto_handle* h) {
-    if (h->lists != kListsMuonMajor || h->N == 0) return;
+    if (h->lists != kListsMuonMajor) return;
+    const double avg = h->N ? static_cast<double>(h->npairs) / static_cast<double>(h->N) : 0.0;
+    const bool forced = h->P.fused_variant >= 0;
+    if (!forced && !h->fp64() && !h->P.fused_prefetch) {
+        // Mixed: the one-pass kernel, faster than every other form on cubes of
+        // 16 to 150 voxels a side and on the 256 x 256 x 128 grid (mean paths of
+        // 23 to 221 pairs) and equal below, so nothing is timed here.  16 lanes
+        // a muon up to a mean path of 160 pairs, 32 beyond (0.8 M muons): 247
+        // against 438 us at 46 pairs, 309 against 455 at 91, 493 against 507 at
+        // 142, 759 against 686 at 213.
+        h->fused_variant = kFusedOnce;
+        h->once_group = avg <= 160.0 ? 16 : 32;
+        h->overlap = false;
+        return;
+    }
+    if (h->N == 0) return;
     HostPhase ph(h, "autotune");
-    const double avg = static_cast<double>(h->npairs) / static_cast<double>(h->N);
     int log2n = 0;
     while ((h->N >> log2n) > 1) ++log2n;
     const TuneShape shape{h->fp64() ? 1 : 0, h->device, log2n, static_cast<int>(avg / 8.0)};
     std::vector<int> cands;
-    const bool forced = h->P.fused_variant >= 0;
     if (forced) cands.push_back(h->P.fused_variant);
     for (int v = 0; v < kFusedVariants && !forced; ++v) {
         const int held = fused_variant_held(v);
@@ -2126,6 +2148,11 @@ int muto_get_status(const muto_handle* hc, muto_status* out) {
         out->muon_group = h->scatter_group;
         out->tile_pairs = h->scatter_depth;
         out->tile_muons = h->overlap ? muto_handle::kOverlapChunks : 0;
+    } else if (h->method != kPoca && h->lists == kListsMuonMajor && h->fused_variant == kFusedOnce) {
+        out->muon_pass = 3;
+        out->muon_group = h->once_group;
+        out->tile_pairs = h->once_group * kOnceHeld;
+        out->tile_muons = 32 / h->once_group;
     } else if (h->method != kPoca && h->lists == kListsMuonMajor) {
         const bool staged = h->fused_variant == kFusedStaged;
         out->muon_pass = staged ? 6 : 3;
