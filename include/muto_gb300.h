@@ -111,9 +111,9 @@ typedef struct muto_handle muto_handle;
  * ("mixed" default, or "fp64"), "use_graph" (true), "random_seed",
  * "compute_cost" (computed when early_stop/log_results is set, or when true),
  * "newton_max_iter" (MAP cubic cap, 200), "tile_pairs" (pairs per TMA tile),
- * "muon_pass" ("auto": the warp-batched variant, its group size chosen by
- * timing on the scan's data at prepare and reused for later scans of the
- * same shape in the process; "tile" or "warp" force one),
+ * "muon_pass" ("auto": the warp-batched variant, its group size by the mean
+ * path in fp64, and in the mixed form chosen by timing on the scan's data at
+ * prepare and reused for later scans of the same shape in the process; "tile" or "warp" force one),
  * "muon_layout" ("auto": the per-muon coefficient table in column order of
  * the muons' PoCA points when it would take more than a third of L2, else
  * in muon order; "columns" or "index" force one),
@@ -133,10 +133,10 @@ typedef struct muto_handle muto_handle;
  * "muon_major" and "recompute" require the mean update),
  * "fused_variant" ("auto": the mean update's pass over muon-major lists
  * is, in the mixed form, the one-pass kernel without block barriers, its
- * lanes per muon by the scan's mean path; in fp64 it takes the lanes per
- * muon and pairs held per lane by timing the variants that suit the mean
- * path and the split form (the muon pass, then a second pass over the lists
- * adding the terms) at prepare; "4x8", "8x4",
+ * lanes per muon by the scan's mean path; in fp64 the split form (the muon
+ * pass, then a second pass over the lists adding the terms); with
+ * "fused_prefetch" the one-pass variants that suit the mean path and the
+ * split form are timed at prepare; "4x8", "8x4",
  * "8x8", "8x16", "16x8", "16x16", "split", "split8" (its scatter with 8
  * pairs in flight per lane), "split8_overlap" (the same, the scatter of one
  * chunk of muons running beside the muon pass of the next) or "staged"

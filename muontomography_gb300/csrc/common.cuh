@@ -256,11 +256,19 @@ struct MuonPassArgs {
     const Real* lam;                          // V: lambda gathered by the muons
     typename Vec4<Real>::type* kout;          // N: (k0, k1, k2, 0)
     const uint32_t* kslot;                    // N: the row of kout each muon writes (null: its own index)
+    const uint32_t* order;                    // N (or null): the muons by decreasing path length (warp-batched variant)
+    const Real* W11;                          // P (or null): FP64, W11 of each pair; T then holds its W01
     uint32_t V;
     double E00, E01, E11;
     int compute_cost;
     Counters* ctr;
 };
+// FP64 pairs: T -> W01 in place and W11 from (L, T)
+void launch_pair_weights(const double* L, double* T, uint64_t P, double* W11, cudaStream_t s);
+// the tails T of every path from its lengths, summed as the set-up walk sums them
+void launch_path_tails(const uint64_t* off, uint64_t n, const double* L, double* T, cudaStream_t s);
+// len[i] = off[i+1] - off[i]
+void launch_path_lengths(const uint64_t* off, uint64_t n, uint32_t* len, cudaStream_t s);
 template <typename Real>
 void launch_em_muon(const MuonPassArgs<Real>& a, int tile_pairs, int tile_muons, int blocks, int group,
                     cudaStream_t s);
@@ -396,6 +404,7 @@ struct FusedArgs {
     const Real* pr2;                          // N
     const Real* lam;                          // lambda gathered by the muons (bricked copy when brick)
     Real* G;                                  // per-voxel sums of g_ij, zero on entry
+    const Real* W11;                          // split form: as in MuonPassArgs (or null)
     uint32_t V;                               // entries of lam and G
     uint32_t N;                               // kept muons
     double E00, E01, E11;
@@ -407,7 +416,8 @@ struct FusedArgs {
     const uint32_t* kept;
     const double* scat;                       // 3N PoCA points
     const double* ltot;                       // N in-grid path lengths (-1: dropped walk)
-    const uint32_t* order;                    // N (or null): the muons in the order their walks run
+    const uint32_t* order;                    // N (or null): the muons in the order their walks (recompute form)
+                                              // or scatters (split form) run
     DevGrid g;
     int straight;
     BrickDims bdims;

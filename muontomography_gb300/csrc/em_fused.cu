@@ -720,7 +720,9 @@ int fused_blocks_per_sm() {
 // are in flight per lane; with AHEAD the next muon's offsets and
 // coefficients are loaded while the current muon's pairs are, so a muon's
 // pair loads do not wait on its offsets.
-template <typename Real, int GROUP, int U, bool AHEAD>
+// WEIGHTS (FP64): the pairs hold W01 and W11 beside L, so a pair costs three
+// FP64 operations instead of seven.
+template <typename Real, int GROUP, int U, bool AHEAD, bool WEIGHTS = false>
 __global__ void __launch_bounds__(256) k_em_scatter(FusedArgs<Real> a, const typename Vec4<Real>::type* __restrict__ kvec) {
     using R4 = typename Vec4<Real>::type;
     const uint64_t gid = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / GROUP;
@@ -731,10 +733,12 @@ __global__ void __launch_bounds__(256) k_em_scatter(FusedArgs<Real> a, const typ
     uint64_t m = gid;
     R4 kv{};
     uint64_t pb = 0, pe = 0;
+    auto muon = [&](uint64_t i) -> uint64_t { return a.order ? a.order[i] : i; };
     if (AHEAD && m < a.N) {
-        kv = kvec[m];
-        pb = a.off[m];
-        pe = a.off[m + 1];
+        const uint64_t i = muon(m);
+        kv = kvec[i];
+        pb = a.off[i];
+        pe = a.off[i + 1];
     }
     for (; m < a.N; m += ngroups) {
         R4 kn{};
@@ -742,18 +746,20 @@ __global__ void __launch_bounds__(256) k_em_scatter(FusedArgs<Real> a, const typ
         if (AHEAD) {
             const uint64_t mn = m + ngroups;
             if (mn < a.N) {
-                kn = kvec[mn];
-                pbn = a.off[mn];
-                pen = a.off[mn + 1];
+                const uint64_t i = muon(mn);
+                kn = kvec[i];
+                pbn = a.off[i];
+                pen = a.off[i + 1];
             }
         } else {
-            kv = kvec[m];
-            pb = a.off[m];
-            pe = a.off[m + 1];
+            const uint64_t i = muon(m);
+            kv = kvec[i];
+            pb = a.off[i];
+            pe = a.off[i + 1];
         }
         for (uint64_t k0 = pb + glane; k0 < pe; k0 += static_cast<uint64_t>(GROUP) * U) {
             uint32_t jj[U];
-            Real ll[U], tt[U];
+            Real ll[U], tt[U], qq[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const uint64_t k = k0 + static_cast<uint64_t>(u) * GROUP;
@@ -762,11 +768,23 @@ __global__ void __launch_bounds__(256) k_em_scatter(FusedArgs<Real> a, const typ
                     jj[u] = __ldcs(a.vidx + k);
                     ll[u] = __ldcs(a.L + k);
                     tt[u] = __ldcs(a.T + k);
+                    if (WEIGHTS) qq[u] = __ldcs(a.W11 + k);
                 }
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (jj[u] < V) red_add(a.G + jj[u], g_term(kv.x, kv.y, kv.z, ll[u], tt[u]), keep);
+                if (jj[u] < V) {
+                    Real g;
+                    if constexpr (WEIGHTS) {
+                        g = fma(kv.z, qq[u], fma(kv.y, tt[u], kv.x * ll[u]));
+                    } else if constexpr (sizeof(Real) == 8) {
+                        const Real mid = fma(0.5, ll[u], tt[u]);
+                        g = ll[u] * fma(kv.z, fma(mid, mid, ll[u] * ll[u] * (1.0 / 12.0)), fma(kv.y, mid, kv.x));
+                    } else {
+                        g = g_term(kv.x, kv.y, kv.z, ll[u], tt[u]);
+                    }
+                    red_add(a.G + jj[u], g, keep);
+                }
         }
         if (AHEAD) {
             kv = kn;
@@ -1131,6 +1149,7 @@ int scatter_blocks_per_sm() {
 
 template <typename Real>
 int em_scatter_blocks(int group, int depth) {
+    if (group <= 4) return scatter_blocks_per_sm<Real, 4, 4, true>();
     if (depth > 4) {
         if (group <= 8) return scatter_blocks_per_sm<Real, 8, 8, true>();
         if (group <= 16) return scatter_blocks_per_sm<Real, 16, 8, true>();
@@ -1149,7 +1168,17 @@ void launch_em_scatter(const FusedArgs<Real>& a, const typename Vec4<Real>::type
     if (a.N == 0) return;
     const uint64_t need = (static_cast<uint64_t>(a.N) * group + 255) / 256;
     const unsigned nb = static_cast<unsigned>(need < static_cast<uint64_t>(blocks) ? need : blocks);
-    if (depth > 4) {
+    if constexpr (sizeof(Real) == 8) {
+        if (a.W11) {  // (the grid was sized for the plain form, which keeps fewer values per pair)
+            if (group <= 4) k_em_scatter<Real, 4, 4, true, true><<<nb, 256, 0, s>>>(a, kvec);
+            else k_em_scatter<Real, 8, 8, true, true><<<nb, 256, 0, s>>>(a, kvec);
+            count_launches(1);
+            return;
+        }
+    }
+    if (group <= 4) {
+        k_em_scatter<Real, 4, 4, true><<<nb, 256, 0, s>>>(a, kvec);
+    } else if (depth > 4) {
         if (group <= 8) k_em_scatter<Real, 8, 8, true><<<nb, 256, 0, s>>>(a, kvec);
         else if (group <= 16) k_em_scatter<Real, 16, 8, true><<<nb, 256, 0, s>>>(a, kvec);
         else k_em_scatter<Real, 32, 8, true><<<nb, 256, 0, s>>>(a, kvec);
@@ -1163,6 +1192,51 @@ void launch_em_scatter(const FusedArgs<Real>& a, const typename Vec4<Real>::type
 template void launch_em_scatter<float>(const FusedArgs<float>&, const float4*, int, int, int, cudaStream_t);
 template void launch_em_scatter<double>(const FusedArgs<double>&, const double4*, int, int, int, cudaStream_t);
 template void launch_em_fused<double>(const FusedArgs<double>&, int, int, cudaStream_t);
+
+namespace {
+__global__ void __launch_bounds__(256) k_pair_weights(const double* __restrict__ L, double* __restrict__ T, uint64_t P,
+                                                      double* __restrict__ W11) {
+    const uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= P) return;
+    const double l = L[k], mid = fma(0.5, l, T[k]);
+    T[k] = l * mid;
+    W11[k] = l * fma(mid, mid, l * l * (1.0 / 12.0));
+}
+__global__ void __launch_bounds__(128) k_path_tails(const uint64_t* __restrict__ off, uint64_t n,
+                                                    const double* __restrict__ L, double* __restrict__ T) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t b = off[i];
+    double t = 0.0;  // as k_path_fill_bounded sums them
+    for (uint64_t k = off[i + 1]; k-- > b;) {
+        T[k] = t;
+        t = dadd(t, L[k]);
+    }
+}
+__global__ void __launch_bounds__(256) k_path_lengths(const uint64_t* __restrict__ off, uint64_t n,
+                                                      uint32_t* __restrict__ len) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) len[i] = static_cast<uint32_t>(off[i + 1] - off[i]);
+}
+}  // namespace
+
+void launch_pair_weights(const double* L, double* T, uint64_t P, double* W11, cudaStream_t s) {
+    if (P == 0) return;
+    k_pair_weights<<<static_cast<unsigned>((P + 255) / 256), 256, 0, s>>>(L, T, P, W11);
+    count_launches(1);
+}
+
+void launch_path_tails(const uint64_t* off, uint64_t n, const double* L, double* T, cudaStream_t s) {
+    if (n == 0) return;
+    k_path_tails<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(off, n, L, T);
+    count_launches(1);
+}
+
+void launch_path_lengths(const uint64_t* off, uint64_t n, uint32_t* len, cudaStream_t s) {
+    if (n == 0) return;
+    k_path_lengths<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(off, n, len);
+    count_launches(1);
+}
 
 template <typename Real>
 void launch_em_fused_walk(const FusedArgs<Real>& a, int num_sms, cudaStream_t s) {

@@ -16,6 +16,8 @@
 //   sum     GROUP lanes per muon add lambda_j W_ij in the storage precision;
 //   2x2     one thread per muon: Sigma in FP64, determinant and inverse in
 //           FP64, cost in FP64, the k coefficients written to global memory.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace muto {
@@ -292,7 +294,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_em_muon(MuonPassArgs<Real> a, i
 // algebra of their 32 muons together (the FP64 pipe is busy for one warp
 // instruction per 32 muons, not per muon).
 // ---------------------------------------------------------------------------
-template <typename Real, int GROUP>
+// WEIGHTS (FP64): the pairs hold W01 and W11 beside L, so a pair costs three
+// FP64 operations instead of eight.
+template <typename Real, int GROUP, bool WEIGHTS>
 __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a, uint32_t n_muons) {
     using R4 = typename Vec4<Real>::type;
     constexpr int U = 5;                    // pair loads in flight per lane per round
@@ -311,13 +315,14 @@ __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a,
         const uint64_t m0 = bt * 32;
         Real my0 = 0, my1 = 0, my2 = 0;  // the sums of muon m0 + lane
         for (int q = 0; q < 32; q += kPer) {
-            const uint64_t m = m0 + q + sub;
+            const uint64_t mi = m0 + q + sub;
             Real c0 = 0, c1 = 0, c2 = 0;
-            if (m < n_muons) {
+            if (mi < n_muons) {
+                const uint64_t m = a.order ? a.order[mi] : mi;
                 const uint64_t pb = a.off[m], pe = a.off[m + 1];
                 for (uint64_t k0 = pb + glane; k0 < pe; k0 += GROUP * U) {
                     uint32_t jj[U];
-                    Real ll[U], tt[U], lam[U];
+                    Real ll[U], tt[U], qq[U], lam[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const uint64_t k = k0 + static_cast<uint64_t>(u) * GROUP;
@@ -326,6 +331,7 @@ __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a,
                             jj[u] = __ldcs(a.vidx + k);
                             ll[u] = __ldcs(a.L + k);
                             tt[u] = __ldcs(a.T + k);
+                            if (WEIGHTS) qq[u] = __ldcs(a.W11 + k);
                         }
                     }
 #pragma unroll
@@ -334,10 +340,22 @@ __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a,
                     for (int u = 0; u < U; ++u) {
                         if (jj[u] != 0xffffffffu) {
                             const Real L = ll[u], T = tt[u], l = lam[u];
-                            const Real LT = L * T;
-                            c0 += l * L;
-                            c1 += l * (LT + L * L * Real(0.5));
-                            c2 += l * (L * L * L * Real(1.0 / 3.0) + (L + T) * LT);
+                            if constexpr (WEIGHTS) {
+                                c0 = fma(l, L, c0);
+                                c1 = fma(l, T, c1);
+                                c2 = fma(l, qq[u], c2);
+                            } else if constexpr (sizeof(Real) == 8) {
+                                // W00 = L, W01 = L U, W11 = L (U^2 + L^2/12), U = T + L/2
+                                const Real mid = fma(0.5, L, T), lL = l * L;
+                                c0 += lL;
+                                c1 = fma(lL, mid, c1);
+                                c2 = fma(lL, fma(mid, mid, L * L * (1.0 / 12.0)), c2);
+                            } else {
+                                const Real LT = L * T;
+                                c0 += l * L;
+                                c1 += l * (LT + L * L * Real(0.5));
+                                c2 += l * (L * L * L * Real(1.0 / 3.0) + (L + T) * LT);
+                            }
                         }
                     }
                 }
@@ -359,8 +377,8 @@ __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a,
             }
         }
         // ---- FP64 2x2 algebra of the warp's 32 muons, one per lane ----------
-        const uint64_t m = m0 + lane;
-        if (m < n_muons) {
+        if (m0 + lane < n_muons) {
+            const uint64_t m = a.order ? a.order[m0 + lane] : m0 + lane;
             const Real pr2 = a.pr2[m];
             const double p2 = static_cast<double>(pr2);
             const double S00 = p2 * static_cast<double>(my0) + a.E00;
@@ -454,14 +472,19 @@ void launch_em_muon(const MuonPassArgs<Real>& a, int tile_pairs, int tile_muons,
 template void launch_em_muon<float>(const MuonPassArgs<float>&, int, int, int, int, cudaStream_t);
 template void launch_em_muon<double>(const MuonPassArgs<double>&, int, int, int, int, cudaStream_t);
 
-template <typename Real>
-int em_muon_warp_blocks(int group) {
+template <typename Real, bool WEIGHTS>
+static int warp_blocks(int group) {
     int n = 0;
     cudaError_t e;
-    if (group <= 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 8>, kThreads, 0);
-    else if (group <= 16) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 16>, kThreads, 0);
-    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 32>, kThreads, 0);
+    if (group <= 4) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 4, WEIGHTS>, kThreads, 0);
+    else if (group <= 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 8, WEIGHTS>, kThreads, 0);
+    else if (group <= 16) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 16, WEIGHTS>, kThreads, 0);
+    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 32, WEIGHTS>, kThreads, 0);
     return (e == cudaSuccess && n > 0) ? n : 1;
+}
+template <typename Real>
+int em_muon_warp_blocks(int group) {
+    return warp_blocks<Real, false>(group);
 }
 template int em_muon_warp_blocks<float>(int);
 template int em_muon_warp_blocks<double>(int);
@@ -472,9 +495,19 @@ void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int bloc
     const uint64_t batches = (static_cast<uint64_t>(n_muons) + 31) / 32;
     const uint64_t need = (batches + kThreads / 32 - 1) / (kThreads / 32);
     const unsigned nb = static_cast<unsigned>(need < static_cast<uint64_t>(blocks) ? need : blocks);
-    if (group <= 8) k_em_muon_warp<Real, 8><<<nb, kThreads, 0, s>>>(a, n_muons);
-    else if (group <= 16) k_em_muon_warp<Real, 16><<<nb, kThreads, 0, s>>>(a, n_muons);
-    else k_em_muon_warp<Real, 32><<<nb, kThreads, 0, s>>>(a, n_muons);
+    auto go = [&](auto w) {
+        constexpr bool W = decltype(w)::value;
+        if (group <= 4) k_em_muon_warp<Real, 4, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+        else if (group <= 8) k_em_muon_warp<Real, 8, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+        else if (group <= 16) k_em_muon_warp<Real, 16, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+        else k_em_muon_warp<Real, 32, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+    };
+    if constexpr (sizeof(Real) == 8) {
+        if (a.W11) go(std::true_type{});
+        else go(std::false_type{});
+    } else {
+        go(std::false_type{});
+    }
     count_launches(1);
 }
 template void launch_em_muon_warp<float>(const MuonPassArgs<float>&, uint32_t, int, int, cudaStream_t);

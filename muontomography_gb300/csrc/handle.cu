@@ -408,7 +408,9 @@ struct muto_handle {
     uint32_t slr_levels = 0;          // levels of the SLRIter schedule (0: none or sequential)
     uint64_t vclass_off[kVoxClasses] = {};
     DevMem kslot;                     // per kept muon: its row of kvec (empty: its own index)
-    DevMem walk_order;                // recompute form: the kept muons by decreasing path bound
+    DevMem walk_order;                // recompute form: the kept muons by decreasing path bound; FP64 lists: by
+                                      // decreasing path length
+    DevMem pair_w11;                  // FP64 lists: W11 of every pair (T then holds W01), when the memory allows
     DevMem mult, start, kvec, keys;   // keys: the voxel pass's order key of every pair
     DevMem win;                       // per voxel: the last selection window (center, half-width)
     int lists = kListsVoxelMajor;     // how the pair lists are kept (Lists)
@@ -1017,6 +1019,8 @@ void prepare_em(muto_handle* h) {
     h->pr2.alloc((N + kPad) * sizeof(Real), &h->dev_bytes);
     h->scat.alloc(std::max<uint64_t>(N, 1) * 3 * sizeof(double), &h->dev_bytes);
     h->pr64.alloc(std::max<uint64_t>(N, 1) * sizeof(double), &h->dev_bytes);
+    h->pair_w11.release();
+    h->walk_order.release();
     // --- how the lists are kept: the voxel-major copy for the median and
     // percentile updates; for the mean update the muon-major lists alone, or
     // none (the paths walked again every iteration) ---
@@ -1310,6 +1314,8 @@ MuonPassArgs<Real> muon_args(muto_handle* h, const Real* lam, bool cost) {
     a.lam = lam;
     a.kout = h->kvec.as<R4>();
     a.kslot = h->kslot.empty() ? nullptr : h->kslot.as<uint32_t>();
+    a.order = h->walk_order.empty() ? nullptr : h->walk_order.as<uint32_t>();
+    a.W11 = h->pair_w11.empty() ? nullptr : h->pair_w11.as<Real>();
     a.V = static_cast<uint32_t>(h->V());
     a.E00 = 4.0 * exy * exy / (ezo * ezo);
     a.E11 = 2.0 * exy * exy * (1.0 + (ezi / ezo + 1.0) * ezi / ezo);
@@ -1379,6 +1385,8 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
     }
     if (h->lists == kListsMuonMajor && h->fused_variant == kFusedVariants) {
         // split form: the muon pass writes every muon's coefficients, the scatter adds g_ij
+        a.order = h->walk_order.empty() ? nullptr : h->walk_order.as<uint32_t>();
+        a.W11 = h->pair_w11.empty() ? nullptr : h->pair_w11.as<Real>();
         const MuonPassArgs<Real> m = muon_args<Real>(h, lam, cost);
         if (!h->overlap || profiled || h->N < static_cast<uint64_t>(muto_handle::kOverlapChunks)) {
             // (profiled passes time each kernel alone)
@@ -1449,6 +1457,54 @@ void launch_fused_update(muto_handle* h, const Real* lam, OutT* out, double* gra
 // warm-up and two timed launches each); the per-voxel sums are cleared after.
 std::map<TuneShape, int> g_fused_choice;  // the tuner's pick per scan shape (guarded by g_tune_mu)
 
+// FP64 lists, set-up of their passes, which are bound by the FP64 pipe (an
+// instruction holds it for 16 cycles however few lanes are active): the muons by
+// decreasing path length, so that a warp's lane groups run out of pairs
+// together; and W01 (in place of T) and W11 of every pair, when W11's 8 bytes
+// beside the lists' 20 are at most a quarter of the memory that is left.  A pair
+// then costs three FP64 operations in either pass, not eight and seven.
+// The FP64 passes a config may name (the TMA tile pass, a one-pass variant or
+// its prefetch) keep the lists as they are.
+bool fp64_passes(const muto_handle* h) {
+    return h->fp64() && h->N > 0 && h->lists != kListsRecompute && h->P.muon_pass != 1 && h->P.fused_variant < 0 &&
+           !h->P.fused_prefetch;
+}
+void prepare_fp64_passes(muto_handle* h) {
+    if (!fp64_passes(h)) return;
+    cudaStream_t s = h->stream;
+    size_t free_b = 0, total_b = 0;
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    unsigned long long held = 0, used = 0;  // the pool's blocks that are mapped but free
+    CK(cudaMemPoolGetAttribute(device_pool(h->device), cudaMemPoolAttrReservedMemCurrent, &held));
+    CK(cudaMemPoolGetAttribute(device_pool(h->device), cudaMemPoolAttrUsedMemCurrent, &used));
+    const uint64_t left = free_b + (held > used ? held - used : 0);
+    DevMem len, work;
+    len.alloc(h->N * sizeof(uint32_t), &h->dev_bytes);
+    work.alloc(512 * sizeof(uint32_t), &h->dev_bytes);
+    h->walk_order.alloc(h->N * sizeof(uint32_t), &h->dev_bytes);
+    run(h, "path_order", [&] {
+        launch_path_lengths(h->off.as<uint64_t>(), h->N, len.as<uint32_t>(), s);
+        launch_length_order(len.as<uint32_t>(), nullptr, h->N, h->walk_order.as<uint32_t>(), work.as<uint32_t>(), s);
+    });
+    if (h->npairs * sizeof(double) <= left / 4) {
+        h->pair_w11.alloc((h->npairs + kPad) * sizeof(double), &h->dev_bytes);
+        run(h, "pair_weights", [&] {
+            launch_pair_weights(h->L.as<double>(), h->T.as<double>(), h->npairs, h->pair_w11.as<double>(), s);
+        });
+    }
+    CK(cudaStreamSynchronize(s));  // the lengths go out of scope
+}
+
+// The FP64 muon pass: 4 lanes a muon up to a mean path of 80 pairs, 8 beyond (few
+// lanes: each level of the lanes' sum is an FP64 instruction per value; 422
+// against 490 us for an iteration at 46 pairs, 787 against 705 at 91).
+void set_fp64_muon_pass(muto_handle* h) {
+    const double avg = h->N ? static_cast<double>(h->npairs) / static_cast<double>(h->N) : 0.0;
+    h->muon_kind = 2;
+    h->muon_group = avg <= 80.0 ? 4 : 8;
+    h->warp_blocks = em_muon_warp_blocks<double>(h->muon_group) * h->num_sms;
+}
+
 template <typename Real>
 void autotune_fused(muto_handle* h) {
     if (h->lists != kListsMuonMajor) return;
@@ -1467,6 +1523,18 @@ void autotune_fused(muto_handle* h) {
         return;
     }
     if (h->N == 0) return;
+    if (fp64_passes(h)) {
+        // FP64: the split form, whose two passes spend the fewest FP64
+        // operations on a pair (0.4 M muons, 71 / 142 pairs a path: 585 / 1 052
+        // us; the one-pass form 1 513 / 2 135 us)
+        h->fused_variant = kFusedVariants;
+        set_fp64_muon_pass(h);
+        h->scatter_group = 8;
+        h->scatter_depth = 8;
+        h->scatter_blocks = em_scatter_blocks<Real>(8, 8) * h->num_sms;
+        h->overlap = false;
+        return;
+    }
     HostPhase ph(h, "autotune");
     int log2n = 0;
     while ((h->N >> log2n) > 1) ++log2n;
@@ -1569,11 +1637,15 @@ void autotune_fused(muto_handle* h) {
 }
 
 
-// In-project autotuner: time the candidate muon-pass variants on this scan's
+// In-project autotuner (mixed form): time the candidate muon-pass variants on this scan's
 // own lists (one warm-up and two timed launches each) and keep the fastest.
 template <typename Real>
 void autotune_muon_pass(muto_handle* h) {
     if (h->N == 0) return;
+    if (h->P.muon_pass == 0 && fp64_passes(h)) {
+        set_fp64_muon_pass(h);
+        return;
+    }
     HostPhase ph(h, "autotune");
     int log2n = 0;
     while ((h->N >> log2n) > 1) ++log2n;
@@ -2224,6 +2296,7 @@ int muto_prepare(muto_handle* h) {
             prepare_poca(h);
         } else if (h->fp64()) {
             prepare_em<double>(h);
+            prepare_fp64_passes(h);
             if (h->lists == kListsVoxelMajor) {
                 autotune_muon_pass<double>(h);
                 autotune_voxel_pass<double>(h);
@@ -2381,7 +2454,15 @@ int muto_export_paths(muto_handle* h, uint32_t* kept, double* info, uint64_t* of
             }
         };
         fetch(h->L, len, Pn);
-        fetch(h->T, tail, Pn);
+        if (tail && !h->pair_w11.empty()) {  // T holds the weights
+            DevMem tmp;
+            tmp.alloc(std::max<uint64_t>(Pn, 1) * sizeof(double), nullptr);
+            launch_path_tails(h->off.as<uint64_t>(), N, h->L.as<double>(), tmp.as<double>(), s);
+            fetch(tmp, tail, Pn);
+            CK(cudaStreamSynchronize(s));
+        } else {
+            fetch(h->T, tail, Pn);
+        }
         if (info && N) {
             std::vector<double> pr(N);
             CK(cudaMemcpyAsync(pr.data(), h->pr64.as<void>(), N * sizeof(double), cudaMemcpyDeviceToHost, s));
