@@ -485,7 +485,13 @@ void launch_finalize_cost(Counters* ctr, double n_muons, double* hist, uint32_t 
 struct MapParams {
     double beta, p, delta, eps;
     int all_neighbours, add_object_prior, newton_max_iter;
+    double inv_bp;  // 1 / (beta p); NaN without a prior weight (the cubic then has no leading term)
 };
+inline MapParams map_params(double beta, double p, double delta, double eps, bool all_neighbours, bool add_object_prior,
+                            int newton_max_iter) {
+    return MapParams{beta, p, delta, eps, all_neighbours ? 1 : 0, add_object_prior ? 1 : 0, newton_max_iter,
+                     beta * p != 0.0 ? 1.0 / (beta * p) : __builtin_nan("")};
+}
 template <typename LamT>
 void launch_map_voxel(const LamT* last, double* ml_inout, const uint32_t* mult, DevGrid g, MapParams mp,
                       Counters* ctr, cudaStream_t s);

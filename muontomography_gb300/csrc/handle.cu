@@ -1848,7 +1848,7 @@ void enqueue_iteration(muto_handle* h) {
             run(h, "em_update", [&] {
                 launch_fused_update<Real, double>(h, h->lam.as<Real>(), h->lam_ml.as<double>(), nullptr, nullptr, s);
             });
-            MapParams mp{P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter};
+            const MapParams mp = map_params(P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter);
             run(h, "map_voxel", [&] {
                 launch_map_voxel<Real>(h->lam.as<Real>(), h->lam_ml.as<double>(), h->mult.as<uint32_t>(),
                                        make_dev_grid(h->grid), mp, h->ctr(), s);
@@ -1868,7 +1868,7 @@ void enqueue_iteration(muto_handle* h) {
     if (h->method == kMap) {  // ML step into lambda_ML, then the MAP step from the snapshot (src/MutoMAP.cpp:138-184)
         const auto v = voxel_args<Real, double>(h, h->lam.as<Real>(), mode, h->lam_ml.as<double>());
         run(h, "em_voxel", [&] { launch_voxel_pass<Real, double>(h, v, s); });
-        MapParams mp{P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter};
+        const MapParams mp = map_params(P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter);
         run(h, "map_voxel", [&] {
             launch_map_voxel<Real>(h->lam.as<Real>(), h->lam_ml.as<double>(), h->mult.as<uint32_t>(),
                                    make_dev_grid(h->grid), mp, h->ctr(), s);
@@ -2007,7 +2007,7 @@ double nll_eval(muto_handle* h, const double* loglam_host, double* grad_host) {
     }
     const Params& P = h->P;
     if (h->method == kMap) {
-        MapParams mp{P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter};
+        const MapParams mp = map_params(P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter);
         DevMem gdummy;
         double* gp = h->grad.as<double>();
         if (!grad_host) {
