@@ -205,21 +205,23 @@ struct SlrPass {
 void launch_slr_pair_terms(const SlrArgs& a, const SlrPass& p, cudaStream_t s);
 // one later pass, muon after muon
 void launch_slr_iter_pass(const SlrArgs& a, const SlrPass& p, cudaStream_t s);
-// the same pairs in level order: muon q of the level order (order[q]) has
-// its pairs at fo[q] .. fo[q+1]
+// the same pairs (fewer than 2^32) in level order: muon q of the level order
+// (order[q]) has its pairs at fo[q] .. fo[q+1]
 struct SlrFlat {
-    const uint64_t* fo;
+    const uint32_t* fo;
     uint32_t* vox;
-    double* iv0;
+    double* iv0;      // times ein^2 with has_energy
     double* winc;
-    double* e2;
+    uint8_t* place;   // the pair's muon in its step (0 .. kSlrStep-1)
 };
-void launch_slr_flatten(const SlrPass& p, const uint32_t* order, uint64_t nt, const SlrFlat& f, cudaStream_t s);
-// the same pass level by level: level l's muons are q = lstart[l] ..
-// lstart[l+1] of the level order; the image and weight sums are kept in
-// shared memory when 2 V doubles fit in smem_optin bytes
-void launch_slr_iter_levels(const SlrArgs& a, const SlrFlat& f, const uint32_t* lstart, uint32_t levels,
-                            size_t smem_optin, cudaStream_t s);
+constexpr int kSlrStep = 24;  // muons of a step at most (a group of 16 of a block's 384 threads each)
+void launch_slr_flatten(const SlrArgs& a, const SlrPass& p, const uint32_t* order, const uint8_t* place, uint64_t nt,
+                        const SlrFlat& f, cudaStream_t s);
+// the same pass level by level, in steps of one level or part of one: step s's
+// muons are q = sstart[s] .. sstart[s+1] of the level order; the image and
+// weight sums are kept in shared memory when 2 V doubles fit in smem_optin bytes
+void launch_slr_iter_steps(const SlrArgs& a, const SlrFlat& f, const uint32_t* sstart, uint32_t steps,
+                           size_t smem_optin, cudaStream_t s);
 
 // PoCut's per-voxel step (src/MutoPoCut.cpp:113-118), after launch_poca:
 // the kept values grouped by voxel (counts, then offsets, then a scatter of

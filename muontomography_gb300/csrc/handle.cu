@@ -591,8 +591,10 @@ void alloc_counters(muto_handle* h) {
 // The level schedule of SLRIter's later passes (slr_levels.h), made once
 // from the walked paths, which do not change between passes; the muons are
 // then grouped by level (index order inside a level) for the device.
-void slr_level_schedule(muto_handle* h, const DevMem& off, const DevMem& vox, uint64_t nt, uint64_t np, DevMem& order,
-                        DevMem& lstart, DevMem& fo) {
+// sstart: the steps' first muons in level order (a level, or kSlrStep muons of a
+// longer one, a step); returns the number of steps.
+uint32_t slr_level_schedule(muto_handle* h, const DevMem& off, const DevMem& vox, uint64_t nt, uint64_t np,
+                            DevMem& order, DevMem& place, DevMem& sstart, DevMem& fo) {
     const uint64_t V = h->V();
     cudaStream_t s = h->stream;
     if (nt >= 0xffffffffull) throw Error(MUTO_ERR_CAPACITY, "slr_iter: more than 2^32-1 rays");
@@ -611,23 +613,35 @@ void slr_level_schedule(muto_handle* h, const DevMem& off, const DevMem& vox, ui
         start[l] = acc;
         acc += c;
     }
-    // start[l] is now where level l begins (level 0 is empty); the device
-    // reads level l (0-based) at start[l + 1] .. start[l + 2]
+    // start[l] is now where level l begins (level 0 is empty)
     std::vector<uint32_t> cur(start.begin(), start.end());
     for (uint64_t i = 0; i < nt; ++i) order_h[cur[level[i]]++] = static_cast<uint32_t>(i);
     start.push_back(static_cast<uint32_t>(nt));
+    std::vector<uint32_t> steps_h;
+    std::vector<uint8_t> place_h(nt);
+    for (uint32_t l = 1; l <= levels; ++l)
+        for (uint32_t q = start[l]; q < start[l + 1]; ++q) {
+            const uint32_t in = (q - start[l]) % kSlrStep;
+            if (in == 0) steps_h.push_back(q);
+            place_h[q] = static_cast<uint8_t>(in);
+        }
+    const uint32_t steps = static_cast<uint32_t>(steps_h.size());
+    steps_h.push_back(static_cast<uint32_t>(nt));
     // where each muon's pairs go in level order
-    std::vector<uint64_t> fo_h(nt + 1, 0);
-    for (uint64_t q = 0; q < nt; ++q) fo_h[q + 1] = fo_h[q] + (off_h[order_h[q] + 1] - off_h[order_h[q]]);
+    std::vector<uint32_t> fo_h(nt + 1, 0);
+    for (uint64_t q = 0; q < nt; ++q) fo_h[q + 1] = fo_h[q] + static_cast<uint32_t>(off_h[order_h[q] + 1] - off_h[order_h[q]]);
     order.alloc(std::max<uint64_t>(nt, 1) * sizeof(uint32_t), &h->dev_bytes);
-    lstart.alloc(start.size() * sizeof(uint32_t), &h->dev_bytes);
-    fo.alloc((nt + 1) * sizeof(uint64_t), &h->dev_bytes);
+    place.alloc(std::max<uint64_t>(nt, 1), &h->dev_bytes);
+    sstart.alloc(steps_h.size() * sizeof(uint32_t), &h->dev_bytes);
+    fo.alloc((nt + 1) * sizeof(uint32_t), &h->dev_bytes);
     CK(cudaMemcpyAsync(order.as<uint32_t>(), order_h.data(), nt * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(lstart.as<uint32_t>(), start.data() + 1, (start.size() - 1) * sizeof(uint32_t),
-                       cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(fo.as<uint64_t>(), fo_h.data(), (nt + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(place.as<uint8_t>(), place_h.data(), nt, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(sstart.as<uint32_t>(), steps_h.data(), steps_h.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                       s));
+    CK(cudaMemcpyAsync(fo.as<uint32_t>(), fo_h.data(), (nt + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));  // the host vectors go out of scope
     h->slr_levels = levels;
+    return steps;
 }
 
 void prepare_slr(muto_handle* h, uint64_t nt) {
@@ -669,27 +683,30 @@ void prepare_slr(muto_handle* h, uint64_t nt) {
         const SlrPass sp{off.as<uint64_t>(), vox.as<uint32_t>(), len.as<double>(), iv0.as<double>(), winc.as<double>(),
                          e2.as<double>()};
         run(h, "slr_paths", [&] { launch_slr_pair_terms(a, sp, s); });
-        DevMem order, lstart, fo, fvox, fiv0, fwinc, fe2;
+        DevMem order, place, sstart, fo, fvox, fiv0, fwinc, fplace;
         SlrFlat fl{};
-        if (!h->P.slr_sequential) {
+        uint32_t steps = 0;
+        // (2^32 pairs and more: muon after muon, the level order's offsets have 32 bits)
+        const bool by_level = !h->P.slr_sequential && np < 0xffffffffull;
+        if (by_level) {
             {
                 HostPhase ph(h, "slr_levels");
-                slr_level_schedule(h, off, vox, nt, np, order, lstart, fo);
+                steps = slr_level_schedule(h, off, vox, nt, np, order, place, sstart, fo);
             }
             // the pairs copied into level order
             fvox.alloc(std::max<uint64_t>(np, 1) * sizeof(uint32_t), &h->dev_bytes);
             fiv0.alloc(std::max<uint64_t>(np, 1) * sizeof(double), &h->dev_bytes);
             fwinc.alloc(std::max<uint64_t>(np, 1) * sizeof(double), &h->dev_bytes);
-            fe2.alloc(nt * sizeof(double), &h->dev_bytes);
-            fl = SlrFlat{fo.as<uint64_t>(), fvox.as<uint32_t>(), fiv0.as<double>(), fwinc.as<double>(), fe2.as<double>()};
-            run(h, "slr_paths", [&] { launch_slr_flatten(sp, order.as<uint32_t>(), nt, fl, s); });
+            fplace.alloc(std::max<uint64_t>(np, 1), &h->dev_bytes);
+            fl = SlrFlat{fo.as<uint32_t>(), fvox.as<uint32_t>(), fiv0.as<double>(), fwinc.as<double>(), fplace.as<uint8_t>()};
+            run(h, "slr_paths", [&] { launch_slr_flatten(a, sp, order.as<uint32_t>(), place.as<uint8_t>(), nt, fl, s); });
         }
         for (int p = 1; p < passes; ++p)
             run(h, "slr_iter_pass", [&] {
-                if (h->P.slr_sequential)
+                if (!by_level)
                     launch_slr_iter_pass(a, sp, s);
                 else
-                    launch_slr_iter_levels(a, fl, lstart.as<uint32_t>(), h->slr_levels, h->smem_optin, s);
+                    launch_slr_iter_steps(a, fl, sstart.as<uint32_t>(), steps, h->smem_optin, s);
             });
         CK(cudaStreamSynchronize(s));  // the path arrays go out of scope
     }

@@ -6,7 +6,7 @@
 // mean squared projected angle shared by length^2 or equally.  Sums are FP64
 // atomics.  The later passes of the iterative form are order-dependent (each
 // muon sees the image the muons before it left): they run over the walked
-// paths level by level (k_slr_iter_levels: muons of one level share no
+// paths level by level (k_slr_iter_steps: muons of one level share no
 // voxel), or muon after muon on one warp (k_slr_iter_pass).
 #include "common.cuh"
 #include "geometry.cuh"
@@ -183,127 +183,166 @@ __global__ void k_slr_iter_pass(SlrArgs a, SlrPass p) {
 
 // The pairs of every muon copied into level order: muon q of the level
 // order (order[q]) gets its pairs at fo[q] .. fo[q+1], so a level's data is
-// contiguous and found from the level's start alone.  A warp per muon.
-__global__ void k_slr_flatten(SlrPass p, const uint32_t* __restrict__ order, uint64_t nt, SlrFlat f) {
+// contiguous and found from the level's start alone; with ein^2 folded into the
+// image increment (:87-89) and the muon's place in its step (below).  A warp per
+// muon.
+__global__ void k_slr_flatten(SlrPass p, const uint32_t* __restrict__ order, const uint8_t* __restrict__ place,
+                              uint64_t nt, int has_energy, SlrFlat f) {
     const uint64_t q = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (q >= nt) return;
     const uint32_t i = order[q];
     const uint64_t s0 = p.off[i], n = p.off[i + 1] - s0, d0 = f.fo[q];
+    const double e2 = has_energy ? p.e2[i] : 1.0;
     for (uint64_t k = lane; k < n; k += 32) {
         f.vox[d0 + k] = p.vox[s0 + k];
-        f.iv0[d0 + k] = p.iv0[s0 + k];
+        f.iv0[d0 + k] = has_energy ? dmul(p.iv0[s0 + k], e2) : p.iv0[s0 + k];
         f.winc[d0 + k] = p.winc[s0 + k];
+        f.place[d0 + k] = place[q];
     }
-    if (lane == 0) f.e2[q] = p.e2[i];
 }
 
-// One muon of the level order on one warp, the arithmetic of slr_iter_muon;
-// the first pair of each lane (k = lane) comes in already loaded (v0, i0,
-// w0; valid when lane < n), the rest is loaded here.
-__device__ __forceinline__ void slr_flat_muon(const SlrArgs& a, const SlrFlat& f, uint64_t p0, uint32_t n, double e2,
-                                              uint32_t v0, double i0, double w0, int lane, double* img,
-                                              double* weight) {
-    double part = 0.0;  // :49-52, the same order of additions as slr_iter_muon
-    if (static_cast<uint32_t>(lane) < n) part = dadd(part, img[v0]);
-    for (uint32_t k = lane + 32; k < n; k += 32) part = dadd(part, img[f.vox[p0 + k]]);
-    const double total = warp_sum(part);
-    if (static_cast<uint32_t>(lane) < n) {
-        weight[v0] = dadd(weight[v0], w0);
-        double iv = dmul(i0, ddiv(img[v0], total));
-        if (a.has_energy) iv = dmul(iv, e2);  // :87-89
-        img[v0] = dadd(img[v0], iv);
-    }
-    for (uint32_t k = lane + 32; k < n; k += 32) {
-        const uint32_t j = f.vox[p0 + k];
-        weight[j] = dadd(weight[j], f.winc[p0 + k]);
-        double iv = dmul(f.iv0[p0 + k], ddiv(img[j], total));
-        if (a.has_energy) iv = dmul(iv, e2);
-        img[j] = dadd(img[j], iv);
-    }
+// 1 / x for the paths' sums: one third-order step in FP64 from the FP32
+// reciprocal (an error of 2^-23 becomes 2^-66), three dependent operations
+// instead of a division's dozen; outside the FP32 range (and for 0, infinities
+// and NaN) the division.
+__device__ __forceinline__ double slr_reciprocal(double x) {
+    const float f = static_cast<float>(x);
+    if (!(f > 1.0e-30f && f < 1.0e30f)) return ddiv(1.0, x);
+    const double r = static_cast<double>(1.0f / f), e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
 
 // A later pass level by level.  A muon's level is one more than the highest
 // level among the earlier muons that share a voxel with it, so two muons of
 // one level share no voxel, and every voxel meets its muons in index order:
 // each muon reads and writes the image state it would see in the sequential
-// loop, whatever the order inside a level.  One block: its warps take the
-// muons of a level, and the block barrier orders the levels (global stores
-// before it are visible to the whole block after it).  With SMEM the image
-// and weight sums (2 V doubles) are copied into shared memory for the pass
-// and back after it.  The next level's muon offsets are loaded while the
-// current level runs, and its first pair per lane just before the barrier
-// (neither depends on the image).
+// loop, whatever the order inside a level.  One block; a step is a level, or at
+// most kSlrStep muons of a longer one.  In a step
+//   sum     sixteen lanes a muon add up the image on its path (:49-52) and take
+//           the sum's reciprocal;
+//   pairs   a thread per pair adds its weight increment and multiplies its
+//           image increment with the voxel's image (:64-66);
+//   (barrier) the pair adds that product times the reciprocal to its voxel;
+//   (barrier) the next step.
+// Bound by the chain of a step (six FP64 operations in the sum, four with the
+// conversions in the reciprocal, one after it, each about 70 cycles on this
+// part's two FP64 lanes a clock per SM, two barriers) and by that pipe.  20^3
+// voxels, 30 k muons, 2 449 levels: 1.29 us a step; 2.82 us with a warp a muon
+// (a division a pair, a 32-lane sum a muon).  8 and 4 lanes a muon, 512 and 640
+// threads took 1.29 to 1.51 us, 32 lanes 1.95.
+// With SMEM the image and weight sums (2 V doubles) are copied into shared
+// memory for the pass and back after it.  Nothing that a step loads from the
+// lists depends on the image: a step's bounds are loaded five steps ahead,
+// its offsets three, its pairs two.
+constexpr int kSlrThreads = 384;  // a step of the 20^3 grid has about 12 muons and 300 pairs
+constexpr int kSlrLanes = 16;     // of a muon's sum
+static_assert(kSlrThreads / kSlrLanes >= kSlrStep, "a lane group for every muon of a step");
+
 template <bool SMEM>
-__global__ void __launch_bounds__(1024) k_slr_iter_levels(SlrArgs a, SlrFlat f, const uint32_t* __restrict__ lstart,
-                                                          uint32_t levels) {
+__global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFlat f,
+                                                                const uint32_t* __restrict__ sstart, uint32_t steps) {
     extern __shared__ double slr_smem[];
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    __shared__ double s_rec[kSlrStep];
+    constexpr int H = 32 / kSlrLanes;  // pairs of a muon's sum held per lane
+    const int tid = threadIdx.x, l8 = tid % kSlrLanes, slot = tid / kSlrLanes;
     const uint32_t V = a.g.nx * a.g.ny * a.g.nz;
     double* img = a.img;
     double* weight = a.weight;
     if (SMEM) {
         img = slr_smem;
         weight = slr_smem + V;
-        for (uint32_t j = threadIdx.x; j < V; j += blockDim.x) {
+        for (uint32_t j = tid; j < V; j += blockDim.x) {
             img[j] = a.img[j];
             weight[j] = a.weight[j];
         }
         __syncthreads();
     }
-    // this warp's first muon of level 0 and its first pair per lane
-    uint32_t e = lstart[1];
-    uint32_t q = lstart[0] + warp;
-    uint64_t p0 = 0;
-    uint32_t n = 0, v0 = 0;
-    double i0 = 0.0, w0 = 0.0, e2 = 0.0;
-    if (q < e) {
-        p0 = f.fo[q];
-        n = static_cast<uint32_t>(f.fo[q + 1] - p0);
-        e2 = f.e2[q];
-        if (static_cast<uint32_t>(lane) < n) {
-            v0 = f.vox[p0 + lane];
-            i0 = f.iv0[p0 + lane];
-            w0 = f.winc[p0 + lane];
+    // a step's offsets: this lane group's muon [b, e), the step's pairs [p, q)
+    struct Offsets {
+        uint32_t b, e, p, q;
+    };
+    auto offsets = [&](uint32_t q0, uint32_t q1) -> Offsets {  // of the step with muons [q0, q1)
+        Offsets o{0, 0, 0, 0};
+        const uint32_t m = q0 + slot;
+        if (q0 < q1) {
+            o.p = f.fo[q0];
+            o.q = f.fo[q1];
         }
-    }
-    for (uint32_t l = 0; l < levels; ++l) {
-        // the next level's first muon for this warp: its offsets now
-        const uint32_t en = l + 1 < levels ? lstart[l + 2] : e;
-        const uint32_t qn = e + warp;
-        const bool has_next = l + 1 < levels && qn < en;
-        uint64_t p0n = 0, p1n = 0;
-        if (has_next) {
-            p0n = f.fo[qn];
-            p1n = f.fo[qn + 1];
+        if (m < q1) {
+            o.b = f.fo[m];
+            o.e = f.fo[m + 1];
         }
-        if (q < e) slr_flat_muon(a, f, p0, n, e2, v0, i0, w0, lane, img, weight);
-        for (uint32_t q2 = q + nw; q2 < e; q2 += nw) {  // more muons than warps in this level
-            const uint64_t s0 = f.fo[q2];
-            const uint32_t m = static_cast<uint32_t>(f.fo[q2 + 1] - s0);
-            const bool in = static_cast<uint32_t>(lane) < m;
-            slr_flat_muon(a, f, s0, m, f.e2[q2], in ? f.vox[s0 + lane] : 0u, in ? f.iv0[s0 + lane] : 0.0,
-                          in ? f.winc[s0 + lane] : 0.0, lane, img, weight);
+        return o;
+    };
+    struct Pairs {
+        uint32_t v[H];  // the muon's sum
+        uint32_t j;     // this thread's pair
+        uint32_t place;
+        double iv0, winc;
+    };
+    auto pairs = [&](const Offsets& o) -> Pairs {
+        Pairs r{};
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+            if (o.b + l8 + h * kSlrLanes < o.e) r.v[h] = f.vox[o.b + l8 + h * kSlrLanes];
+        if (o.p + tid < o.q) {
+            r.j = f.vox[o.p + tid];
+            r.place = f.place[o.p + tid];
+            r.iv0 = f.iv0[o.p + tid];
+            r.winc = f.winc[o.p + tid];
         }
-        // the next level's first pair per lane, before the barrier
-        q = qn;
-        e = en;
-        n = 0;
-        if (has_next) {
-            p0 = p0n;
-            n = static_cast<uint32_t>(p1n - p0n);
-            e2 = f.e2[qn];
-            if (static_cast<uint32_t>(lane) < n) {
-                v0 = f.vox[p0 + lane];
-                i0 = f.iv0[p0 + lane];
-                w0 = f.winc[p0 + lane];
-            }
+        return r;
+    };
+    auto first = [&](uint32_t s) -> uint32_t { return sstart[min(s, steps)]; };
+    uint32_t q1 = first(1), q2 = first(2), q3 = first(3), q4 = first(4);
+    Offsets o = offsets(first(0), q1), o1 = offsets(q1, q2), o2 = offsets(q2, q3);
+    Pairs c = pairs(o), c1 = pairs(o1);
+    for (uint32_t s = 0; s < steps; ++s) {
+        if (__any_sync(kFull, o.b < o.e)) {
+            double w[H];
+#pragma unroll
+            for (int h = 0; h < H; ++h) w[h] = o.b + l8 + h * kSlrLanes < o.e ? img[c.v[h]] : 0.0;
+#pragma unroll
+            for (int d = H / 2; d > 0; d >>= 1)
+#pragma unroll
+                for (int h = 0; h < d; ++h) w[h] = dadd(w[h], w[h + d]);
+            double part = w[0];
+            for (uint32_t k = o.b + l8 + H * kSlrLanes; k < o.e; k += kSlrLanes) part = dadd(part, img[f.vox[k]]);
+            __syncwarp();
+#pragma unroll
+            for (int d = kSlrLanes / 2; d > 0; d >>= 1) part = dadd(part, __shfl_xor_sync(kFull, part, d));
+            if (l8 == 0 && o.b < o.e) s_rec[slot] = slr_reciprocal(part);
+        }
+        const bool mine = o.p + tid < o.q;
+        double x = 0.0, inc = 0.0;
+        if (mine) {
+            x = img[c.j];
+            inc = dmul(c.iv0, x);
+            weight[c.j] = dadd(weight[c.j], c.winc);
+        }
+        // the lists' loads for the steps to come, while the sums' last operations run
+        const Pairs c2 = pairs(o2);
+        const Offsets o3 = offsets(q3, q4);
+        q3 = q4;
+        q4 = first(s + 5);
+        __syncthreads();
+        if (mine) img[c.j] = fma(inc, s_rec[c.place], x);
+        for (uint32_t k = o.p + tid + kSlrThreads; k < o.q; k += kSlrThreads) {  // more pairs than threads
+            const uint32_t j = f.vox[k];
+            const double xk = img[j];
+            weight[j] = dadd(weight[j], f.winc[k]);
+            img[j] = fma(dmul(f.iv0[k], xk), s_rec[f.place[k]], xk);
         }
         __syncthreads();
+        o = o1;
+        o1 = o2;
+        o2 = o3;
+        c = c1;
+        c1 = c2;
     }
     if (SMEM) {
-        for (uint32_t j = threadIdx.x; j < V; j += blockDim.x) {
+        for (uint32_t j = tid; j < V; j += blockDim.x) {
             a.img[j] = img[j];
             a.weight[j] = weight[j];
         }
@@ -337,23 +376,24 @@ void launch_slr_iter_pass(const SlrArgs& a, const SlrPass& p, cudaStream_t s) {
     count_launches(1);
 }
 
-void launch_slr_flatten(const SlrPass& p, const uint32_t* order, uint64_t nt, const SlrFlat& f, cudaStream_t s) {
+void launch_slr_flatten(const SlrArgs& a, const SlrPass& p, const uint32_t* order, const uint8_t* place, uint64_t nt,
+                        const SlrFlat& f, cudaStream_t s) {
     if (nt == 0) return;
-    k_slr_flatten<<<static_cast<unsigned>((nt * 32 + 255) / 256), 256, 0, s>>>(p, order, nt, f);
+    k_slr_flatten<<<static_cast<unsigned>((nt * 32 + 255) / 256), 256, 0, s>>>(p, order, place, nt, a.has_energy, f);
     count_launches(1);
 }
 
-void launch_slr_iter_levels(const SlrArgs& a, const SlrFlat& f, const uint32_t* lstart, uint32_t levels,
-                            size_t smem_optin, cudaStream_t s) {
-    if (a.n == 0 || levels == 0) return;
+void launch_slr_iter_steps(const SlrArgs& a, const SlrFlat& f, const uint32_t* sstart, uint32_t steps,
+                           size_t smem_optin, cudaStream_t s) {
+    if (a.n == 0 || steps == 0) return;
     const size_t bytes = 2 * sizeof(double) * static_cast<size_t>(a.g.nx) * a.g.ny * a.g.nz;
-    if (bytes <= smem_optin &&
-        cudaFuncSetAttribute(k_slr_iter_levels<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (bytes + kSlrStep * sizeof(double) + 1024 <= smem_optin &&
+        cudaFuncSetAttribute(k_slr_iter_steps<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(bytes)) == cudaSuccess) {
-        k_slr_iter_levels<true><<<1, 1024, bytes, s>>>(a, f, lstart, levels);
+        k_slr_iter_steps<true><<<1, kSlrThreads, bytes, s>>>(a, f, sstart, steps);
     } else {
         (void)cudaGetLastError();  // a refused attribute: the pass stays in global memory
-        k_slr_iter_levels<false><<<1, 1024, 0, s>>>(a, f, lstart, levels);
+        k_slr_iter_steps<false><<<1, kSlrThreads, 0, s>>>(a, f, sstart, steps);
     }
     count_launches(1);
 }
