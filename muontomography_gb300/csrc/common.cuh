@@ -117,14 +117,17 @@ void launch_path_fill(const muto_ray* rays, const uint32_t* kept, const double* 
 // into scratch sized for the chunk alone.
 void launch_path_bound(const muto_ray* rays, const uint32_t* kept, const double* scat, uint64_t n, muto_grid g,
                        int straight, uint32_t* bounds, cudaStream_t s);
-template <typename Real>
-void launch_path_fill_bounded(const muto_ray* rays, const uint32_t* kept, const double* scat, const uint64_t* boff,
-                              uint64_t slot_base, uint64_t n, muto_grid g, int straight, uint32_t* vidx, double* l64,
-                              Real* L, Real* T, uint32_t* counts, Counters* ctr, cudaStream_t s);
-template <typename Real>
+// (T: the FP64 lists' tails, or null)
+void launch_path_walk(const muto_ray* rays, const uint32_t* kept, const double* scat, const uint64_t* boff,
+                      uint64_t slot_base, uint64_t n, muto_grid g, int straight, uint32_t* vidx, double* l64, double* T,
+                      uint32_t* counts, Counters* ctr, cudaStream_t s);
+// the walked slots to the exact slots off: the mixed form's lists with their tails
+void launch_path_finish(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
+                        const uint32_t* vidx_b, const double* l64, uint32_t* vidx, float* L, float* T, cudaStream_t s);
+// and the FP64 form's
 void launch_path_compact(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
-                         const uint32_t* vidx_b, const Real* L_b, const Real* T_b, uint32_t* vidx, Real* L, Real* T,
-                         cudaStream_t s);
+                         const uint32_t* vidx_b, const double* L_b, const double* T_b, uint32_t* vidx, double* L,
+                         double* T, cudaStream_t s);
 // scan-local voxel indices j < V_scan become voff + j; others become 0xffffffff
 void launch_offset_voxels(uint32_t* vidx, uint64_t n, uint32_t v_scan, uint32_t voff, cudaStream_t s);
 void launch_voxel_hist(const uint32_t* vidx, uint64_t P, uint32_t V, uint32_t* mult, Counters* ctr, cudaStream_t s);

@@ -19,13 +19,20 @@ struct DevGrid {
     uint32_t n[3];
     double lo[3];
     double w[3];
+    double rw[3];   // 1 / w
+    int ordinary;   // every lo and w of a magnitude for which quotient() is exact
 };
 
-__host__ __device__ inline DevGrid make_dev_grid(const muto_grid& g) {
+inline DevGrid make_dev_grid(const muto_grid& g) {
     DevGrid d;
     d.n[0] = g.nx; d.n[1] = g.ny; d.n[2] = g.nz;
     d.lo[0] = g.x_min; d.lo[1] = g.y_min; d.lo[2] = g.z_min;
     d.w[0] = g.dx; d.w[1] = g.dy; d.w[2] = g.dz;
+    d.ordinary = 1;
+    for (int k = 0; k < 3; ++k) {
+        d.rw[k] = 1.0 / d.w[k];
+        if (!(d.w[k] > 1e-100 && d.w[k] < 1e100 && d.lo[k] > -1e100 && d.lo[k] < 1e100)) d.ordinary = 0;
+    }
     return d;
 }
 
@@ -33,6 +40,24 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
+// a / b, correctly rounded, from y = 1 / b correctly rounded: the product a y
+// corrected by its remainder twice (Markstein's theorem: the second correction of
+// a faithful quotient is the rounded quotient; the remainders are exact).  Five
+// FP64 operations where several quotients share a divisor, against about twenty
+// for a division; for operands within 1e-100 .. 1e100 (or a = 0), so that no
+// product or remainder leaves the range.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    const double q1 = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q1, b, a), y, q1);
+}
+__device__ __forceinline__ double positive_zero(double x) {  // -0.0 as 0.0
+    const long long b = __double_as_longlong(x);
+    return __longlong_as_double((b << 1) == 0 ? 0ll : b);
+}
+__device__ __forceinline__ bool ordinary(double x) {  // finite and below about 1e100
+    return (__double2hiint(x) & 0x7fffffff) < 0x54b00000;
+}
 // std::max / std::min argument semantics
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
@@ -88,19 +113,120 @@ __device__ __forceinline__ uint32_t walk_bound(const DevGrid& g, const double* a
     return n;
 }
 
+// The steps of a walk (src/MutoSiddon.cpp:108-138) from the first crossings on.
+// INTS: every value non-negative and finite, compared by bit pattern; three FP64
+// operations a step (the crossing stepped to, the difference, the length).
+template <bool INTS, class Sink>
+__device__ __forceinline__ int siddon_steps(const DevGrid& g, uint32_t (&idx)[3], const int (&dir)[3], double (&an)[3],
+                                            const double (&da)[3], double alpha, double amax, double seg, Sink& sink) {
+    const double eps = 1.0e-6;  // :19
+    const long long amax_b = dbits(amax), eps_b = dbits(eps);
+    double alpha_last = alpha;
+    int count = 0;
+    int left = siddon_step_bound(g);
+    // The lanes of a warp that walk together step together: every iteration
+    // ends with a ballot over the lanes still walking, which makes it a
+    // reconvergence point (the three-way step below would otherwise let the
+    // lanes drift apart for the rest of the walk, each then issuing its own
+    // FP64 instructions).
+    unsigned live = __activemask();
+    bool more = INTS ? dbits(alpha) < amax_b : alpha < amax;
+    live = __ballot_sync(live, more);
+    while (more) {
+        const uint32_t vx = idx[0], vy = idx[1], vz = idx[2];
+        // min of the three next crossings, reference tie-break order
+        bool t0, t1;
+        if (INTS) {
+            const long long b0 = dbits(an[0]), b1 = dbits(an[1]), b2 = dbits(an[2]);
+            t0 = b0 < b1 && b0 < b2;
+            t1 = b1 < b2;
+        } else {
+            t0 = an[0] < an[1] && an[0] < an[2];
+            t1 = an[1] < an[2];
+        }
+        // the axis stepped, then one FP64 add for it: the lanes of a warp step
+        // along different axes, and a branch per axis would issue the add
+        // once per axis taken in the warp (selects are integer instructions)
+        const int k = t0 ? 0 : (t1 ? 1 : 2);
+        const double ak = k == 0 ? an[0] : (k == 1 ? an[1] : an[2]);
+        const double dk = k == 0 ? da[0] : (k == 1 ? da[1] : da[2]);
+        const double next = dadd(ak, dk);
+        an[0] = k == 0 ? next : an[0];
+        an[1] = k == 1 ? next : an[1];
+        an[2] = k == 2 ? next : an[2];
+        idx[0] += k == 0 ? static_cast<uint32_t>(dir[0]) : 0u;
+        idx[1] += k == 1 ? static_cast<uint32_t>(dir[1]) : 0u;
+        idx[2] += k == 2 ? static_cast<uint32_t>(dir[2]) : 0u;
+        // not yet at the end: the next step's test, and min(alpha, amax) here
+        const bool before = INTS ? dbits(ak) < amax_b : ak < amax;
+        const double upto = INTS ? (before ? ak : amax) : smin(ak, amax);
+        const double dalpha = dsub(upto, alpha_last);
+        if (INTS ? eps_b < dbits(dalpha) : eps < dalpha) {  // eps is positive
+            sink(vx, vy, vz, dmul(dalpha, seg));
+            ++count;
+            alpha_last = ak;
+        }
+        more = before && --left > 0;  // the step bound: never for a walk that ends
+        if (before && !more) count = -1;
+        live = __ballot_sync(live, more);
+    }
+    return count;
+}
+
+// ORDINARY: coordinates and grid of ordinary magnitudes (the divisions go
+// through quotient, the steps' comparisons through integers where they can).
+template <bool ORDINARY, class Sink>
+__device__ __forceinline__ int siddon_walk_as(const DevGrid& g, const double* p1, const double* p2, Sink& sink);
+
+// Anything else, and the rare walk with a negative crossing: out of line, the
+// sink by value, so that the common walk's state stays in registers.
+template <class Sink>
+struct Walked {
+    Sink sink;
+    int count;
+};
+template <class Sink>
+__device__ __noinline__ Walked<Sink> siddon_walk_any(DevGrid g, double3 a, double3 b, Sink sink) {
+    const double p1[3] = {a.x, a.y, a.z}, p2[3] = {b.x, b.y, b.z};
+    const int n = siddon_walk_as<false>(g, p1, p2, sink);
+    return Walked<Sink>{sink, n};
+}
+
 template <class Sink>
 __device__ __forceinline__ int siddon_walk(const DevGrid& g, const double* p1, const double* p2, Sink& sink) {
+    int n = -2;
+    if (g.ordinary && ordinary(p1[0]) && ordinary(p1[1]) && ordinary(p1[2]) && ordinary(p2[0]) && ordinary(p2[1]) &&
+        ordinary(p2[2]))
+        n = siddon_walk_as<true>(g, p1, p2, sink);
+    if (n == -2) {
+        const Walked<Sink> w = siddon_walk_any(g, make_double3(p1[0], p1[1], p1[2]), make_double3(p2[0], p2[1], p2[2]), sink);
+        sink = w.sink;
+        n = w.count;
+    }
+    return n;
+}
+
+// (returns -2, before the sink has seen anything, where ORDINARY does not hold)
+template <bool ORDINARY, class Sink>
+__device__ __forceinline__ int siddon_walk_as(const DevGrid& g, const double* p1, const double* p2, Sink& sink) {
     const double eps = 1.0e-6;  // :19
-    double d[3], first[3], last[3];
+    double d[3], first[3], last[3], y[3];
     for (int k = 0; k < 3; ++k) d[k] = dsub(p2[k], p1[k]);
     const double seg = __dsqrt_rn(dot3(d, d));  // :14
 #pragma unroll
     for (int k = 0; k < 3; ++k) {  // :25-48
         double a0 = -0.1, an = 1.1;
         const double hi = dadd(g.lo[k], dmul(g.w[k], static_cast<double>(g.n[k])));
+        y[k] = 0.0;
         if (eps < fabs(d[k])) {
-            a0 = ddiv(dsub(g.lo[k], p1[k]), d[k]);
-            an = ddiv(dsub(hi, p1[k]), d[k]);
+            if (ORDINARY) {
+                y[k] = __drcp_rn(d[k]);
+                a0 = quotient(dsub(g.lo[k], p1[k]), d[k], y[k]);
+                an = quotient(dsub(hi, p1[k]), d[k], y[k]);
+            } else {
+                a0 = ddiv(dsub(g.lo[k], p1[k]), d[k]);
+                an = ddiv(dsub(hi, p1[k]), d[k]);
+            }
         } else if (p1[k] < g.lo[k] || hi <= p1[k]) {
             return 0;
         }
@@ -118,11 +244,12 @@ __device__ __forceinline__ int siddon_walk(const DevGrid& g, const double* p1, c
 #pragma unroll
     for (int k = 0; k < 3; ++k) {  // :62-81
         const double nudge = (d[k] <= 0) ? -eps : eps;
-        idx[k] = u32_cast_x86(dadd(ddiv(dsub(dadd(dmul(alpha, d[k]), p1[k]), g.lo[k]), g.w[k]), nudge));
+        const double at = dsub(dadd(dmul(alpha, d[k]), p1[k]), g.lo[k]);
+        idx[k] = u32_cast_x86(dadd(ORDINARY ? quotient(at, g.w[k], g.rw[k]) : ddiv(at, g.w[k]), nudge));
         dir[k] = 0;
         da[k] = 0.0;
         if (eps < fabs(d[k])) {
-            da[k] = ddiv(g.w[k], fabs(d[k]));
+            da[k] = ORDINARY ? quotient(g.w[k], fabs(d[k]), fabs(y[k])) : ddiv(g.w[k], fabs(d[k]));
             dir[k] = d[k] < 0 ? -1 : 1;
         }
     }
@@ -133,65 +260,21 @@ __device__ __forceinline__ int siddon_walk(const DevGrid& g, const double* p1, c
             an[k] = dadd(amin, da[k]);
         } else if (dir[k] != 0) {
             const double plane = dsub(dadd(dmul(static_cast<double>(idx[k]), g.w[k]), g.lo[k]), p1[k]);
-            an[k] = dadd(ddiv(plane, d[k]), dir[k] == 1 ? da[k] : 0.0);
+            an[k] = dadd(ORDINARY ? quotient(plane, d[k], y[k]) : ddiv(plane, d[k]), dir[k] == 1 ? da[k] : 0.0);
         }
     }
-    double alpha_last = alpha;
-    int count = 0;
-    const int bound = siddon_step_bound(g);
-    int steps = 0;
-    // integer compares need finite values (then every later crossing is finite too)
-    const bool fast = isfinite(alpha) && isfinite(amax) && isfinite(an[0]) && isfinite(an[1]) && isfinite(an[2]);
-    const long long amax_b = fast ? dbits(amax) : -1, eps_b = dbits(eps);
-    // The lanes of a warp that walk together step together: every iteration
-    // starts with a ballot over the lanes still walking, which makes it a
-    // reconvergence point (the three-way step below would otherwise let the
-    // lanes drift apart for the rest of the walk, each then issuing its own
-    // FP64 instructions).
-    unsigned live = __activemask();
-    for (;;) {  // :108-138
-        const long long alpha_b = fast ? dbits(alpha) : -1;
-        const bool more = (alpha_b | amax_b) >= 0 ? alpha_b < amax_b : alpha < amax;
-        const bool over = more && steps >= bound;  // the step bound: never for a walk that ends
-        live = __ballot_sync(live, more && !over);
-        if (!more) break;
-        if (over) return -1;
-        ++steps;
-        const uint32_t vx = idx[0], vy = idx[1], vz = idx[2];
-        // min of the three next crossings, reference tie-break order
-        const long long b0 = fast ? dbits(an[0]) : -1, b1 = dbits(an[1]), b2 = dbits(an[2]);
-        bool t0, t1;
-        if ((b0 | b1 | b2) >= 0) {
-            t0 = b0 < b1 && b0 < b2;
-            t1 = b1 < b2;
-        } else {
-            t0 = an[0] < an[1] && an[0] < an[2];
-            t1 = an[1] < an[2];
-        }
-        // the axis stepped, then one FP64 add for it: the lanes of a warp step
-        // along different axes, and a branch per axis would issue the add
-        // once per axis taken in the warp (selects are integer instructions)
-        const int k = t0 ? 0 : (t1 ? 1 : 2);
-        const double ak = k == 0 ? an[0] : (k == 1 ? an[1] : an[2]);
-        const double dk = k == 0 ? da[0] : (k == 1 ? da[1] : da[2]);
-        const double next = dadd(ak, dk);
-        alpha = ak;
-        an[0] = k == 0 ? next : an[0];
-        an[1] = k == 1 ? next : an[1];
-        an[2] = k == 2 ? next : an[2];
-        idx[0] += k == 0 ? static_cast<uint32_t>(dir[0]) : 0u;
-        idx[1] += k == 1 ? static_cast<uint32_t>(dir[1]) : 0u;
-        idx[2] += k == 2 ? static_cast<uint32_t>(dir[2]) : 0u;
-        const long long ab = dbits(alpha);
-        const double upto = (ab | amax_b) >= 0 ? (amax_b < ab ? amax : alpha) : smin(alpha, amax);
-        const double dalpha = dsub(upto, alpha_last);
-        if (fast ? eps_b < dbits(dalpha) : eps < dalpha) {  // eps is positive
-            sink(vx, vy, vz, dmul(dalpha, seg));
-            ++count;
-            alpha_last = alpha;
-        }
-    }
-    return count;
+    // Every crossing finite and every sign bit clear (the crossings only grow):
+    // the steps' comparisons then run on the integer pipe.  A track that starts
+    // on the grid's top plane has a first crossing of -0.0, which stands for 0.0
+    // in every operation to come.
+    alpha = positive_zero(alpha);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) an[k] = positive_zero(an[k]);
+    if (!ORDINARY) return siddon_steps<false>(g, idx, dir, an, da, alpha, amax, seg, sink);
+    if (!(isfinite(amax) && isfinite(an[0]) && isfinite(an[1]) && isfinite(an[2]) &&
+          (dbits(alpha) | dbits(amax) | dbits(an[0]) | dbits(an[1]) | dbits(an[2])) >= 0))
+        return -2;
+    return siddon_steps<true>(g, idx, dir, an, da, alpha, amax, seg, sink);
 }
 
 // Point of closest approach of the in and out lines (src/MutoMLSD.cpp:328-348,
@@ -209,8 +292,16 @@ __device__ __forceinline__ bool poca_point(const muto_ray& r, double eps, double
         for (int k = 0; k < 3; ++k) out[k] = dmul(0.5, dadd(r.pin[k], r.pout[k]));
         return false;
     }
-    const double cin = ddiv(dsub(dmul(b, e), dmul(c, d)), den);
-    const double cout = ddiv(dsub(dmul(a, e), dmul(b, d)), den);
+    const double ni = dsub(dmul(b, e), dmul(c, d)), no = dsub(dmul(a, e), dmul(b, d));
+    double cin, cout;
+    if (ordinary(ni) && ordinary(no) && ordinary(den) && fabs(den) > 1e-100) {
+        const double y = __drcp_rn(den);
+        cin = quotient(ni, den, y);
+        cout = quotient(no, den, y);
+    } else {
+        cin = ddiv(ni, den);
+        cout = ddiv(no, den);
+    }
     for (int k = 0; k < 3; ++k)
         out[k] = dmul(0.5, dadd(dadd(dadd(r.pin[k], dmul(cin, r.din[k])), r.pout[k]), dmul(cout, r.dout[k])));
     return true;
@@ -229,22 +320,23 @@ __device__ __forceinline__ double scat_angle_square(const double* d1, const doub
     return ddiv(dadd(dmul(axz, axz), dmul(ayz, ayz)), 2.0);
 }
 
-// Displacement in the xz and yz planes (src/MutoMLSD.cpp:356-376)
+// Displacement in the xz and yz planes (src/MutoMLSD.cpp:356-376): with the
+// lines' slopes t = tan(angle) = d_x / d_z, the reference's
+//   (x_out - x_in) cos(a_in) l_xy cos(a_out) / cos(a_out - a_in)
+// is (x_out - x_in) l_xy / (1 + t_in t_out).  The difference, which cancels, is
+// formed in the reference's order.
 __device__ __forceinline__ void displacement(const muto_ray& r, double z_min, double* dxz, double* dyz) {
-    const double axin = atan2(r.din[0], r.din[2]);
-    const double axout = atan2(r.dout[0], r.dout[2]);
-    const double ayin = atan2(r.din[1], r.din[2]);
-    const double ayout = atan2(r.dout[1], r.dout[2]);
     const double sin_ = ddiv(dsub(z_min, r.pin[2]), r.din[2]);
     const double sout = ddiv(dsub(z_min, r.pout[2]), r.dout[2]);
     const double xp = dadd(r.pin[0], dmul(sin_, r.din[0]));
     const double yp = dadd(r.pin[1], dmul(sin_, r.din[1]));
     const double xt = dadd(r.pout[0], dmul(sout, r.dout[0]));
     const double yt = dadd(r.pout[1], dmul(sout, r.dout[1]));
-    const double tx = tan(axin), ty = tan(ayin);
-    const double lxy = __dsqrt_rn(dadd(dadd(1.0, dmul(tx, tx)), dmul(ty, ty)));
-    *dxz = ddiv(dmul(dmul(dmul(dsub(xt, xp), cos(axin)), lxy), cos(axout)), cos(dsub(axout, axin)));
-    *dyz = ddiv(dmul(dmul(dmul(dsub(yt, yp), cos(ayin)), lxy), cos(ayout)), cos(dsub(ayout, ayin)));
+    const double yi = 1.0 / r.din[2], yo = 1.0 / r.dout[2];
+    const double tx = r.din[0] * yi, ty = r.din[1] * yi, ox = r.dout[0] * yo, oy = r.dout[1] * yo;
+    const double lxy = sqrt(fma(tx, tx, fma(ty, ty, 1.0)));
+    *dxz = dsub(xt, xp) * lxy / fma(tx, ox, 1.0);
+    *dyz = dsub(yt, yp) * lxy / fma(ty, oy, 1.0);
 }
 
 }  // namespace muto

@@ -845,7 +845,7 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
     cudaStream_t s = h->stream;
     const uint64_t N = h->N;
     const size_t S = h->scans.size();
-    const bool real64 = std::is_same<Real, double>::value;
+    constexpr bool real64 = std::is_same<Real, double>::value;
     HostPhase ph(h, "fill");
     DevMem boff;
     boff.alloc((N + 1) * sizeof(uint64_t), &h->dev_bytes);
@@ -858,19 +858,17 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
     h->vidx.alloc((Pb + kPad) * sizeof(uint32_t), &h->dev_bytes);
     h->L.alloc((Pb + kPad) * sizeof(Real), &h->dev_bytes);
     h->T.alloc((Pb + kPad) * sizeof(Real), &h->dev_bytes);
-    // one chunk's bounded slots: voxel, FP64 length (tails are summed in FP64), L, T
-    const uint64_t per_pair = sizeof(uint32_t) + sizeof(double) + (real64 ? 0 : sizeof(Real)) + sizeof(Real);
+    // one chunk's bounded slots: voxel, FP64 length, and the FP64 form's tail
+    const uint64_t per_pair = sizeof(uint32_t) + sizeof(double) + (real64 ? sizeof(double) : 0);
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
     const uint64_t budget = std::min<uint64_t>(free_b / 4, uint64_t(12) << 30);
     uint64_t cap = std::min<uint64_t>(std::max<uint64_t>(Pb, 1), std::max<uint64_t>(budget / per_pair, uint64_t(1) << 20));
     if (P.setup_chunk_pairs > 0) cap = static_cast<uint64_t>(P.setup_chunk_pairs);
-    DevMem vidx_b, l64_b, L_b, T_b;
+    DevMem vidx_b, l64_b, T_b;
     vidx_b.alloc((cap + kPad) * sizeof(uint32_t), &h->dev_bytes);
     l64_b.alloc((cap + kPad) * sizeof(double), &h->dev_bytes);
-    if (!real64) L_b.alloc((cap + kPad) * sizeof(Real), &h->dev_bytes);
-    T_b.alloc((cap + kPad) * sizeof(Real), &h->dev_bytes);
-    Real* Lb = real64 ? reinterpret_cast<Real*>(l64_b.as<double>()) : L_b.as<Real>();
+    if (real64) T_b.alloc((cap + kPad) * sizeof(double), &h->dev_bytes);
     const double avg = N ? static_cast<double>(Pb) / static_cast<double>(N) : 1.0;
     const uint64_t chunk0 = std::max<uint64_t>(P.setup_chunk_pairs > 0 ? 1 : 1024,
                                                static_cast<uint64_t>(static_cast<double>(cap) / (1.25 * avg + 1.0)));
@@ -890,19 +888,23 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
             }
             if (b[1] - b[0] > cap) throw Error(MUTO_ERR_CAPACITY, "a muon's path bound exceeds the set-up scratch");
             run(h, "siddon_fill", [&] {
-                launch_path_fill_bounded<Real>(h->scan_rays(k), h->kept.as<uint32_t>() + m, h->scat.as<double>() + 3 * m,
-                                               boff.as<uint64_t>() + m, b[0], nc, sc.grid, P.straight_line,
-                                               vidx_b.as<uint32_t>(), l64_b.as<double>(), Lb, T_b.as<Real>(),
-                                               counts.as<uint32_t>() + m, h->ctr(), s);
+                launch_path_walk(h->scan_rays(k), h->kept.as<uint32_t>() + m, h->scat.as<double>() + 3 * m,
+                                 boff.as<uint64_t>() + m, b[0], nc, sc.grid, P.straight_line, vidx_b.as<uint32_t>(),
+                                 l64_b.as<double>(), T_b.as<double>(), counts.as<uint32_t>() + m, h->ctr(), s);
             });
             run(h, "scan", [&] {
                 scan_u32_to_u64(counts.as<uint32_t>() + m, h->off.as<uint64_t>() + m, nc, scratch.as<void>(), s);
                 launch_add_u64(h->off.as<uint64_t>() + m, nc + 1, base, s);
             });
             run(h, "path_compact", [&] {
-                launch_path_compact<Real>(boff.as<uint64_t>() + m, b[0], h->off.as<uint64_t>() + m, nc,
-                                          vidx_b.as<uint32_t>(), Lb, T_b.as<Real>(), h->vidx.as<uint32_t>(),
-                                          h->L.as<Real>(), h->T.as<Real>(), s);
+                if constexpr (real64)
+                    launch_path_compact(boff.as<uint64_t>() + m, b[0], h->off.as<uint64_t>() + m, nc,
+                                        vidx_b.as<uint32_t>(), l64_b.as<double>(), T_b.as<double>(),
+                                        h->vidx.as<uint32_t>(), h->L.as<Real>(), h->T.as<Real>(), s);
+                else
+                    launch_path_finish(boff.as<uint64_t>() + m, b[0], h->off.as<uint64_t>() + m, nc,
+                                       vidx_b.as<uint32_t>(), l64_b.as<double>(), h->vidx.as<uint32_t>(),
+                                       h->L.as<Real>(), h->T.as<Real>(), s);
             });
             CK(cudaMemcpyAsync(&base, h->off.as<uint64_t>() + m + nc, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
@@ -911,7 +913,6 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
     }
     vidx_b.release();
     l64_b.release();
-    L_b.release();
     T_b.release();
     boff.release();
     unsigned long long over_bound = 0;

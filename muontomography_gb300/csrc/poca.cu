@@ -1,7 +1,8 @@
 // PoCA reconstruction (MutoPoCA::reconstruct, src/MutoPoCA.cpp:51-134): a
-// thread per ray for the PoCA point, mean squared angle, unsigned-cast binning
-// with the reference's reject test and the image sum; then a thread per kept
-// ray for the Siddon weights of the in and out halves (or the straight line).
+// thread per ray for the PoCA point, the unsigned-cast binning and the
+// reference's reject test; then a thread per kept ray for the mean squared angle,
+// the image sum and the Siddon weights of the in and out halves (or the straight
+// line).
 // Sums are FP64 atomics; the voxel each ray is binned to is bit-exact with
 // the reference.
 //
@@ -31,8 +32,7 @@ struct WeightSink {
     }
 };
 
-// Per ray: PoCA point, value and binning; the image sum (or PoCut's value
-// and voxel); kept rays are appended to a.walk (warp-aggregated) for the
+// Per ray: PoCA point and binning (PoCut's voxel); kept rays are appended to a.walk (warp-aggregated) for the
 // walk kernel, so that the FP64 walks run on full warps (a warp of rays
 // usually keeps fewer than half of them, and an FP64 instruction takes the
 // same pipe time however few of its lanes are active), with a bound on each
@@ -40,18 +40,19 @@ struct WeightSink {
 __device__ __forceinline__ bool poca_bin(const DevGrid& g, const muto_ray& r, double eps, double zmin, double zmax,
                                          double* ps, uint32_t* xyz, bool* parallel_ok) {
     *parallel_ok = poca_point(r, eps, ps);
-    xyz[0] = u32_cast_x86(ddiv(dsub(ps[0], g.lo[0]), g.w[0]));  // :121-123
-    xyz[1] = u32_cast_x86(ddiv(dsub(ps[1], g.lo[1]), g.w[1]));
-    xyz[2] = u32_cast_x86(ddiv(dsub(ps[2], g.lo[2]), g.w[2]));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // :121-123 (an infinite quotient and a NaN both cast to 0)
+        const double at = dsub(ps[k], g.lo[k]);
+        xyz[k] = u32_cast_x86(g.ordinary ? quotient(at, g.w[k], g.rw[k]) : ddiv(at, g.w[k]));
+    }
     return !(g.n[0] <= xyz[0] || g.n[1] <= xyz[1] || g.n[2] <= xyz[2] || ps[2] < zmin || zmax < ps[2]);  // :125-129
 }
 
-__global__ void k_poca(PocaArgs a) {
+__global__ void __launch_bounds__(128) k_poca(PocaArgs a, DevGrid g) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     bool parallel_ok = false, kept = false;
     uint32_t wlen = 0;  // a bound on the kept ray's walk, for the walk list's order
     if (i < a.n) {
-        const DevGrid g = make_dev_grid(a.g);
         const muto_ray r = a.rays[i];
         const double zmin = a.rays[0].pout[2], zmax = a.rays[0].pin[2];  // :111-112
         double ps[3];
@@ -64,19 +65,10 @@ __global__ void k_poca(PocaArgs a) {
             a.assign[3 * i + 1] = kept ? static_cast<long long>(xyz[1]) : -1;
             a.assign[3 * i + 2] = kept ? static_cast<long long>(xyz[2]) : -1;
         }
-        if (a.vox) a.vox[i] = 0xffffffffu;
-        if (kept) {
-            const uint64_t js = static_cast<uint64_t>(xyz[0]) +
-                                static_cast<uint64_t>(g.n[0]) * (xyz[1] + static_cast<uint64_t>(g.n[1]) * xyz[2]);
-            const double a2 = scat_angle_square(r.din, r.dout, a.mag);
-            const double v = a.has_energy ? dmul(dmul(a2, r.ein), r.ein) : a2;  // :134-138 (PoCut :60-64)
-            if (a.vox) {
-                a.vox[i] = static_cast<uint32_t>(js);
-                a.value[i] = v;
-            } else {
-                atomicAdd(a.img + js, v);
-            }
-        }
+        if (a.vox)
+            a.vox[i] = kept ? static_cast<uint32_t>(xyz[0] + static_cast<uint64_t>(g.n[0]) *
+                                                                 (xyz[1] + static_cast<uint64_t>(g.n[1]) * xyz[2]))
+                            : 0xffffffffu;
     }
     // kept rays to the walk list, one atomic per warp
     const unsigned act = __activemask(), b = __ballot_sync(act, kept);
@@ -161,26 +153,41 @@ __global__ void k_order_place(const uint32_t* __restrict__ len, const unsigned l
 // (not a grid-stride loop: lanes that finished a ray would start their next
 // one while the others still walk, and the warp would not step together
 // again).
-__global__ void k_poca_walk(PocaArgs a) {
+// Here too the ray's value, on the list's full warps (its four arctangents cost
+// more FP64 operations than the binning above).
+__global__ void __launch_bounds__(128) k_poca_walk(PocaArgs a, DevGrid g) {
     const uint64_t n = *a.walk_count;
-    const DevGrid g = make_dev_grid(a.g);
     const double zmin = a.rays[0].pout[2], zmax = a.rays[0].pin[2];
     const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const unsigned lanes = walk_lanes(t < n);
     if (t < n) {
-        const muto_ray r = a.rays[a.walk[a.walk_order ? a.walk_order[t] : t]];
+        const uint32_t i = a.walk[a.walk_order ? a.walk_order[t] : t];
+        const muto_ray r = a.rays[i];
         double ps[3];
         uint32_t xyz[3];
         bool parallel_ok;
         poca_bin(g, r, a.eps, zmin, zmax, ps, xyz, &parallel_ok);  // the kernel above kept it
+        const double a2 = scat_angle_square(r.din, r.dout, a.mag);
+        const double v = a.has_energy ? dmul(dmul(a2, r.ein), r.ein) : a2;  // :134-138 (PoCut :60-64)
+        if (a.vox)
+            a.value[i] = v;
+        else
+            atomicAdd(a.img + (xyz[0] + static_cast<uint64_t>(g.n[0]) * (xyz[1] + static_cast<uint64_t>(g.n[1]) * xyz[2])), v);
         WeightSink sink{a.weight, g.n[0], g.n[1], g.n[2], g.w[2], a.length_weighted, 0, xyz[0], xyz[1], xyz[2]};
-        if (a.straight) {
-            siddon_walk(g, r.pin, r.pout, sink);
-        } else {
-            siddon_walk(g, r.pin, ps, sink);
+        double from[3] = {r.pin[0], r.pin[1], r.pin[2]}, to[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) to[k] = a.straight ? r.pout[k] : ps[k];
+        // one copy of the walk's code for both halves
+#pragma unroll 1
+        for (int half = 0; half < (a.straight ? 1 : 2); ++half) {
+            siddon_walk(g, from, to, sink);
             sink.skip_scat = !a.length_weighted;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                from[k] = ps[k];
+                to[k] = r.pout[k];
+            }
             __syncwarp(lanes);
-            siddon_walk(g, ps, r.pout, sink);
         }
     }
 }
@@ -311,10 +318,11 @@ void launch_poca(const PocaArgs& a, cudaStream_t s) {
     if (a.n == 0) return;
     cudaMemsetAsync(a.walk_count, 0, sizeof(unsigned long long), s);
     const unsigned nb = static_cast<unsigned>((a.n + 127) / 128);
-    k_poca<<<nb, 128, 0, s>>>(a);
+    const DevGrid g = make_dev_grid(a.g);
+    k_poca<<<nb, 128, 0, s>>>(a, g);
     if (a.walk_len && a.walk_order && a.order_work)  // the list by decreasing walk bound
         launch_length_order(a.walk_len, a.walk_count, a.n, a.walk_order, a.order_work, s);
-    k_poca_walk<<<nb, 128, 0, s>>>(a);  // one thread per ray that can have been kept
+    k_poca_walk<<<nb, 128, 0, s>>>(a, g);  // one thread per ray that can have been kept
     count_launches(2);
 }
 

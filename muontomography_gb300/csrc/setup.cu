@@ -197,62 +197,137 @@ __global__ void k_path_bound(const muto_ray* __restrict__ rays, const uint32_t* 
     }
 }
 
-// the fill walk into bounded slots [boff[i], boff[i+1]) - slot_base; counts[i]
-// = the path's length (0 for a walk that hit its step guard, as in the count walk)
-template <typename Real>
-__global__ void k_path_fill_bounded(const muto_ray* __restrict__ rays, const uint32_t* __restrict__ kept,
-                                    const double* __restrict__ scat, const uint64_t* __restrict__ boff, uint64_t n,
-                                    DevGrid g, int straight, uint32_t* __restrict__ vidx, double* __restrict__ l64,
-                                    Real* __restrict__ L, Real* __restrict__ T, uint32_t* __restrict__ counts,
-                                    Counters* ctr, uint64_t slot_base) {
+// The merged path of one muon into its bounded slots: every voxel as it is
+// walked, the out-half's first length added to the last in-voxel's (or dropped
+// when the in-half is empty), :396-402.
+struct PathSink {
+    uint32_t* vidx;
+    double* l64;
+    uint32_t n, cap;       // pairs written, slots
+    uint32_t nx, nxy;
+    bool merge;            // the next voxel is the out-half's first
+    __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
+        if (merge) {
+            merge = false;
+            if (n > 0 && n <= cap) l64[n - 1] = dadd(l64[n - 1], l);
+            return;
+        }
+        if (n < cap) {  // (a path longer than its bound is counted by the caller)
+            vidx[n] = x + y * nx + z * nxy;  // xyz2index, include/MutoMLSD.h:76
+            l64[n] = l;
+        }
+        ++n;
+    }
+};
+
+// The FP64 walk of every kept muon into bounded slots [boff[i], boff[i+1]) -
+// slot_base; counts[i] = the path's length (0 for a walk that hit its step
+// guard, as in the count walk).  TAILS (FP64 lists): also the tails, summed
+// backwards like src/MutoMLSD.cpp:407-413; the mixed form's come from
+// k_path_finish.
+template <bool TAILS>
+__global__ void __launch_bounds__(128) k_path_walk(const muto_ray* __restrict__ rays, const uint32_t* __restrict__ kept,
+                                                   const double* __restrict__ scat, const uint64_t* __restrict__ boff,
+                                                   uint64_t n, DevGrid g, int straight, uint32_t* __restrict__ vidx,
+                                                   double* __restrict__ l64, double* __restrict__ T,
+                                                   uint32_t* __restrict__ counts, Counters* ctr, uint64_t slot_base) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const unsigned lanes = walk_lanes(i < n);
     if (i >= n) return;
-    const uint64_t b = boff[i] - slot_base, e = boff[i + 1] - slot_base;
+    const uint64_t b = boff[i] - slot_base;
     const muto_ray& r = rays[kept[i]];
     const double ps[3] = {scat[3 * i], scat[3 * i + 1], scat[3 * i + 2]};
-    const uint32_t nx = g.n[0], nxy = g.n[0] * g.n[1];
-    uint64_t end;
+    PathSink s{vidx + b, l64 + b, 0u, static_cast<uint32_t>(boff[i + 1] - slot_base - b), g.n[0], g.n[0] * g.n[1], false};
     bool overflow = false;
-    if (straight) {
-        StraightSink s{vidx, l64, b, e, nx, nxy};
-        overflow = siddon_walk(g, r.pin, r.pout, s) < 0;
-        end = s.pos;
-    } else {
-        FillSink s{vidx, l64, b, e, nx, nxy};
-        const int ci = siddon_walk(g, r.pin, ps, s);
-        s.phase = 1;
+    double from[3] = {r.pin[0], r.pin[1], r.pin[2]}, to[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) to[k] = straight ? r.pout[k] : ps[k];
+    // one copy of the walk's code for both halves
+#pragma unroll 1
+    for (int half = 0; half < (straight ? 1 : 2); ++half) {
+        overflow = siddon_walk(g, from, to, s) < 0 || overflow;
+        s.merge = true;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            from[k] = ps[k];
+            to[k] = r.pout[k];
+        }
         __syncwarp(lanes);
-        const int co = siddon_walk(g, ps, r.pout, s);
-        if (s.pending) s.emit(s.pj, dadd(s.pl, 0.0));  // out-half empty: length += 0.0
-        overflow = ci < 0 || co < 0;
-        end = s.pos;
     }
     if (overflow) {  // dropped, like the count walk does
         atomicAdd(&ctr->overflow, 1ull);
-        end = b;
+        s.n = 0;
     }
-    if (end > e) {
+    if (s.n > s.cap) {
         atomicAdd(&ctr->over_bound, 1ull);
-        end = e;
+        s.n = s.cap;
     }
-    counts[i] = static_cast<uint32_t>(end - b);
-    // tail lengths, summed backwards in FP64 like src/MutoMLSD.cpp:407-413
-    double t = 0.0;
-    for (uint64_t k = end; k-- > b;) {
-        const double lk = l64[k];
-        if (L != reinterpret_cast<Real*>(l64)) L[k] = static_cast<Real>(lk);
-        T[k] = static_cast<Real>(t);
-        t = dadd(t, lk);
+    counts[i] = s.n;
+    if (TAILS) {
+        double t = 0.0;
+        for (uint32_t k = s.n; k-- > 0;) {
+            T[b + k] = t;
+            t = dadd(t, s.l64[k]);
+        }
     }
 }
 
-// warp per muon: its path from the bounded slots (boff[i] - slot_base) to the exact ones
-template <typename Real>
+// The mixed form's lists from the walked slots, a warp per muon, coalesced: the
+// voxel, L and the tail T to the exact slots.  The reference sums a tail one
+// length after the other from the path's end; here 32 lengths at a time by a
+// scan.  The two FP64 sums differ by at most (m + 16) units of their last place
+// (m lengths, each sum's roundings), so they round to the same FP32 value unless
+// the scan's sum lies that near to the middle of two: a muon with such a tail
+// (one in some thousands) is summed again in the reference's order.  FP64
+// operations a pair: a quarter, against one on each lane of a thread-per-muon
+// loop with 14 of 32 lanes at work.
+__global__ void __launch_bounds__(256) k_path_finish(const uint64_t* __restrict__ boff, uint64_t slot_base,
+                                                     const uint64_t* __restrict__ off, uint64_t n,
+                                                     const uint32_t* __restrict__ vidx_b,
+                                                     const double* __restrict__ l64, uint32_t* __restrict__ vidx,
+                                                     float* __restrict__ L, float* __restrict__ T) {
+    const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const uint64_t src = boff[i] - slot_base, dst = off[i];
+    const int m = static_cast<int>(off[i + 1] - dst);
+    double carry = 0.0;
+    bool near = false;
+    for (int k0 = (m - 1) & ~31; k0 >= 0; k0 -= 32) {
+        const int k = k0 + lane;
+        const double l = k < m ? l64[src + k] : 0.0;
+        double s = l;  // of this length and those after it, up to the 32nd
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double t = __shfl_down_sync(kFull, s, o);
+            if (lane + o < 32) s = dadd(s, t);
+        }
+        const double after = __shfl_down_sync(kFull, s, 1);
+        const double t = lane < 31 ? dadd(carry, after) : carry;
+        if (k < m) {
+            vidx[dst + k] = vidx_b[src + k];
+            L[dst + k] = static_cast<float>(l);
+            T[dst + k] = static_cast<float>(t);
+            // 29 bits of the sum's mantissa lie below the float's last place
+            const int from_middle = (__double2loint(t) & 0x1fffffff) - 0x10000000;
+            near = near || abs(from_middle) <= m + 16;
+        }
+        carry = dadd(carry, __shfl_sync(kFull, s, 0));
+    }
+    if (__any_sync(kFull, near) && lane == 0) {
+        double t = 0.0;
+        for (int k = m; k-- > 0;) {
+            T[dst + k] = static_cast<float>(t);
+            t = dadd(t, l64[src + k]);
+        }
+    }
+}
+
+// warp per muon: its FP64 path from the bounded slots (boff[i] - slot_base) to the exact ones
 __global__ void k_path_compact(const uint64_t* __restrict__ boff, uint64_t slot_base, const uint64_t* __restrict__ off,
-                               uint64_t n, const uint32_t* __restrict__ vidx_b, const Real* __restrict__ L_b,
-                               const Real* __restrict__ T_b, uint32_t* __restrict__ vidx, Real* __restrict__ L,
-                               Real* __restrict__ T) {
+                               uint64_t n, const uint32_t* __restrict__ vidx_b, const double* __restrict__ L_b,
+                               const double* __restrict__ T_b, uint32_t* __restrict__ vidx, double* __restrict__ L,
+                               double* __restrict__ T) {
     const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
@@ -510,35 +585,33 @@ void launch_path_bound(const muto_ray* rays, const uint32_t* kept, const double*
     count_launches(1);
 }
 
-template <typename Real>
-void launch_path_fill_bounded(const muto_ray* rays, const uint32_t* kept, const double* scat, const uint64_t* boff,
-                              uint64_t slot_base, uint64_t n, muto_grid g, int straight, uint32_t* vidx, double* l64,
-                              Real* L, Real* T, uint32_t* counts, Counters* ctr, cudaStream_t s) {
+void launch_path_walk(const muto_ray* rays, const uint32_t* kept, const double* scat, const uint64_t* boff,
+                      uint64_t slot_base, uint64_t n, muto_grid g, int straight, uint32_t* vidx, double* l64, double* T,
+                      uint32_t* counts, Counters* ctr, cudaStream_t s) {
     if (n == 0) return;
-    k_path_fill_bounded<Real><<<blocks_for(n, 128), 128, 0, s>>>(rays, kept, scat, boff, n, make_dev_grid(g), straight,
-                                                                  vidx, l64, L, T, counts, ctr, slot_base);
+    if (T)
+        k_path_walk<true><<<blocks_for(n, 128), 128, 0, s>>>(rays, kept, scat, boff, n, make_dev_grid(g), straight, vidx,
+                                                             l64, T, counts, ctr, slot_base);
+    else
+        k_path_walk<false><<<blocks_for(n, 128), 128, 0, s>>>(rays, kept, scat, boff, n, make_dev_grid(g), straight, vidx,
+                                                              l64, T, counts, ctr, slot_base);
     count_launches(1);
 }
-template void launch_path_fill_bounded<float>(const muto_ray*, const uint32_t*, const double*, const uint64_t*,
-                                              uint64_t, uint64_t, muto_grid, int, uint32_t*, double*, float*, float*,
-                                              uint32_t*, Counters*, cudaStream_t);
-template void launch_path_fill_bounded<double>(const muto_ray*, const uint32_t*, const double*, const uint64_t*,
-                                               uint64_t, uint64_t, muto_grid, int, uint32_t*, double*, double*,
-                                               double*, uint32_t*, Counters*, cudaStream_t);
 
-template <typename Real>
-void launch_path_compact(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
-                         const uint32_t* vidx_b, const Real* L_b, const Real* T_b, uint32_t* vidx, Real* L, Real* T,
-                         cudaStream_t s) {
+void launch_path_finish(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
+                        const uint32_t* vidx_b, const double* l64, uint32_t* vidx, float* L, float* T, cudaStream_t s) {
     if (n == 0) return;
-    k_path_compact<Real><<<blocks_for(n * 32), kThreads, 0, s>>>(boff, slot_base, off, n, vidx_b, L_b, T_b, vidx, L,
-                                                                 T);
+    k_path_finish<<<blocks_for(n * 32), kThreads, 0, s>>>(boff, slot_base, off, n, vidx_b, l64, vidx, L, T);
     count_launches(1);
 }
-template void launch_path_compact<float>(const uint64_t*, uint64_t, const uint64_t*, uint64_t, const uint32_t*,
-                                         const float*, const float*, uint32_t*, float*, float*, cudaStream_t);
-template void launch_path_compact<double>(const uint64_t*, uint64_t, const uint64_t*, uint64_t, const uint32_t*,
-                                          const double*, const double*, uint32_t*, double*, double*, cudaStream_t);
+
+void launch_path_compact(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
+                         const uint32_t* vidx_b, const double* L_b, const double* T_b, uint32_t* vidx, double* L,
+                         double* T, cudaStream_t s) {
+    if (n == 0) return;
+    k_path_compact<<<blocks_for(n * 32), kThreads, 0, s>>>(boff, slot_base, off, n, vidx_b, L_b, T_b, vidx, L, T);
+    count_launches(1);
+}
 
 void launch_offset_voxels(uint32_t* vidx, uint64_t n, uint32_t v_scan, uint32_t voff, cudaStream_t s) {
     if (n == 0) return;

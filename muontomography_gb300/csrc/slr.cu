@@ -68,10 +68,9 @@ struct SlrSink {
     }
 };
 
-__global__ void k_slr(SlrArgs a) {
+__global__ void k_slr(SlrArgs a, DevGrid g) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    const DevGrid g = make_dev_grid(a.g);
     const muto_ray r = a.rays[i];
     const double z_lo = a.g.z_min;                                               // :57
     const double z_hi = dadd(a.g.z_min, dmul(a.g.dz, static_cast<double>(a.g.nz)));  // :58
@@ -104,11 +103,10 @@ struct PathSink {
     }
 };
 
-__global__ void k_slr_paths(SlrArgs a, const uint64_t* __restrict__ off, uint32_t* __restrict__ counts,
+__global__ void k_slr_paths(SlrArgs a, DevGrid g, const uint64_t* __restrict__ off, uint32_t* __restrict__ counts,
                             uint32_t* __restrict__ vox, double* __restrict__ len) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    const DevGrid g = make_dev_grid(a.g);
     const double z_lo = a.g.z_min;
     const double z_hi = dadd(a.g.z_min, dmul(a.g.dz, static_cast<double>(a.g.nz)));
     const SlrRay s = slr_ray(a.rays[i], g, z_lo, z_hi, a.mag);
@@ -122,10 +120,9 @@ __global__ void k_slr_paths(SlrArgs a, const uint64_t* __restrict__ off, uint32_
 // by the voxel's part of the path's sum (a^2 / 2 (length / l_total)^2, or the
 // equal share a^2 / 2 / n^2), with the arithmetic of :80-89; and ein^2 per
 // muon.  A thread per muon.
-__global__ void k_slr_pair_terms(SlrArgs a, SlrPass p) {
+__global__ void k_slr_pair_terms(SlrArgs a, DevGrid g, SlrPass p) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    const DevGrid g = make_dev_grid(a.g);
     const double z_lo = a.g.z_min;
     const double z_hi = dadd(a.g.z_min, dmul(a.g.dz, static_cast<double>(a.g.nz)));
     const muto_ray r = a.rays[i];
@@ -353,20 +350,20 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
 
 void launch_slr(const SlrArgs& a, cudaStream_t s) {
     if (a.n == 0) return;
-    k_slr<<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, s>>>(a);
+    k_slr<<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, s>>>(a, make_dev_grid(a.g));
     count_launches(1);
 }
 
 void launch_slr_paths(const SlrArgs& a, const uint64_t* off, uint32_t* counts, uint32_t* vox, double* len,
                       cudaStream_t s) {
     if (a.n == 0) return;
-    k_slr_paths<<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, s>>>(a, off, counts, vox, len);
+    k_slr_paths<<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, s>>>(a, make_dev_grid(a.g), off, counts, vox, len);
     count_launches(1);
 }
 
 void launch_slr_pair_terms(const SlrArgs& a, const SlrPass& p, cudaStream_t s) {
     if (a.n == 0) return;
-    k_slr_pair_terms<<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, s>>>(a, p);
+    k_slr_pair_terms<<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, s>>>(a, make_dev_grid(a.g), p);
     count_launches(1);
 }
 
