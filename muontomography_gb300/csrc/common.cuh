@@ -92,6 +92,8 @@ struct Counters {
 // (out[n] = total).  scratch must hold scan_scratch_bytes(n) bytes.
 size_t scan_scratch_bytes(uint64_t n);
 void scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, void* scratch, cudaStream_t s);
+// out[i] = src[at[i]]
+void launch_gather_u64(const uint64_t* src, const uint64_t* at, uint64_t n, uint64_t* out, cudaStream_t s);
 // a[i] += add for i < n
 void launch_add_u64(uint64_t* a, uint64_t n, uint64_t add, cudaStream_t s);
 
@@ -502,6 +504,9 @@ void launch_map_voxel(const LamT* last, double* ml_inout, const uint32_t* mult, 
                       Counters* ctr, cudaStream_t s);
 template <typename LamT>
 void launch_copy_to(const double* in, LamT* out, uint64_t n, cudaStream_t s);
+void launch_widen(const float* in, double* out, uint64_t n, cudaStream_t s);
+template <typename Real>
+void launch_fill(Real* out, uint64_t n, Real value, cudaStream_t s);
 
 // adjoint.cu
 template <typename Real>

@@ -964,6 +964,16 @@ __global__ void k_copy_to(const double* __restrict__ in, LamT* __restrict__ out,
     if (i < n) out[i] = static_cast<LamT>(in[i]);
 }
 
+__global__ void k_widen(const float* __restrict__ in, double* __restrict__ out, uint64_t n) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = static_cast<double>(in[i]);
+}
+
+template <typename Real>
+__global__ void k_fill(Real* __restrict__ out, uint64_t n, Real value) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = value;
+}
 
 inline unsigned blocks_for(uint64_t n, int threads) {
     const uint64_t b = (n + threads - 1) / threads;
@@ -1110,5 +1120,20 @@ void launch_copy_to(const double* in, LamT* out, uint64_t n, cudaStream_t s) {
 }
 template void launch_copy_to<float>(const double*, float*, uint64_t, cudaStream_t);
 template void launch_copy_to<double>(const double*, double*, uint64_t, cudaStream_t);
+
+void launch_widen(const float* in, double* out, uint64_t n, cudaStream_t s) {
+    if (n == 0) return;
+    k_widen<<<blocks_for(n, 256), 256, 0, s>>>(in, out, n);
+    count_launches(1);
+}
+
+template <typename Real>
+void launch_fill(Real* out, uint64_t n, Real value, cudaStream_t s) {
+    if (n == 0) return;
+    k_fill<Real><<<blocks_for(n, 256), 256, 0, s>>>(out, n, value);
+    count_launches(1);
+}
+template void launch_fill<float>(float*, uint64_t, float, cudaStream_t);
+template void launch_fill<double>(double*, uint64_t, double, cudaStream_t);
 
 }  // namespace muto

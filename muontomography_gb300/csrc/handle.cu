@@ -73,7 +73,23 @@ cudaMemPool_t device_pool(int dev) {
     return pools[dev];
 }
 
-// Owned device allocation.
+// The stream that this thread's allocations and frees are ordered on: the
+// handle's (or the call's own) stream inside an entry point, none outside.
+thread_local cudaStream_t t_alloc_stream = nullptr;
+struct AllocScope {
+    cudaStream_t before;
+    explicit AllocScope(cudaStream_t s) : before(t_alloc_stream) { t_alloc_stream = s; }
+    ~AllocScope() { t_alloc_stream = before; }
+    AllocScope(const AllocScope&) = delete;
+    AllocScope& operator=(const AllocScope&) = delete;
+};
+
+// Owned device allocation, ordered on the stream of the entry point that made it:
+// every use is on that stream, or on streams forked from it and joined back, so
+// neither the allocation nor the free waits for the device (a wait at each of the
+// forty or so allocations of a reconstruction took a third of a small call).  The
+// owner of the stream outlives the allocation.  The pool makes another stream that
+// is given the block wait for the free.
 class DevMem {
 public:
     DevMem() = default;
@@ -85,16 +101,17 @@ public:
         if (bytes == 0) bytes = 16;
         int dev = 0;
         CK(cudaGetDevice(&dev));
-        CK(cudaMallocFromPoolAsync(&p_, bytes, device_pool(dev), 0));
-        CK(cudaStreamSynchronize(0));  // usable from any stream once this returns
+        stream_ = t_alloc_stream;
+        CK(cudaMallocFromPoolAsync(&p_, bytes, device_pool(dev), stream_));
+        if (!stream_) CK(cudaStreamSynchronize(nullptr));  // usable from any stream once this returns
         bytes_ = bytes;
         tally_ = tally;
         if (tally_) *tally_ += bytes_;
     }
     void release() {
         if (p_) {
-            cudaDeviceSynchronize();
-            cudaFreeAsync(p_, 0);
+            if (!stream_) cudaDeviceSynchronize();
+            cudaFreeAsync(p_, stream_);
             if (tally_) *tally_ -= bytes_;
         }
         p_ = nullptr;
@@ -107,18 +124,102 @@ public:
 private:
     void* p_ = nullptr;
     size_t bytes_ = 0;
+    cudaStream_t stream_ = nullptr;
     std::atomic<uint64_t>* tally_ = nullptr;
 };
 
-// A non-blocking stream owned by one call, destroyed on every way out.
+// A non-blocking stream owned by one call, destroyed on every way out; the call's
+// allocations are ordered on it.
 struct OwnedStream {
     cudaStream_t s = nullptr;
-    OwnedStream() { CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
+    std::unique_ptr<AllocScope> scope;
+    OwnedStream() {
+        CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        scope.reset(new AllocScope(s));
+    }
     ~OwnedStream() {
         if (s) cudaStreamDestroy(s);
     }
     OwnedStream(const OwnedStream&) = delete;
     OwnedStream& operator=(const OwnedStream&) = delete;
+};
+
+// The streams and events of one handle, from a small pool per device: creating
+// and destroying them takes longer than a small scan's iterations.  A set goes
+// back to the pool idle (the handle's destructor waits for its stream); the pool
+// keeps at most kKept sets a device and destroys the rest.
+struct HandleStreams {
+    static constexpr int kOverlap = 5;
+    int device = 0;
+    cudaStream_t stream = nullptr;
+    ClassFan fan{};
+    cudaEvent_t ov_ev[kOverlap] = {};
+
+    void create(int dev) {
+        device = dev;
+        CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&fan.fork, cudaEventDisableTiming));
+        for (int k = 0; k < ClassFan::kSide; ++k) {
+            CK(cudaStreamCreateWithFlags(&fan.side[k], cudaStreamNonBlocking));
+            CK(cudaEventCreateWithFlags(&fan.join[k], cudaEventDisableTiming));
+            fan.n = k + 1;
+        }
+        for (cudaEvent_t& e : ov_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    void destroy() {
+        for (int k = 0; k < ClassFan::kSide; ++k) {
+            if (fan.side[k]) cudaStreamDestroy(fan.side[k]);
+            if (fan.join[k]) cudaEventDestroy(fan.join[k]);
+        }
+        if (fan.fork) cudaEventDestroy(fan.fork);
+        for (cudaEvent_t e : ov_ev)
+            if (e) cudaEventDestroy(e);
+        if (stream) cudaStreamDestroy(stream);
+        *this = HandleStreams{};
+    }
+    static constexpr size_t kKept = 8;
+    static std::mutex& mutex() {
+        static std::mutex m;
+        return m;
+    }
+    static std::map<int, std::vector<HandleStreams>>& kept() {
+        static std::map<int, std::vector<HandleStreams>> k;
+        return k;
+    }
+    // the device's streams for a new handle
+    static HandleStreams take(int dev) {
+        {
+            std::lock_guard<std::mutex> lock(mutex());
+            auto& k = kept()[dev];
+            if (!k.empty()) {
+                HandleStreams h = k.back();
+                k.pop_back();
+                return h;
+            }
+        }
+        HandleStreams h;
+        try {
+            h.create(dev);
+        } catch (...) {
+            h.destroy();
+            throw;
+        }
+        return h;
+    }
+    // back to the pool, its work done
+    void give() {
+        if (!stream) return;
+        if (cudaStreamSynchronize(stream) == cudaSuccess) {
+            std::lock_guard<std::mutex> lock(mutex());
+            auto& k = kept()[device];
+            if (k.size() < kKept) {
+                k.push_back(*this);
+                *this = HandleStreams{};
+                return;
+            }
+        }
+        destroy();
+    }
 };
 
 enum Method { kPoca, kMlsd, kMap };
@@ -360,11 +461,15 @@ public:
 using namespace muto;
 
 struct muto_handle {
+    // first: the allocations below are freed on its stream
+    struct Streams : HandleStreams {
+        ~Streams() { give(); }
+    } streams;
     Method method = kMlsd;
     Params P;
     muto_grid grid{};          // current grid (may be adopted from the initial image)
-    cudaStream_t stream = nullptr;
-    ClassFan fan;                 // side streams of the voxel pass's class kernels
+    cudaStream_t stream = nullptr;  // = streams.stream
+    ClassFan fan;                   // = streams.fan: side streams of the voxel pass's class kernels
     int device = 0, num_sms = 148;
     uint64_t l2_bytes = 0;         // the device's L2 size
     size_t smem_optin = 0;
@@ -425,7 +530,7 @@ struct muto_handle {
     static constexpr int kOverlapChunks = 4;
     bool overlap = false;
     int warp_blocks_ov = 0, scatter_blocks_ov = 0;  // each kernel's grid when they share the GPU
-    cudaEvent_t ov_ev[kOverlapChunks + 1] = {};
+    cudaEvent_t ov_ev[kOverlapChunks + 1] = {};  // = streams.ov_ev
     bool brick = false;               // path voxel indices are bricked (single scans), see lam_b
     BrickDims bdims{};
     uint64_t vb = 0;                  // bricked index space (>= V)
@@ -464,14 +569,6 @@ struct muto_handle {
     }
     ~muto_handle() {
         drop_graph();
-        for (int k = 0; k < fan.n; ++k) {
-            cudaStreamDestroy(fan.side[k]);
-            cudaEventDestroy(fan.join[k]);
-        }
-        if (fan.n) cudaEventDestroy(fan.fork);
-        for (cudaEvent_t e : ov_ev)
-            if (e) cudaEventDestroy(e);
-        if (stream) cudaStreamDestroy(stream);
     }
 };
 
@@ -486,6 +583,7 @@ void set_err(muto_handle* h, int code, const std::string& msg) {
 template <class F>
 int guarded(muto_handle* h, F&& f) {
     try {
+        AllocScope scope(h ? h->stream : nullptr);
         f();
         return MUTO_OK;
     } catch (const Error& e) {
@@ -551,7 +649,11 @@ void sync_and_harvest(muto_handle* h, size_t first) {
 // ---------------------------------------------------------------------------
 // Setup
 // ---------------------------------------------------------------------------
+// A constant start (any initialize_method but 0 and 1) is filled on the device.
+bool constant_start(const muto_handle* h) { return h->P.initialize_method != 0 && h->P.initialize_method != 1; }
+
 void resolve_initial_image(muto_handle* h, std::vector<double>& img, uint64_t seed_offset = 0) {
+    if (constant_start(h)) return;
     int method = h->P.initialize_method;
     if (method == 0) {  // src/MutoMLSD.cpp:228-245
         if (!h->init_set || h->init_missing || h->init_img.empty()) {
@@ -564,7 +666,7 @@ void resolve_initial_image(muto_handle* h, std::vector<double>& img, uint64_t se
         }
     }
     img.assign(static_cast<uint64_t>(h->grid.nx) * h->grid.ny * h->grid.nz, 0.0);
-    if (method == 1) {  // N(2, 0.5) * 1e-7, at least 1e-10 (src/MutoMLSD.cpp:251-261)
+    {  // N(2, 0.5) * 1e-7, at least 1e-10 (src/MutoMLSD.cpp:251-261)
         uint64_t seed = (h->P.seed_set ? h->P.random_seed : std::random_device{}()) + seed_offset;
         std::mt19937_64 gen(seed);
         const double two_pi = 6.283185307179586;
@@ -575,8 +677,6 @@ void resolve_initial_image(muto_handle* h, std::vector<double>& img, uint64_t se
             const double v = (2.0 + 0.5 * z) * 1.0e-7;
             img[i] = 1.0e-10 <= v ? v : 1.0e-10;
         }
-    } else {
-        std::fill(img.begin(), img.end(), h->P.initialize_value);
     }
 }
 
@@ -830,6 +930,52 @@ void prepare_poca(muto_handle* h) {
     CK(cudaStreamSynchronize(s));  // the scratch arrays go out of scope
 }
 
+// The scans of a batch spread over the handle's streams: f(k, stream) for every
+// scan, whose launches touch nothing that another scan's do; what the handle's
+// stream runs before and after is ordered around all of them.  (A small scan's
+// kernels leave the GPU mostly idle.)
+template <class F>
+void fan_scans(muto_handle* h, F&& f) {
+    const size_t S = h->scans.size();
+    const int side = S > 1 && !h->prof.on ? h->fan.n : 0;
+    if (side) {
+        CK(cudaEventRecord(h->fan.fork, h->stream));
+        for (int q = 0; q < side; ++q) CK(cudaStreamWaitEvent(h->fan.side[q], h->fan.fork, 0));
+    }
+    try {
+        for (size_t k = 0; k < S; ++k) {
+            const size_t q = k % static_cast<size_t>(side + 1);
+            f(k, q == 0 ? h->stream : h->fan.side[q - 1]);
+        }
+    } catch (...) {  // nothing is freed under the launches that were made
+        for (int q = 0; q < side; ++q) cudaStreamSynchronize(h->fan.side[q]);
+        throw;
+    }
+    for (int q = 0; q < side; ++q) {
+        CK(cudaEventRecord(h->fan.join[q], h->fan.side[q]));
+        CK(cudaStreamWaitEvent(h->stream, h->fan.join[q], 0));
+    }
+}
+
+// src[at[k]] of every k on the host, in one copy; waits for the handle's stream
+std::vector<uint64_t> read_at(muto_handle* h, const uint64_t* src, const std::vector<uint64_t>& at) {
+    std::vector<uint64_t> v(at.size());
+    cudaStream_t s = h->stream;
+    if (at.size() <= 2) {
+        for (size_t k = 0; k < at.size(); ++k)
+            CK(cudaMemcpyAsync(&v[k], src + at[k], sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    } else {
+        DevMem idx, val;
+        idx.alloc(at.size() * sizeof(uint64_t), &h->dev_bytes);
+        val.alloc(at.size() * sizeof(uint64_t), &h->dev_bytes);
+        CK(cudaMemcpyAsync(idx.as<void>(), at.data(), at.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
+        launch_gather_u64(src, idx.as<uint64_t>(), at.size(), val.as<uint64_t>(), s);
+        CK(cudaMemcpyAsync(v.data(), val.as<void>(), at.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    }
+    CK(cudaStreamSynchronize(s));
+    return v;
+}
+
 // The merged paths of all kept muons into the muon-major lists (vidx, L, T)
 // with their offsets.  Per chunk of muons: one FP64 walk into slots sized by
 // the FP32 path bounds (scratch for the chunk alone), then compaction to the
@@ -860,10 +1006,13 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
     h->T.alloc((Pb + kPad) * sizeof(Real), &h->dev_bytes);
     // one chunk's bounded slots: voxel, FP64 length, and the FP64 form's tail
     const uint64_t per_pair = sizeof(uint32_t) + sizeof(double) + (real64 ? sizeof(double) : 0);
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    const uint64_t budget = std::min<uint64_t>(free_b / 4, uint64_t(12) << 30);
-    uint64_t cap = std::min<uint64_t>(std::max<uint64_t>(Pb, 1), std::max<uint64_t>(budget / per_pair, uint64_t(1) << 20));
+    uint64_t cap = std::max<uint64_t>(Pb, 1);
+    if (cap > uint64_t(1) << 20) {  // (a smaller scan is one chunk whatever memory is left)
+        size_t free_b = 0, total_b = 0;
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        const uint64_t budget = std::min<uint64_t>(free_b / 4, uint64_t(12) << 30);
+        cap = std::min<uint64_t>(cap, std::max<uint64_t>(budget / per_pair, uint64_t(1) << 20));
+    }
     if (P.setup_chunk_pairs > 0) cap = static_cast<uint64_t>(P.setup_chunk_pairs);
     DevMem vidx_b, l64_b, T_b;
     vidx_b.alloc((cap + kPad) * sizeof(uint32_t), &h->dev_bytes);
@@ -872,43 +1021,58 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
     const double avg = N ? static_cast<double>(Pb) / static_cast<double>(N) : 1.0;
     const uint64_t chunk0 = std::max<uint64_t>(P.setup_chunk_pairs > 0 ? 1 : 1024,
                                                static_cast<uint64_t>(static_cast<double>(cap) / (1.25 * avg + 1.0)));
-    uint64_t base = 0;
-    for (size_t k = 0; k < S; ++k) {
-        const auto& sc = h->scans[k];
-        const uint64_t end = sc.noff + sc.N;
-        for (uint64_t m = sc.noff; m < end;) {
-            uint64_t nc = std::min<uint64_t>(end - m, chunk0);
-            uint64_t b[2] = {0, 0};
-            for (;;) {  // the chunk's bounded slots must fit the scratch
-                CK(cudaMemcpyAsync(&b[0], boff.as<uint64_t>() + m, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-                CK(cudaMemcpyAsync(&b[1], boff.as<uint64_t>() + m + nc, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-                CK(cudaStreamSynchronize(s));
-                if (b[1] - b[0] <= cap || nc == 1) break;
-                nc = (nc + 1) / 2;
-            }
-            if (b[1] - b[0] > cap) throw Error(MUTO_ERR_CAPACITY, "a muon's path bound exceeds the set-up scratch");
+    auto finish = [&](uint64_t m, uint64_t slot0, uint64_t nc) {  // muons m .. m + nc - 1, their slots from slot0 on
+        run(h, "path_finish", [&] {
+            if constexpr (real64)
+                launch_path_compact(boff.as<uint64_t>() + m, slot0, h->off.as<uint64_t>() + m, nc, vidx_b.as<uint32_t>(),
+                                    l64_b.as<double>(), T_b.as<double>(), h->vidx.as<uint32_t>(), h->L.as<Real>(),
+                                    h->T.as<Real>(), s);
+            else
+                launch_path_finish(boff.as<uint64_t>() + m, slot0, h->off.as<uint64_t>() + m, nc, vidx_b.as<uint32_t>(),
+                                   l64_b.as<double>(), h->vidx.as<uint32_t>(), h->L.as<Real>(), h->T.as<Real>(), s);
+        });
+    };
+    if (Pb <= cap) {  // one chunk: every scan's walk, then one scan and one copy
+        fan_scans(h, [&](size_t k, cudaStream_t on) {
+            const auto& sc = h->scans[k];
             run(h, "siddon_fill", [&] {
-                launch_path_walk(h->scan_rays(k), h->kept.as<uint32_t>() + m, h->scat.as<double>() + 3 * m,
-                                 boff.as<uint64_t>() + m, b[0], nc, sc.grid, P.straight_line, vidx_b.as<uint32_t>(),
-                                 l64_b.as<double>(), T_b.as<double>(), counts.as<uint32_t>() + m, h->ctr(), s);
+                launch_path_walk(h->scan_rays(k), h->kept.as<uint32_t>() + sc.noff, h->scat.as<double>() + 3 * sc.noff,
+                                 boff.as<uint64_t>() + sc.noff, 0, sc.N, sc.grid, P.straight_line, vidx_b.as<uint32_t>(),
+                                 l64_b.as<double>(), T_b.as<double>(), counts.as<uint32_t>() + sc.noff, h->ctr(), on);
             });
-            run(h, "scan", [&] {
-                scan_u32_to_u64(counts.as<uint32_t>() + m, h->off.as<uint64_t>() + m, nc, scratch.as<void>(), s);
-                launch_add_u64(h->off.as<uint64_t>() + m, nc + 1, base, s);
-            });
-            run(h, "path_compact", [&] {
-                if constexpr (real64)
-                    launch_path_compact(boff.as<uint64_t>() + m, b[0], h->off.as<uint64_t>() + m, nc,
-                                        vidx_b.as<uint32_t>(), l64_b.as<double>(), T_b.as<double>(),
-                                        h->vidx.as<uint32_t>(), h->L.as<Real>(), h->T.as<Real>(), s);
-                else
-                    launch_path_finish(boff.as<uint64_t>() + m, b[0], h->off.as<uint64_t>() + m, nc,
-                                       vidx_b.as<uint32_t>(), l64_b.as<double>(), h->vidx.as<uint32_t>(),
-                                       h->L.as<Real>(), h->T.as<Real>(), s);
-            });
-            CK(cudaMemcpyAsync(&base, h->off.as<uint64_t>() + m + nc, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            m += nc;
+        });
+        run(h, "scan", [&] { scan_u32_to_u64(counts.as<uint32_t>(), h->off.as<uint64_t>(), N, scratch.as<void>(), s); });
+        finish(0, 0, N);
+    } else {
+        uint64_t base = 0;
+        for (size_t k = 0; k < S; ++k) {
+            const auto& sc = h->scans[k];
+            const uint64_t end = sc.noff + sc.N;
+            for (uint64_t m = sc.noff; m < end;) {
+                uint64_t nc = std::min<uint64_t>(end - m, chunk0);
+                uint64_t b[2] = {0, 0};
+                for (;;) {  // the chunk's bounded slots must fit the scratch
+                    CK(cudaMemcpyAsync(&b[0], boff.as<uint64_t>() + m, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+                    CK(cudaMemcpyAsync(&b[1], boff.as<uint64_t>() + m + nc, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+                    CK(cudaStreamSynchronize(s));
+                    if (b[1] - b[0] <= cap || nc == 1) break;
+                    nc = (nc + 1) / 2;
+                }
+                if (b[1] - b[0] > cap) throw Error(MUTO_ERR_CAPACITY, "a muon's path bound exceeds the set-up scratch");
+                run(h, "siddon_fill", [&] {
+                    launch_path_walk(h->scan_rays(k), h->kept.as<uint32_t>() + m, h->scat.as<double>() + 3 * m,
+                                     boff.as<uint64_t>() + m, b[0], nc, sc.grid, P.straight_line, vidx_b.as<uint32_t>(),
+                                     l64_b.as<double>(), T_b.as<double>(), counts.as<uint32_t>() + m, h->ctr(), s);
+                });
+                run(h, "scan", [&] {
+                    scan_u32_to_u64(counts.as<uint32_t>() + m, h->off.as<uint64_t>() + m, nc, scratch.as<void>(), s);
+                    launch_add_u64(h->off.as<uint64_t>() + m, nc + 1, base, s);
+                });
+                finish(m, b[0], nc);
+                CK(cudaMemcpyAsync(&base, h->off.as<uint64_t>() + m + nc, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+                CK(cudaStreamSynchronize(s));
+                m += nc;
+            }
         }
     }
     vidx_b.release();
@@ -954,16 +1118,39 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
     counts.release();
     // pair offsets on the host: each scan's first pair and the total, and
     // every muon's for the tile schedule
-    for (size_t k = 0; k < S; ++k)
-        CK(cudaMemcpyAsync(&scan_off[k], h->off.as<uint64_t>() + h->scans[k].noff, sizeof(uint64_t),
-                           cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&scan_off[S], h->off.as<uint64_t>() + N, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    std::vector<uint64_t> bounds_at;
+    for (const auto& sc : h->scans) bounds_at.push_back(sc.noff);
+    bounds_at.push_back(N);
+    scan_off = read_at(h, h->off.as<uint64_t>(), bounds_at);
     if (P.muon_pass == 1 && h->lists == kListsVoxelMajor) {
         off_h.resize(N + 1);
         CK(cudaMemcpyAsync(off_h.data(), h->off.as<uint64_t>(), (N + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     }
     CK(cudaStreamSynchronize(s));
     h->npairs = scan_off[S];
+}
+
+// Resident blocks of the class kernels on the whole GPU: the same for every
+// handle on a device, so asked for once (some fifty driver calls).
+template <typename Real>
+void voxel_occupancy(muto_handle* h) {
+    struct Blocks {
+        int real[2 * kVoxClasses], f64[2 * kVoxClasses];
+    };
+    static std::mutex m;
+    static std::map<int, Blocks> known;
+    std::lock_guard<std::mutex> lock(m);
+    auto it = known.find(h->device);
+    if (it == known.end()) {
+        Blocks b;
+        em_voxel_occupancy<Real, Real>(b.real);
+        em_voxel_occupancy<Real, double>(b.f64);
+        it = known.emplace(h->device, b).first;
+    }
+    for (int c = 0; c < 2 * kVoxClasses; ++c) {
+        h->vox_blocks_real[c] = it->second.real[c] * h->num_sms;
+        h->vox_blocks_f64[c] = it->second.f64[c] * h->num_sms;
+    }
 }
 
 template <typename Real>
@@ -997,37 +1184,37 @@ void prepare_em(muto_handle* h) {
         }
         h->grid = h->scans[0].grid;
     }
-    uint64_t nt_max = 0;
     for (auto& sc : h->scans) {
         uint64_t nt = P.total_num_rays > 0 ? static_cast<uint64_t>(P.total_num_rays) : sc.n_rays;
         sc.n_total = nt > sc.n_rays ? sc.n_rays : nt;  // the reference would read past the end
-        nt_max = std::max(nt_max, sc.n_total);
     }
     h->n_total = 0;
     for (auto& sc : h->scans) h->n_total += sc.n_total;
 
     // --- gatherInformation per scan: keep flags, order-preserving compaction ---
-    // (the flags are computed again in the second loop; the flag buffer is shared)
-    DevMem flags, scratch;
-    std::vector<std::unique_ptr<DevMem>> pos(S);
+    // (the flags of all scans end to end and one scan of them: a kept muon's
+    // position is its place among the kept muons of every scan)
+    DevMem flags, pos, scratch;
     std::unique_ptr<HostPhase> ph(new HostPhase(h, "gather"));
-    flags.alloc(std::max<uint64_t>(nt_max, 1) * sizeof(uint32_t), &h->dev_bytes);
-    uint64_t N = 0;
+    std::vector<uint64_t> first(S + 1, 0);
+    for (size_t k = 0; k < S; ++k) first[k + 1] = first[k] + h->scans[k].n_total;
+    const uint64_t n_all = first[S];
+    flags.alloc(std::max<uint64_t>(n_all, 1) * sizeof(uint32_t), &h->dev_bytes);
+    pos.alloc((n_all + 1) * sizeof(uint64_t), &h->dev_bytes);
+    scratch.alloc(scan_scratch_bytes(std::max<uint64_t>(n_all, V) + 1), &h->dev_bytes);
+    fan_scans(h, [&](size_t k, cudaStream_t on) {
+        const auto& sc = h->scans[k];
+        run(h, "keep_flags", [&] {
+            launch_keep_flags(h->scan_rays(k), sc.n_total, sc.grid, P.eps, flags.as<uint32_t>() + first[k], on);
+        });
+    });
+    run(h, "scan", [&] { scan_u32_to_u64(flags.as<uint32_t>(), pos.as<uint64_t>(), n_all, scratch.as<void>(), s); });
+    const std::vector<uint64_t> at = read_at(h, pos.as<uint64_t>(), first);
     for (size_t k = 0; k < S; ++k) {
-        auto& sc = h->scans[k];
-        pos[k].reset(new DevMem());
-        pos[k]->alloc((sc.n_total + 1) * sizeof(uint64_t), &h->dev_bytes);
-        if (scratch.bytes() < scan_scratch_bytes(sc.n_total + 1))
-            scratch.alloc(scan_scratch_bytes(std::max<uint64_t>(sc.n_total, V) + 1), &h->dev_bytes);
-        run(h, "keep_flags", [&] { launch_keep_flags(h->scan_rays(k), sc.n_total, sc.grid, P.eps, flags.as<uint32_t>(), s); });
-        run(h, "scan", [&] { scan_u32_to_u64(flags.as<uint32_t>(), pos[k]->as<uint64_t>(), sc.n_total, scratch.as<void>(), s); });
-        uint64_t n = 0;
-        CK(cudaMemcpyAsync(&n, pos[k]->as<uint64_t>() + sc.n_total, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        sc.N = n;
-        sc.noff = N;
-        N += n;
+        h->scans[k].noff = at[k];
+        h->scans[k].N = at[k + 1] - at[k];
     }
+    const uint64_t N = at[S];
     if (N >= 0xffffffffull) throw Error(MUTO_ERR_CAPACITY, "more than 2^32-1 kept muons");
     h->N = N;
     h->kept.alloc(std::max<uint64_t>(N, 1) * sizeof(uint32_t), &h->dev_bytes);
@@ -1052,24 +1239,26 @@ void prepare_em(muto_handle* h) {
     DevMem counts;
     counts.alloc(std::max<uint64_t>(N, 1) * sizeof(uint32_t), &h->dev_bytes);
     ph.reset(new HostPhase(h, "info_count"));
-    for (size_t k = 0; k < S; ++k) {
+    fan_scans(h, [&](size_t k, cudaStream_t on) {
         const auto& sc = h->scans[k];
         const muto_ray* r = h->scan_rays(k);
-        uint32_t* kept = h->kept.as<uint32_t>() + sc.noff;
+        const uint32_t* kept = h->kept.as<uint32_t>() + sc.noff;
         double* scat = h->scat.as<double>() + 3 * sc.noff;
-        run(h, "keep_flags", [&] { launch_keep_flags(r, sc.n_total, sc.grid, P.eps, flags.as<uint32_t>(), s); });
-        run(h, "compact", [&] { launch_compact(flags.as<uint32_t>(), pos[k]->as<uint64_t>(), sc.n_total, kept, s); });
+        run(h, "compact", [&] {
+            launch_compact(flags.as<uint32_t>() + first[k], pos.as<uint64_t>() + first[k], sc.n_total,
+                           h->kept.as<uint32_t>(), on);
+        });
         run(h, "muon_info", [&] {
             launch_muon_info<Real>(r, kept, sc.N, sc.grid, P.eps, P.has_energy, h->sd.as<R4>() + sc.noff,
-                                   h->pr2.as<Real>() + sc.noff, scat, h->pr64.as<double>() + sc.noff, s);
+                                   h->pr2.as<Real>() + sc.noff, scat, h->pr64.as<double>() + sc.noff, on);
         });
         if (h->lists != kListsRecompute)
             run(h, "path_bound", [&] {
-                launch_path_bound(r, kept, scat, sc.N, sc.grid, P.straight_line, counts.as<uint32_t>() + sc.noff, s);
+                launch_path_bound(r, kept, scat, sc.N, sc.grid, P.straight_line, counts.as<uint32_t>() + sc.noff, on);
             });
-    }
+    });
     flags.release();
-    pos.clear();
+    pos.release();
     if (scratch.bytes() < scan_scratch_bytes(std::max<uint64_t>(N, V) + 1))
         scratch.alloc(scan_scratch_bytes(std::max<uint64_t>(N, V) + 1), &h->dev_bytes);
     h->mult.alloc(V * sizeof(uint32_t), &h->dev_bytes);
@@ -1214,12 +1403,7 @@ void prepare_em(muto_handle* h) {
             h->vox_streamed = P.voxel_stream_above < 0 ? 0u
                               : vox_streamed_mask(static_cast<uint32_t>(std::min<long long>(P.voxel_stream_above, 0xffffffffLL)));
             h->keys.alloc((Pn + kPad) * sizeof(typename KeyOf<Real>::type), &h->dev_bytes);
-            em_voxel_occupancy<Real, Real>(h->vox_blocks_real);
-            em_voxel_occupancy<Real, double>(h->vox_blocks_f64);
-            for (int c = 0; c < 2 * kVoxClasses; ++c) {
-                h->vox_blocks_real[c] *= h->num_sms;
-                h->vox_blocks_f64[c] *= h->num_sms;
-            }
+            voxel_occupancy<Real>(h);
         }
     }
     scratch.release();
@@ -1291,7 +1475,9 @@ void prepare_em(muto_handle* h) {
         if (h->lists == kListsMuonMajor) h->kvec.alloc((N + kPad) * sizeof(R4), &h->dev_bytes);
         h->kslot.release();
     }
-    {
+    if (constant_start(h)) {
+        run(h, "image", [&] { launch_fill<Real>(h->lam.as<Real>(), V, static_cast<Real>(P.initialize_value), s); });
+    } else {
         std::vector<Real> init_r(init.begin(), init.end());
         CK(cudaMemcpyAsync(h->lam.as<void>(), init_r.data(), V * sizeof(Real), cudaMemcpyHostToDevice, s));
         CK(cudaStreamSynchronize(s));
@@ -1957,21 +2143,48 @@ void check_handle(muto_handle* h) {
     if (!h) throw Error(MUTO_ERR_ARG, "null handle");
 }
 
+// Images cross as doubles, converted on the device (on the host a 256 x 256 x 128
+// image cost 9 ms a direction), kImageChunk voxels at a time.
+constexpr uint64_t kImageChunk = uint64_t(1) << 25;
+
+template <typename Real>
+void download_voxels(muto_handle* h, uint64_t first, uint64_t n, double* out) {
+    cudaStream_t s = h->stream;
+    if constexpr (std::is_same<Real, double>::value) {
+        CK(cudaMemcpyAsync(out, h->lam.as<double>() + first, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    } else {
+        DevMem wide;
+        wide.alloc(std::min(n, kImageChunk) * sizeof(double), &h->dev_bytes);
+        for (uint64_t k = 0; k < n; k += kImageChunk) {
+            const uint64_t m = std::min(kImageChunk, n - k);
+            run(h, "image", [&] { launch_widen(h->lam.as<float>() + first + k, wide.as<double>(), m, s); });
+            CK(cudaMemcpyAsync(out + k, wide.as<double>(), m * sizeof(double), cudaMemcpyDeviceToHost, s));
+        }
+    }
+    CK(cudaStreamSynchronize(s));
+}
+
 template <typename Real>
 void download_image(muto_handle* h, double* out) {
-    const uint64_t V = h->V();
-    std::vector<Real> tmp(V);
-    CK(cudaMemcpyAsync(tmp.data(), h->lam.as<Real>(), V * sizeof(Real), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    for (uint64_t j = 0; j < V; ++j) out[j] = static_cast<double>(tmp[j]);
+    download_voxels<Real>(h, 0, h->V(), out);
 }
 
 template <typename Real>
 void upload_image(muto_handle* h, const double* in) {
     const uint64_t V = h->V();
-    std::vector<Real> tmp(in, in + V);
-    CK(cudaMemcpyAsync(h->lam.as<Real>(), tmp.data(), V * sizeof(Real), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    cudaStream_t s = h->stream;
+    if constexpr (std::is_same<Real, double>::value) {
+        CK(cudaMemcpyAsync(h->lam.as<double>(), in, V * sizeof(double), cudaMemcpyHostToDevice, s));
+    } else {
+        DevMem wide;
+        wide.alloc(std::min(V, kImageChunk) * sizeof(double), &h->dev_bytes);
+        for (uint64_t k = 0; k < V; k += kImageChunk) {
+            const uint64_t m = std::min(kImageChunk, V - k);
+            CK(cudaMemcpyAsync(wide.as<double>(), in + k, m * sizeof(double), cudaMemcpyHostToDevice, s));
+            run(h, "image", [&] { launch_copy_to<Real>(wide.as<double>(), h->lam.as<Real>() + k, m, s); });
+        }
+    }
+    CK(cudaStreamSynchronize(s));
 }
 
 // ---------------------------------------------------------------------------
@@ -2171,14 +2384,12 @@ int muto_create(const char* method, const char* config_json, muto_handle** out) 
         int optin = 0;
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
         h->smem_optin = static_cast<size_t>(optin);
-        CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&h->fan.fork, cudaEventDisableTiming));
-        for (int k = 0; k < ClassFan::kSide; ++k) {
-            CK(cudaStreamCreateWithFlags(&h->fan.side[k], cudaStreamNonBlocking));
-            CK(cudaEventCreateWithFlags(&h->fan.join[k], cudaEventDisableTiming));
-            h->fan.n = k + 1;
-        }
-        for (cudaEvent_t& e : h->ov_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        static_cast<HandleStreams&>(h->streams) = HandleStreams::take(h->device);
+        h->stream = h->streams.stream;
+        h->fan = h->streams.fan;
+        static_assert(HandleStreams::kOverlap == muto_handle::kOverlapChunks + 1, "one event a chunk and one more");
+        std::copy(std::begin(h->streams.ov_ev), std::end(h->streams.ov_ev), std::begin(h->ov_ev));
+        AllocScope scope(h->stream);
         alloc_counters(h.get());
         CK(cudaStreamSynchronize(h->stream));
     });
@@ -2698,14 +2909,8 @@ int muto_batch_get_image(muto_handle* h, uint32_t scan, double* out, uint64_t le
         if (scan >= h->scans.size()) throw Error(MUTO_ERR_ARG, "no such scan");
         const auto& sc = h->scans[scan];
         if (len != sc.V) throw Error(MUTO_ERR_ARG, "image length does not match the scan's grid");
-        const size_t es = h->fp64() ? sizeof(double) : sizeof(float);
-        std::vector<unsigned char> tmp(len * es);
-        CK(cudaMemcpyAsync(tmp.data(), static_cast<const unsigned char*>(h->lam.as<void>()) + sc.voff * es, len * es,
-                           cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        for (uint64_t j = 0; j < len; ++j)
-            out[j] = h->fp64() ? reinterpret_cast<const double*>(tmp.data())[j]
-                               : static_cast<double>(reinterpret_cast<const float*>(tmp.data())[j]);
+        if (h->fp64()) download_voxels<double>(h, sc.voff, len, out);
+        else download_voxels<float>(h, sc.voff, len, out);
     });
 }
 

@@ -131,7 +131,18 @@ __global__ void k_add_u64(uint64_t* __restrict__ a, uint64_t n, uint64_t add) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) a[i] += add;
 }
+__global__ void k_gather_u64(const uint64_t* __restrict__ src, const uint64_t* __restrict__ at, uint64_t n,
+                             uint64_t* __restrict__ out) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = src[at[i]];
+}
 }  // namespace
+
+void launch_gather_u64(const uint64_t* src, const uint64_t* at, uint64_t n, uint64_t* out, cudaStream_t s) {
+    if (n == 0) return;
+    k_gather_u64<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(src, at, n, out);
+    count_launches(1);
+}
 
 void launch_add_u64(uint64_t* a, uint64_t n, uint64_t add, cudaStream_t s) {
     if (n == 0 || add == 0) return;
