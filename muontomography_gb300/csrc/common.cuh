@@ -499,6 +499,15 @@ inline MapParams map_params(double beta, double p, double delta, double eps, boo
     return MapParams{beta, p, delta, eps, all_neighbours ? 1 : 0, add_object_prior ? 1 : 0, newton_max_iter,
                      beta * p != 0.0 ? 1.0 / (beta * p) : __builtin_nan("")};
 }
+// x^e with e = (p - 2) / 2
+enum MapPower { kMapAny = 0, kMapOne = 1, kMapTwo = 2 };  // p: any, 1, 2
+
+template <int POWER>
+__device__ __forceinline__ double map_q(double x, double e) {
+    if (POWER == kMapTwo) return 1.0;
+    if (POWER == kMapOne) return rsqrt(x);
+    return e == 0.0 ? 1.0 : pow(x, e);
+}
 template <typename LamT>
 void launch_map_voxel(const LamT* last, double* ml_inout, const uint32_t* mult, DevGrid g, MapParams mp,
                       Counters* ctr, cudaStream_t s);
@@ -510,10 +519,9 @@ void launch_fill(Real* out, uint64_t n, Real value, cudaStream_t s);
 
 // adjoint.cu
 template <typename Real>
-void launch_exp_lambda(const double* loglam, const uint32_t* mult, uint32_t V, Real* lam, cudaStream_t s);
-// adds d prior / d log(lambda) to grad and the prior's value to *value;
-// dl_scratch: V doubles, zero on entry and on return
-void launch_prior(const double* lam64, const uint32_t* mult, DevGrid g, MapParams mp, double* dl_scratch, double* grad,
+void launch_exp_lambda(const double* loglam, const uint32_t* mult, uint32_t V, double* lam64, Real* lam, cudaStream_t s);
+// adds the prior's value to *value and, unless grad is null, d prior / d log(lambda) to grad
+void launch_prior(const double* lam64, const uint32_t* mult, DevGrid g, MapParams mp, int num_sms, double* grad,
                   double* value, cudaStream_t s);
 
 // gen.cu

@@ -781,15 +781,6 @@ __global__ void k_finalize_cost(Counters* ctr, double n_muons, double* hist, uin
 //               values relative to the ML candidate's.
 // 1.05 M voxels, 26 neighbours, p = 2: 0.36 ms; 1.52 ms with Newton in FP64 from
 // the start, a logarithm a candidate and two passes over the neighbours.
-enum MapPower { kMapAny = 0, kMapOne = 1, kMapTwo = 2 };  // p: any, 1, 2
-
-template <int POWER>
-__device__ __forceinline__ double map_q(double x, double e) {
-    if (POWER == kMapTwo) return 1.0;
-    if (POWER == kMapOne) return rsqrt(x);
-    return e == 0.0 ? 1.0 : pow(x, e);
-}
-
 // x^3 + ca x^2 + cb x + cc and the root of it that the reference's iteration
 // finds: cubicEqnSolver, :353-406, Newton capped at newton_max_iter.
 __device__ __forceinline__ double map_cubic(double ca, double cb, double cc, const MapParams& mp, bool* nonconv) {

@@ -547,7 +547,7 @@ struct muto_handle {
     // PoCA outputs
     DevMem img64, weight, assign;
     // adjoint scratch
-    DevMem lam64, grad, dl, fval, loglam;
+    DevMem lam64, grad, fval, loglam;
     // graph
     cudaGraphExec_t graph = nullptr;
     size_t graph_prof_first = 0, graph_prof_last = 0;
@@ -2198,21 +2198,19 @@ double nll_eval(muto_handle* h, const double* loglam_host, double* grad_host) {
     if (h->loglam.empty()) h->loglam.alloc(V * sizeof(double), &h->dev_bytes);
     if (h->lam64.empty()) h->lam64.alloc(V * sizeof(double), &h->dev_bytes);
     if (h->grad.empty()) h->grad.alloc(V * sizeof(double), &h->dev_bytes);
-    if (h->dl.empty()) {
-        h->dl.alloc(V * sizeof(double), &h->dev_bytes);
-        CK(cudaMemsetAsync(h->dl.as<void>(), 0, V * sizeof(double), s));
-    }
     if (h->fval.empty()) h->fval.alloc(sizeof(double), &h->dev_bytes);
     CK(cudaMemcpyAsync(h->loglam.as<double>(), loglam_host, V * sizeof(double), cudaMemcpyHostToDevice, s));
     // lambda in FP64 (prior, chain rule) and in the storage precision (muon pass)
-    run(h, "exp_lambda", [&] { launch_exp_lambda<double>(h->loglam.as<double>(), h->mult.as<uint32_t>(), static_cast<uint32_t>(V), h->lam64.as<double>(), s); });
     DevMem lamR;
     const Real* lam_r = reinterpret_cast<const Real*>(h->lam64.as<double>());
     if (!std::is_same<Real, double>::value) {
         lamR.alloc(V * sizeof(Real), &h->dev_bytes);
-        run(h, "exp_lambda", [&] { launch_exp_lambda<Real>(h->loglam.as<double>(), h->mult.as<uint32_t>(), static_cast<uint32_t>(V), lamR.as<Real>(), s); });
         lam_r = lamR.as<Real>();
     }
+    run(h, "exp_lambda", [&] {
+        launch_exp_lambda<Real>(h->loglam.as<double>(), h->mult.as<uint32_t>(), static_cast<uint32_t>(V),
+                                h->lam64.as<double>(), lamR.empty() ? nullptr : lamR.as<Real>(), s);
+    });
     Counters c0;
     CK(cudaMemcpyAsync(&c0, h->ctr(), sizeof(Counters), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -2239,14 +2237,10 @@ double nll_eval(muto_handle* h, const double* loglam_host, double* grad_host) {
     const Params& P = h->P;
     if (h->method == kMap) {
         const MapParams mp = map_params(P.beta, P.p, P.delta, P.eps, P.all_neighbours, P.add_object_prior, P.newton_max_iter);
-        DevMem gdummy;
-        double* gp = h->grad.as<double>();
-        if (!grad_host) {
-            gdummy.alloc(V * sizeof(double), &h->dev_bytes);
-            gp = gdummy.as<double>();
-        }
-        run(h, "prior", [&] { launch_prior(h->lam64.as<double>(), h->mult.as<uint32_t>(), make_dev_grid(h->grid), mp, h->dl.as<double>(), gp, h->fval.as<double>(), s); });
-        CK(cudaStreamSynchronize(s));
+        run(h, "prior", [&] {
+            launch_prior(h->lam64.as<double>(), h->mult.as<uint32_t>(), make_dev_grid(h->grid), mp, h->num_sms,
+                         grad_host ? h->grad.as<double>() : nullptr, h->fval.as<double>(), s);
+        });
     }
     Counters c1;
     double prior = 0.0;
