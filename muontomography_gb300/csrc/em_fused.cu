@@ -1040,18 +1040,47 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
     if (lane == 0 && singular) atomicAdd(&a.ctr->singular, static_cast<unsigned long long>(singular));
 }
 
-// The cost of every muon (src/MutoMLSD.cpp:465-468) from the sums that
-// k_em_once left, in FP64, a muon per lane.
-__global__ void __launch_bounds__(256) k_once_cost(FusedArgs<float> a, const float4* __restrict__ sums) {
-    const uint64_t m = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    double cost = 0.0;
-    unsigned long long singular = 0;  // counted by k_em_once
-    if (m < a.N) {
-        const float4 c = sums[m], v = a.sd[m];
-        float k0, k1, k2;
-        muon_coefficients<float>(c.x, c.y, c.z, a.pr2[m], v, a.E00, a.E01, a.E11, true, k0, k1, k2, cost, singular);
+// The cost of every muon (src/MutoMLSD.cpp:465-468) from the sums that k_em_once
+// left, in FP64.  Bound by FP64 work, most of it the logarithm and the division: a
+// thread takes kCostMuons muons with one logarithm of the product of their
+// determinants' mantissas (each product's exponent is moved to an integer, which
+// is exact), and their divisions' latencies overlap.  897 k muons: 81 us;
+// 122 us with a logarithm a muon.
+constexpr int kCostMuons = 4, kCostThreads = 256;
+__global__ void __launch_bounds__(kCostThreads) k_once_cost(FusedArgs<float> a, const float4* __restrict__ sums) {
+    const uint64_t m0 = static_cast<uint64_t>(blockIdx.x) * (kCostMuons * kCostThreads) + threadIdx.x;
+    float4 cs[kCostMuons], vs[kCostMuons];
+    float ps[kCostMuons];
+#pragma unroll
+    for (int u = 0; u < kCostMuons; ++u) {  // (a muon past the end repeats the last one's loads)
+        const uint64_t m = m0 + u * kCostThreads < a.N ? m0 + u * kCostThreads : a.N - 1;
+        cs[u] = sums[m];
+        vs[u] = a.sd[m];
+        ps[u] = a.pr2[m];
     }
-    flush_counters<256>(cost, 0ull, 1, a.ctr);
+    double cost = 0.0, prod = 1.0;
+    int ex = 0;
+#pragma unroll
+    for (int u = 0; u < kCostMuons; ++u) {
+        if (m0 + u * kCostThreads >= a.N) continue;
+        const float4 c = cs[u], v = vs[u];
+        const double p2 = ps[u];
+        const double S00 = p2 * c.x + a.E00, S01 = p2 * c.y + a.E01, S11 = p2 * c.z + a.E11;
+        const double det = S00 * S11 - S01 * S01;
+        if (!(det > 1e-12)) continue;  // cost 0; counted by k_em_once
+        const double sx = v.x, dx = v.y, sy = v.z, dy = v.w;
+        cost += ((sx * sx + sy * sy) * S11 + (dx * dx + dy * dy) * S00 - (sx * dx + sy * dy) * 2.0 * S01) / det;
+        if (det > 1.0e300) {
+            cost += 2.0 * log(det);
+            continue;
+        }
+        const double q = prod * det;  // a normal number: 1e-12 < q < 2e300
+        const int hi = __double2hiint(q), e = (hi >> 20) - 1023;
+        ex += e;
+        prod = __hiloint2double(hi - (e << 20), __double2loint(q));  // [1, 2)
+    }
+    cost = 0.5 * cost + log(prod) + ex * 0.69314718055994530942;  // ln 2
+    flush_counters<kCostThreads>(cost, 0ull, 1, a.ctr);
 }
 
 }  // namespace
@@ -1077,7 +1106,8 @@ void launch_em_once(const FusedArgs<float>& a, int group, float4* sums, int num_
     if (group <= 16) run_once<16, kOnceHeld, 6>(a, sums, num_sms, s);
     else run_once<32, kOnceHeld, 7>(a, sums, num_sms, s);
     if (sums) {
-        k_once_cost<<<static_cast<unsigned>((static_cast<uint64_t>(a.N) + 255) / 256), 256, 0, s>>>(a, sums);
+        constexpr uint64_t per = kCostMuons * kCostThreads;
+        k_once_cost<<<static_cast<unsigned>((static_cast<uint64_t>(a.N) + per - 1) / per), kCostThreads, 0, s>>>(a, sums);
         count_launches(1);
     }
 }
