@@ -4,9 +4,10 @@
 // The reference fits each half of a record (src/MutoFile.cpp:248-304) with
 // Eigen's JacobiSVD of the centred hits and takes the first right singular
 // vector as the direction.  That vector is the principal axis of the hits'
-// 3x3 scatter matrix, found here by cyclic Jacobi rotations on the
-// symmetric matrix (Golub & Van Loan, "Matrix Computations", sec. 8.5),
-// then oriented with d_z > 0 (the SVD leaves the sign open).  The point is
+// 3x3 scatter matrix, found here by squaring the matrix until one axis is left
+// (hits along a line), or else by cyclic Jacobi rotations on the symmetric
+// matrix (Golub & Van Loan, "Matrix Computations", sec. 8.5), then oriented
+// with d_z > 0 (the SVD leaves the sign open).  The point is
 // the line at the layer next to the grid: pin on layer n_middle-1, pout on
 // layer n_middle.
 //
@@ -90,6 +91,44 @@ MUTO_FIT_HD inline void principal_axis(double a[3][3], double* out) {
     for (int k = 0; k < 3; ++k) out[k] = v[k][best];
 }
 
+// The same axis, not normalised, where one eigenvalue stands out: the eigenvalue
+// ratio of a's powers falls as the square of the power before, so a column of a^4
+// is the axis to the last bit for hits along a line (ratio up to 9e-5), of a^8 and
+// a^16 for ratios up to 0.009 and 0.09.  A squaring takes 24 operations and a
+// rotation above 110, three to five sweeps of three being needed.  A matrix's
+// ratio (e2 = the sum of the 2x2 principal minors, over its trace squared) comes
+// with its square: trace(a)^2 - trace(a^2) = 2 e2.  Refused, for the rotations to
+// decide: no axis that stands out, powers that leave the range, axes within 1e-6
+// of the horizontal (whose sign the orientation does not settle), inf and NaN.
+MUTO_FIT_HD inline bool outstanding_axis(const double a[3][3], double* out) {
+    double m00 = a[0][0], m01 = a[0][1], m02 = a[0][2], m11 = a[1][1], m12 = a[1][2], m22 = a[2][2];
+    bool alone = false;
+    for (int k = 0; k < 4 && !alone; ++k) {
+        const double q01 = fm(m01, m01), q02 = fm(m02, m02), q12 = fm(m12, m12);
+        const double n00 = fa(fa(fm(m00, m00), q01), q02);
+        const double n11 = fa(fa(fm(m11, m11), q01), q12);
+        const double n22 = fa(fa(fm(m22, m22), q02), q12);
+        const double n01 = fa(fm(m01, fa(m00, m11)), fm(m02, m12));
+        const double n02 = fa(fm(m02, fa(m00, m22)), fm(m01, m12));
+        const double n12 = fa(fm(m12, fa(m11, m22)), fm(m01, m02));
+        const double tr = fa(fa(m00, m11), m22), tr2 = fm(tr, tr);
+        alone = fs(tr2, fa(fa(n00, n11), n22)) <= fm(1.4901161193847656e-08, tr2);  // 2^-26: the square's ratio is below 2^-54
+        m00 = n00, m01 = n01, m02 = n02, m11 = n11, m12 = n12, m22 = n22;
+    }
+    double top;
+    if (m22 >= m00 && m22 >= m11) {
+        top = m22;
+        out[0] = m02, out[1] = m12, out[2] = m22;
+    } else if (m11 >= m00) {
+        top = m11;
+        out[0] = m01, out[1] = m11, out[2] = m12;
+    } else {
+        top = m00;
+        out[0] = m00, out[1] = m01, out[2] = m02;
+    }
+    return alone && top >= 1e-140 && top <= 1e140 && fabs(out[2]) >= fm(1e-6, top);
+}
+
 // Centroid c and unit direction d (d_z >= 0) of the n hits (x, y, z);
 // src/MutoFile.cpp:262-276 and :287-299.
 MUTO_FIT_HD inline void fit_line(const double* x, const double* y, const double* z, int n, double* c, double* d) {
@@ -105,9 +144,10 @@ MUTO_FIT_HD inline void fit_line(const double* x, const double* y, const double*
     for (int i = 0; i < n; ++i) {
         const double r[3] = {fs(x[i], c[0]), fs(y[i], c[1]), fs(z[i], c[2])};
         for (int p = 0; p < 3; ++p)
-            for (int q = 0; q < 3; ++q) a[p][q] = fa(a[p][q], fm(r[p], r[q]));
+            for (int q = p; q < 3; ++q) a[p][q] = fa(a[p][q], fm(r[p], r[q]));
     }
-    principal_axis(a, d);
+    a[1][0] = a[0][1], a[2][0] = a[0][2], a[2][1] = a[1][2];
+    if (!outstanding_axis(a, d)) principal_axis(a, d);
     const double nrm = sqrt(fa(fa(fm(d[0], d[0]), fm(d[1], d[1])), fm(d[2], d[2])));
     if (!(nrm > 0)) {
         d[0] = d[1] = 0.0;
