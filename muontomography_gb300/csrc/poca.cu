@@ -30,6 +30,7 @@ struct WeightSink {
         const uint64_t j = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * (y + static_cast<uint64_t>(ny) * z);
         atomicAdd(weight + j, length_weighted ? l : dz);
     }
+    __device__ void second() { skip_scat = !length_weighted; }
 };
 
 // Per ray: PoCA point and binning (PoCut's voxel); kept rays are appended to a.walk (warp-aggregated) for the
@@ -159,7 +160,6 @@ __global__ void __launch_bounds__(128) k_poca_walk(PocaArgs a, DevGrid g) {
     const uint64_t n = *a.walk_count;
     const double zmin = a.rays[0].pout[2], zmax = a.rays[0].pin[2];
     const uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const unsigned lanes = walk_lanes(t < n);
     if (t < n) {
         const uint32_t i = a.walk[a.walk_order ? a.walk_order[t] : t];
         const muto_ray r = a.rays[i];
@@ -174,21 +174,8 @@ __global__ void __launch_bounds__(128) k_poca_walk(PocaArgs a, DevGrid g) {
         else
             atomicAdd(a.img + (xyz[0] + static_cast<uint64_t>(g.n[0]) * (xyz[1] + static_cast<uint64_t>(g.n[1]) * xyz[2])), v);
         WeightSink sink{a.weight, g.n[0], g.n[1], g.n[2], g.w[2], a.length_weighted, 0, xyz[0], xyz[1], xyz[2]};
-        double from[3] = {r.pin[0], r.pin[1], r.pin[2]}, to[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) to[k] = a.straight ? r.pout[k] : ps[k];
-        // one copy of the walk's code for both halves
-#pragma unroll 1
-        for (int half = 0; half < (a.straight ? 1 : 2); ++half) {
-            siddon_walk(g, from, to, sink);
-            sink.skip_scat = !a.length_weighted;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                from[k] = ps[k];
-                to[k] = r.pout[k];
-            }
-            __syncwarp(lanes);
-        }
+        if (a.straight) siddon_walk(g, r.pin, r.pout, sink);
+        else siddon_walk_two(g, r.pin, ps, r.pout, sink);
     }
 }
 

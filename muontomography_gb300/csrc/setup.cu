@@ -218,6 +218,7 @@ struct PathSink {
         }
         ++n;
     }
+    __device__ void second() { merge = true; }
 };
 
 // The FP64 walk of every kept muon into bounded slots [boff[i], boff[i+1]) -
@@ -232,28 +233,12 @@ __global__ void __launch_bounds__(128) k_path_walk(const muto_ray* __restrict__ 
                                                    double* __restrict__ l64, double* __restrict__ T,
                                                    uint32_t* __restrict__ counts, Counters* ctr, uint64_t slot_base) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const unsigned lanes = walk_lanes(i < n);
     if (i >= n) return;
     const uint64_t b = boff[i] - slot_base;
     const muto_ray& r = rays[kept[i]];
     const double ps[3] = {scat[3 * i], scat[3 * i + 1], scat[3 * i + 2]};
     PathSink s{vidx + b, l64 + b, 0u, static_cast<uint32_t>(boff[i + 1] - slot_base - b), g.n[0], g.n[0] * g.n[1], false};
-    bool overflow = false;
-    double from[3] = {r.pin[0], r.pin[1], r.pin[2]}, to[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) to[k] = straight ? r.pout[k] : ps[k];
-    // one copy of the walk's code for both halves
-#pragma unroll 1
-    for (int half = 0; half < (straight ? 1 : 2); ++half) {
-        overflow = siddon_walk(g, from, to, s) < 0 || overflow;
-        s.merge = true;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            from[k] = ps[k];
-            to[k] = r.pout[k];
-        }
-        __syncwarp(lanes);
-    }
+    const bool overflow = straight ? siddon_walk(g, r.pin, r.pout, s) < 0 : !siddon_walk_two(g, r.pin, ps, r.pout, s);
     if (overflow) {  // dropped, like the count walk does
         atomicAdd(&ctr->overflow, 1ull);
         s.n = 0;
