@@ -125,7 +125,8 @@ void launch_path_walk(const muto_ray* rays, const uint32_t* kept, const double* 
                       uint32_t* counts, Counters* ctr, cudaStream_t s);
 // the walked slots to the exact slots off: the mixed form's lists with their tails
 void launch_path_finish(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
-                        const uint32_t* vidx_b, const double* l64, uint32_t* vidx, float* L, float* T, cudaStream_t s);
+                        const uint32_t* vidx_b, const double* l64, uint32_t* vidx, float* L, float* T,
+                        double mean_bound, cudaStream_t s);
 // and the FP64 form's
 void launch_path_compact(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
                          const uint32_t* vidx_b, const double* L_b, const double* T_b, uint32_t* vidx, double* L,

@@ -1029,7 +1029,7 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
                                     h->T.as<Real>(), s);
             else
                 launch_path_finish(boff.as<uint64_t>() + m, slot0, h->off.as<uint64_t>() + m, nc, vidx_b.as<uint32_t>(),
-                                   l64_b.as<double>(), h->vidx.as<uint32_t>(), h->L.as<Real>(), h->T.as<Real>(), s);
+                                   l64_b.as<double>(), h->vidx.as<uint32_t>(), h->L.as<Real>(), h->T.as<Real>(), avg, s);
         });
     };
     if (Pb <= cap) {  // one chunk: every scan's walk, then one scan and one copy
@@ -1058,7 +1058,9 @@ void fill_lists(muto_handle* h, DevMem& counts, DevMem& scratch, std::vector<uin
                     if (b[1] - b[0] <= cap || nc == 1) break;
                     nc = (nc + 1) / 2;
                 }
-                if (b[1] - b[0] > cap) throw Error(MUTO_ERR_CAPACITY, "a muon's path bound exceeds the set-up scratch");
+                // (a bound is even, and the scratch has room beyond cap)
+                if (b[1] - b[0] > cap + (cap & 1))
+                    throw Error(MUTO_ERR_CAPACITY, "a muon's path bound exceeds the set-up scratch");
                 run(h, "siddon_fill", [&] {
                     launch_path_walk(h->scan_rays(k), h->kept.as<uint32_t>() + m, h->scat.as<double>() + 3 * m,
                                      boff.as<uint64_t>() + m, b[0], nc, sc.grid, P.straight_line, vidx_b.as<uint32_t>(),

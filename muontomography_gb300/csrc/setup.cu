@@ -189,12 +189,14 @@ __global__ void k_path_bound(const muto_ray* __restrict__ rays, const uint32_t* 
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const muto_ray& r = rays[kept[i]];
+    uint32_t b;
     if (straight) {
-        bounds[i] = walk_bound(g, r.pin, r.pout);
+        b = walk_bound(g, r.pin, r.pout);
     } else {
         const double ps[3] = {scat[3 * i], scat[3 * i + 1], scat[3 * i + 2]};
-        bounds[i] = walk_bound(g, r.pin, ps) + walk_bound(g, ps, r.pout);
+        b = walk_bound(g, r.pin, ps) + walk_bound(g, ps, r.pout);
     }
+    bounds[i] = (b + 1u) & ~1u;  // even: the walk stores two pairs at once
 }
 
 // The merged path of one muon into its bounded slots: every voxel as it is
@@ -203,22 +205,45 @@ __global__ void k_path_bound(const muto_ray* __restrict__ rays, const uint32_t* 
 struct PathSink {
     uint32_t* vidx;
     double* l64;
-    uint32_t n, cap;       // pairs written, slots
+    uint32_t n, cap;       // pairs seen, slots (an even number, from an even slot on)
     uint32_t nx, nxy;
     bool merge;            // the next voxel is the out-half's first
+    // the last pair, or two from an even one on: a store takes a cycle a lane here
+    // (every lane has its own line), so two pairs share one: 963 k walks of
+    // 220 pairs in 3.3 ms, 4.1 ms with a store a pair
+    uint32_t j0, j1;
+    double l0, l1;
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
         if (merge) {
             merge = false;
-            if (n > 0 && n <= cap) l64[n - 1] = dadd(l64[n - 1], l);
+            const double sum = dadd((n & 1u) ? l0 : l1, l);
+            if (n & 1u) l0 = sum;
+            else if (n > 0) l1 = sum;
             return;
         }
-        if (n < cap) {  // (a path longer than its bound is counted by the caller)
-            vidx[n] = x + y * nx + z * nxy;  // xyz2index, include/MutoMLSD.h:76
-            l64[n] = l;
+        const uint32_t j = x + y * nx + z * nxy;  // xyz2index, include/MutoMLSD.h:76
+        if (n & 1u) {
+            j1 = j;
+            l1 = l;
+        } else {
+            flush();
+            j0 = j;
+            l0 = l;
         }
         ++n;
     }
     __device__ void second() { merge = true; }
+    // the pairs held, to their slots (a path longer than its bound is counted by the caller)
+    __device__ void flush() {
+        if (n == 0 || n > cap) return;
+        if (n & 1u) {
+            vidx[n - 1] = j0;
+            l64[n - 1] = l0;
+        } else {
+            *reinterpret_cast<uint2*>(vidx + n - 2) = make_uint2(j0, j1);
+            *reinterpret_cast<double2*>(l64 + n - 2) = make_double2(l0, l1);
+        }
+    }
 };
 
 // The FP64 walk of every kept muon into bounded slots [boff[i], boff[i+1]) -
@@ -237,8 +262,10 @@ __global__ void __launch_bounds__(128) k_path_walk(const muto_ray* __restrict__ 
     const uint64_t b = boff[i] - slot_base;
     const muto_ray& r = rays[kept[i]];
     const double ps[3] = {scat[3 * i], scat[3 * i + 1], scat[3 * i + 2]};
-    PathSink s{vidx + b, l64 + b, 0u, static_cast<uint32_t>(boff[i + 1] - slot_base - b), g.n[0], g.n[0] * g.n[1], false};
+    PathSink s{vidx + b, l64 + b, 0u, static_cast<uint32_t>(boff[i + 1] - slot_base - b), g.n[0], g.n[0] * g.n[1], false,
+               0u, 0u, 0.0, 0.0};
     const bool overflow = straight ? siddon_walk(g, r.pin, r.pout, s) < 0 : !siddon_walk_two(g, r.pin, ps, r.pout, s);
+    s.flush();
     if (overflow) {  // dropped, like the count walk does
         atomicAdd(&ctr->overflow, 1ull);
         s.n = 0;
@@ -259,45 +286,84 @@ __global__ void __launch_bounds__(128) k_path_walk(const muto_ray* __restrict__ 
 
 // The mixed form's lists from the walked slots, a warp per muon, coalesced: the
 // voxel, L and the tail T to the exact slots.  The reference sums a tail one
-// length after the other from the path's end; here 32 lengths at a time by a
-// scan.  The two FP64 sums differ by at most (m + 16) units of their last place
-// (m lengths, each sum's roundings), so they round to the same FP32 value unless
-// the scan's sum lies that near to the middle of two: a muon with such a tail
-// (one in some thousands) is summed again in the reference's order.  FP64
-// operations a pair: a quarter, against one on each lane of a thread-per-muon
-// loop with 14 of 32 lanes at work.
-__global__ void __launch_bounds__(256) k_path_finish(const uint64_t* __restrict__ boff, uint64_t slot_base,
-                                                     const uint64_t* __restrict__ off, uint64_t n,
-                                                     const uint32_t* __restrict__ vidx_b,
-                                                     const double* __restrict__ l64, uint32_t* __restrict__ vidx,
-                                                     float* __restrict__ L, float* __restrict__ T) {
+// length after the other from the path's end; here 32 EACH lengths at a time, EACH a
+// lane and a scan over the lanes.  The two FP64 sums differ by at most
+// m + m / 64 + 16 units of their last place (m lengths, each sum's roundings), so
+// they round to the same FP32 value unless the scan's sum lies that near to the
+// middle of two: a muon with such a tail (one in some thousands) is summed again in
+// the reference's order.  Bound by FP64 work: for EACH = 4, 13 additions and 8
+// conversions a lane for 128 pairs (with a length a lane, 28 and 8): 963 k paths of
+// 220 pairs in 2.6 ms against 3.8 ms.  Shorter paths would leave most of
+// 128 places empty: EACH = 2 for mean bounds up to 112 pairs.
+constexpr int kFinishThreads = 256;
+template <int EACH>
+__global__ void __launch_bounds__(kFinishThreads) k_path_finish(const uint64_t* __restrict__ boff, uint64_t slot_base,
+                                                                const uint64_t* __restrict__ off, uint64_t n,
+                                                                const uint32_t* __restrict__ vidx_b,
+                                                                const double* __restrict__ l64,
+                                                                uint32_t* __restrict__ vidx, float* __restrict__ L,
+                                                                float* __restrict__ T) {
+    constexpr int kTile = 32 * EACH;
+    __shared__ __align__(16) double held[kFinishThreads / 32][kTile];
     const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
+    double* const len = held[threadIdx.x >> 5];
+    float* const tail = reinterpret_cast<float*>(len);
     const uint64_t src = boff[i] - slot_base, dst = off[i];
     const int m = static_cast<int>(off[i + 1] - dst);
+    const int close = m + m / 64 + 16;
     double carry = 0.0;
     bool near = false;
-    for (int k0 = (m - 1) & ~31; k0 >= 0; k0 -= 32) {
-        const int k = k0 + lane;
-        const double l = k < m ? l64[src + k] : 0.0;
-        double s = l;  // of this length and those after it, up to the 32nd
+    for (int k0 = m > 0 ? (m - 1) / kTile * kTile : -1; k0 >= 0; k0 -= kTile) {
+#pragma unroll
+        for (int r = 0; r < EACH; ++r) {
+            const int k = k0 + 32 * r + lane;
+            double l = 0.0;
+            if (k < m) {
+                l = l64[src + k];
+                vidx[dst + k] = vidx_b[src + k];
+                L[dst + k] = static_cast<float>(l);
+            }
+            len[32 * r + lane] = l;
+        }
+        __syncwarp();
+        double own[EACH];  // a length and this lane's after it
+#pragma unroll
+        for (int q = 0; q < EACH; q += 2) {
+            const double2 d = reinterpret_cast<const double2*>(len)[(EACH * lane + q) / 2];
+            own[q] = d.x;
+            own[q + 1] = d.y;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = EACH - 2; q >= 0; --q) own[q] = dadd(own[q], own[q + 1]);
+        double s = own[0];  // of this lane's lengths and the later lanes'
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double t = __shfl_down_sync(kFull, s, o);
             if (lane + o < 32) s = dadd(s, t);
         }
-        const double after = __shfl_down_sync(kFull, s, 1);
-        const double t = lane < 31 ? dadd(carry, after) : carry;
-        if (k < m) {
-            vidx[dst + k] = vidx_b[src + k];
-            L[dst + k] = static_cast<float>(l);
-            T[dst + k] = static_cast<float>(t);
+        const double later = __shfl_down_sync(kFull, s, 1);
+        const double after = lane < 31 ? dadd(carry, later) : carry;
+        float tf[EACH];
+#pragma unroll
+        for (int q = 0; q < EACH; ++q) {
+            const double t = q < EACH - 1 ? dadd(after, own[q + 1]) : after;
             // 29 bits of the sum's mantissa lie below the float's last place
             const int from_middle = (__double2loint(t) & 0x1fffffff) - 0x10000000;
-            near = near || abs(from_middle) <= m + 16;
+            near = near || (k0 + EACH * lane + q < m && abs(from_middle) <= close);
+            tf[q] = static_cast<float>(t);
         }
+#pragma unroll
+        for (int q = 0; q < EACH; q += 2)
+            reinterpret_cast<float2*>(tail)[(EACH * lane + q) / 2] = make_float2(tf[q], tf[q + 1]);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < EACH; ++r)
+            if (k0 + 32 * r + lane < m) T[dst + k0 + 32 * r + lane] = tail[32 * r + lane];
         carry = dadd(carry, __shfl_sync(kFull, s, 0));
+        __syncwarp();
     }
     if (__any_sync(kFull, near) && lane == 0) {
         double t = 0.0;
@@ -584,9 +650,14 @@ void launch_path_walk(const muto_ray* rays, const uint32_t* kept, const double* 
 }
 
 void launch_path_finish(const uint64_t* boff, uint64_t slot_base, const uint64_t* off, uint64_t n,
-                        const uint32_t* vidx_b, const double* l64, uint32_t* vidx, float* L, float* T, cudaStream_t s) {
+                        const uint32_t* vidx_b, const double* l64, uint32_t* vidx, float* L, float* T,
+                        double mean_bound, cudaStream_t s) {
     if (n == 0) return;
-    k_path_finish<<<blocks_for(n * 32), kThreads, 0, s>>>(boff, slot_base, off, n, vidx_b, l64, vidx, L, T);
+    const unsigned nb = blocks_for(n * 32, kFinishThreads);
+    if (mean_bound > 112.0)
+        k_path_finish<4><<<nb, kFinishThreads, 0, s>>>(boff, slot_base, off, n, vidx_b, l64, vidx, L, T);
+    else
+        k_path_finish<2><<<nb, kFinishThreads, 0, s>>>(boff, slot_base, off, n, vidx_b, l64, vidx, L, T);
     count_launches(1);
 }
 
