@@ -128,23 +128,7 @@ private:
     std::atomic<uint64_t>* tally_ = nullptr;
 };
 
-// A non-blocking stream owned by one call, destroyed on every way out; the call's
-// allocations are ordered on it.
-struct OwnedStream {
-    cudaStream_t s = nullptr;
-    std::unique_ptr<AllocScope> scope;
-    OwnedStream() {
-        CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        scope.reset(new AllocScope(s));
-    }
-    ~OwnedStream() {
-        if (s) cudaStreamDestroy(s);
-    }
-    OwnedStream(const OwnedStream&) = delete;
-    OwnedStream& operator=(const OwnedStream&) = delete;
-};
-
-// The streams and events of one handle, from a small pool per device: creating
+// The streams and events of one handle (or call), from a small pool per device: creating
 // and destroying them takes longer than a small scan's iterations.  A set goes
 // back to the pool idle (the handle's destructor waits for its stream); the pool
 // keeps at most kKept sets a device and destroys the rest.
@@ -220,6 +204,24 @@ struct HandleStreams {
         }
         destroy();
     }
+};
+
+// A stream owned by one call, from the same pool and back to it, idle, on every way
+// out; the call's allocations are ordered on it.
+struct OwnedStream {
+    HandleStreams set;
+    cudaStream_t s = nullptr;
+    std::unique_ptr<AllocScope> scope;
+    OwnedStream() {
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        set = HandleStreams::take(dev);
+        s = set.stream;
+        scope.reset(new AllocScope(s));
+    }
+    ~OwnedStream() { set.give(); }
+    OwnedStream(const OwnedStream&) = delete;
+    OwnedStream& operator=(const OwnedStream&) = delete;
 };
 
 enum Method { kPoca, kMlsd, kMap };
