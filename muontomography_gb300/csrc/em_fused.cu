@@ -1237,7 +1237,7 @@ __global__ void __launch_bounds__(128) k_path_tails(const uint64_t* __restrict__
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint64_t b = off[i];
-    double t = 0.0;  // as k_path_fill_bounded sums them
+    double t = 0.0;  // as k_path_walk sums them
     for (uint64_t k = off[i + 1]; k-- > b;) {
         T[k] = t;
         t = dadd(t, L[k]);

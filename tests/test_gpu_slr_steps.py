@@ -15,7 +15,7 @@ from muontomography_gb300 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-# 24^3 voxels: 2 V doubles still fit shared memory (221 KB do not on every part);
+# 22^3 voxels: 2 V doubles still fit shared memory (those of 24^3, 221 KB, not on every part);
 # 30^3 do not; 48^3: paths of 48 voxels and more, wide first levels
 @pytest.mark.parametrize("n,n_muons", [(3, 301), (16, 25), (22, 3001), (30, 2003), (48, 4001)])
 @pytest.mark.parametrize("lw,energy", [(True, True), (False, False)])
