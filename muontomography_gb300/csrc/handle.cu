@@ -162,13 +162,14 @@ struct HandleStreams {
         *this = HandleStreams{};
     }
     static constexpr size_t kKept = 8;
+    // (never destroyed: a handle of a program's own static object may outlive them)
     static std::mutex& mutex() {
-        static std::mutex m;
-        return m;
+        static std::mutex* m = new std::mutex;
+        return *m;
     }
     static std::map<int, std::vector<HandleStreams>>& kept() {
-        static std::map<int, std::vector<HandleStreams>> k;
-        return k;
+        static auto* k = new std::map<int, std::vector<HandleStreams>>;
+        return *k;
     }
     // the device's streams for a new handle
     static HandleStreams take(int dev) {
