@@ -416,6 +416,7 @@ struct FusedArgs {
     uint32_t V;                               // entries of lam and G
     uint32_t N;                               // kept muons
     double E00, E01, E11;
+    float reach;                              // no path in a grid is longer (one-pass mixed form)
     int compute_cost;
     int prefetch;                             // stored lists: prefetch every CTA's next batch into L2
     Counters* ctr;
@@ -443,7 +444,7 @@ void launch_em_fused(const FusedArgs<Real>& a, int variant, int blocks, cudaStre
 // The mixed form's one-pass kernel without block barriers: `group` (16 or 32)
 // lanes per muon; sums (N, or null): also adds every muon's cost to the
 // counters, through a second small kernel over the sums.
-constexpr int kOnceHeld = 8;  // pairs held per lane
+constexpr int once_held(int group) { return group <= 16 ? 8 : 7; }  // pairs held per lane
 void launch_em_once(const FusedArgs<float>& a, int group, float4* sums, int num_sms, cudaStream_t s);
 template <typename Real>
 void launch_em_fused_walk(const FusedArgs<Real>& a, int num_sms, cudaStream_t s);

@@ -805,14 +805,15 @@ __global__ void __launch_bounds__(256) k_em_scatter(FusedArgs<Real> a, const typ
 // FP64 pipe, two lanes wide, for 960 cycles a muon).  The lists leave HBM once
 // for all but the pairs beyond the RC held per lane.
 //
-// Bound by the L1-to-L2 request path: 256x256x128 voxels, 2 M muons (212 M
-// pairs), 841 us: request path 69 % busy, L2 72 %, DRAM 55 %, issue 49 %; the
-// reductions' 0.50 sectors a pair are most of it.  With 20 M muons (2.1 G
-// pairs) a pass takes 8.6 ms, against 5.0 + 8.0 ms in the two-pass form (muon
-// pass and scatter).  Tried and slower: the next muon's pairs loaded ahead into
-// registers (16 instead of 24 warps on an SM), lists through shared memory by
-// cp.async or by bulk copies (their reads queue behind the reductions),
-// L2 prefetch of the next muon, muons in spatial order (reductions collide).
+// Bound by the L1-to-L2 request path and issue: 256x256x128 voxels, 2 M tracks
+// (0.96 M muons, 212 M pairs), 853 us; 805 us with the sums about the path's end
+// (request path 69 % busy, L2 72 %, DRAM 55 %, issue 49 %, the reductions' 0.50
+// sectors a pair most of it).  With 20 M tracks (2.1 G pairs) a pass takes 8.3 ms,
+// against 5.0 + 8.0 ms in the two-pass form (muon pass and scatter).  Tried and
+// slower: the next muon's pairs loaded ahead into registers (16 instead of 24 warps
+// on an SM), lists through shared memory by cp.async or by bulk copies (their reads
+// queue behind the reductions), L2 prefetch of the next muon, muons in spatial order
+// (reductions collide).
 constexpr int kOnceThreads = 128;
 
 // A double-float: the unevaluated sum of two floats, about 48 bits.
@@ -845,9 +846,94 @@ __device__ __forceinline__ float rcp_approx(float x) {  // to 1 ulp; refined whe
 struct DfE {  // the hit-error terms of Sigma
     Df e00, e01, e11;
 };
+// The same counted from the place `at` where their correlation is 0, and a length
+// that no path exceeds.
+struct OnceErrors {
+    Df e00, rest;
+    float at, reach;
+};
 
-// A muon's g_ij as a function of a pair's length L and tail midpoint U:
-//   g = 1/2 pr^2 L [ (u_x . (1, U))^2 + (u_y . (1, U))^2 - 2 f11 (U - S01/S00)^2 - 2/S00
+// ---- the moments of a path about its own centre ----
+// Sigma = pr^2 sum lambda_j W_ij + E with W00 = L, W01 = L U, W11 = L (U^2 + L^2/12),
+// U = T + L/2 the pair's place before the path's end.  Where one voxel holds most of
+// a muon's sum lambda L, the three sums about the path's end are nearly those of one
+// place U: the determinant is then L^2 / 12 U^2 of the product it is a difference of,
+// and an FP32 rounding of a sum comes out 1e4 times larger in Sigma^-1 (images of
+// sparse scans were up to 1e-4 off after 20 iterations).  Everything that a muon adds
+// is unchanged when its places are counted from any other point R, D taken as
+// D - R S.  So a muon's pairs are counted from their centre: every term of a sum is
+// then positive, no difference cancels, and the rounding of a sum stays a rounding of
+// Sigma (the same images 3e-6 off at most).  Two FP32 operations a pair more, one sum
+// over the lanes more.
+struct Moments {
+    float a, r, b1, b2;  // sum lambda L; the place counted from; sums of lambda L (U - r) and lambda W11 about r
+};
+// the moments counted from R (the two differences' rounding is one of the places')
+__device__ __forceinline__ void count_from(float R, const Moments& m, float& b1, float& b2) {
+    const float d = m.r - R;
+    b1 = fmaf(m.a, d, m.b1);
+    b2 = fmaf(d, fmaf(m.a, d, 2.f * m.b1), m.b2);
+}
+// sum / weight as a place between 0 and `reach`: any may be counted from, so a weight
+// of 0, negative lambdas, inf and NaN give one too
+__device__ __forceinline__ float centre(float sum, float weight, float reach) {
+    const float r = sum * rcp_approx(weight);
+    return r >= 0.f ? fminf(r, reach) : 0.f;
+}
+// of N pairs of a lane: sums of w = lambda L and of w times the place ...
+template <int N>
+__device__ __forceinline__ void first_sums(const float (&w)[N], const float (&U)[N], float& a, float& s) {
+    a = s = 0.f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        a += w[k];
+        s = fmaf(w[k], U[k], s);
+    }
+}
+// ... and those about R, from which the places are counted afterwards
+template <int N>
+__device__ __forceinline__ void sums_about(float R, const float (&w)[N], const float (&L)[N], float (&U)[N], float& b1,
+                                           float& b2) {
+    b1 = b2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        U[k] -= R;
+        b1 = fmaf(w[k], U[k], b1);
+        b2 = fmaf(w[k], fmaf(U[k], U[k], L[k] * (L[k] * (1.0f / 12.0f))), b2);
+    }
+}
+// two sets of moments counted from their common centre
+__device__ __forceinline__ Moments both(const Moments& m, const Moments& n) {
+    const float a = m.a + n.a, w = n.a * rcp_approx(a);
+    Moments t{a, w >= 0.f ? fmaf(fminf(w, 1.f), n.r - m.r, m.r) : m.r, 0.f, 0.f};
+    float b1, b2;
+    count_from(t.r, m, t.b1, t.b2);
+    count_from(t.r, n, b1, b2);
+    t.b1 += b1;
+    t.b2 += b2;
+    return t;
+}
+// E and (S, D) with the places counted from R.  E's own place is rounded to a float,
+// which moves it by 2^-24 of `at` or R against a spread sqrt(rest / e00) of at's order
+// (the planes' distances); the determinant is e00 * rest wherever it is counted from.
+__device__ __forceinline__ DfE errors_from(float R, const OnceErrors& e) {
+    const float t = e.at - R;  // e01 = e00 t, e11 = rest + e00 t^2
+    Df e01 = df_prod(e.e00.h, t);
+    e01.l = fmaf(e.e00.l, t, e01.l);
+    Df e11 = df_muladd(e01.h, t, e.rest);
+    e11.l = fmaf(e01.l, t, e11.l);
+    return DfE{e.e00, e01, e11};
+}
+__device__ __forceinline__ float4 deviations_from(float R, const float4& v) {
+    return make_float4(v.x, fmaf(-R, v.x, v.y), v.z, fmaf(-R, v.z, v.w));
+}
+__device__ __forceinline__ double e01_from(double R, double E00, double E01) { return E01 - R * E00; }
+__device__ __forceinline__ double e11_from(double R, double E00, double E01, double E11) {
+    return E11 - R * (E01 + (E01 - R * E00));
+}
+
+// A muon's g_ij as a function of a pair's length L and place d, counted from R:
+//   g = 1/2 pr^2 L [ (u_x . (1, d))^2 + (u_y . (1, d))^2 - 2 f11 (d - S01/S00)^2 - 2/S00
 //                    + (u_x1^2 + u_y1^2 - 2 f11) L^2 / 12 ],
 // u = Sigma^-1 (S, D) per plane, f11 = (Sigma^-1)_11: pr^2 (1/2 xyS - tr(Sigma^-1 W))
 // with both forms completed to squares, so that only their difference cancels
@@ -856,12 +942,12 @@ struct OnceCoef {
     float ax, bx, ay, by, f, u0, h, w, c;
 };
 
-// The coefficients of a muon from its sums: Sigma and its determinant in
-// double-floats, Sigma^-1 (S, D) by exact differences of products.  The sums
-// come in as floats, so this leaves the coefficients' own rounding as the
-// largest error.  False where it would not (a determinant that nearly cancels,
-// is near the singular threshold or out of range), and for a NaN: the caller
-// then takes the FP64 algebra.
+// The coefficients of a muon from its sums, E and (S, D), all counted from one
+// place: Sigma and its determinant in double-floats, Sigma^-1 (S, D) by exact
+// differences of products.  The sums come in as floats, so this leaves the
+// coefficients' own rounding as the largest error.  False where it would not (a
+// determinant that nearly cancels, is near the singular threshold or out of range),
+// and for a NaN: the caller then takes the FP64 algebra.
 __device__ __forceinline__ bool once_coefficients(float c0, float c1, float c2, float pr2, const float4& v,
                                                   const DfE& e, OnceCoef& o, unsigned& singular) {
     const Df s00 = df_muladd(pr2, c0, e.e00), s01 = df_muladd(pr2, c1, e.e01), s11 = df_muladd(pr2, c2, e.e11);
@@ -885,21 +971,13 @@ __device__ __forceinline__ bool once_coefficients(float c0, float c1, float c2, 
     if (d.h <= 0.f) ++singular;  // inverse used, cost 0 (:461-464)
     return true;
 }
-__device__ __forceinline__ float once_g(const OnceCoef& o, float L, float T) {
-    const float u = fmaf(0.5f, L, T);
+__device__ __forceinline__ float once_g(const OnceCoef& o, float L, float u) {
     const float x = fmaf(o.bx, u, o.ax), y = fmaf(o.by, u, o.ay), d = u - o.u0;
     return o.c * L * fmaf(x, x, fmaf(y, y, fmaf(-o.f * d, d, fmaf(o.w * L, L, -o.h))));
 }
 
-// the pair's two factors beside its length: U = T + L/2 and q = U^2 + L^2/12, with
-// W00 = L, W01 = L U, W11 = L q
-__device__ __forceinline__ void pair_factors(float L, float T, float& u, float& q) {
-    u = fmaf(0.5f, L, T);
-    q = fmaf(u, u, L * L * (1.0f / 12.0f));
-}
-
 template <int GROUP, int RC, int MB>
-__global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a, DfE e, float4* __restrict__ sums) {
+__global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a, OnceErrors e, float4* __restrict__ sums) {
     constexpr int kPer = 32 / GROUP;  // muons of a warp at once
     constexpr int U = 4;              // loads in flight per lane for the pairs beyond the held ones
     const int lane = threadIdx.x & 31, sub = lane / GROUP, glane = lane % GROUP;
@@ -916,7 +994,7 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
     }
     for (uint32_t mw = m - sub; mw < a.N; mw += step) {
         uint32_t cj[RC];
-        float cL[RC], cT[RC], cl[RC];
+        float cL[RC], cU[RC], cw[RC];  // length, place (loaded as the tail T), lambda L
         {
             const uint32_t* vp = a.vidx + pb + glane;
             const float* lp = a.L + pb + glane;
@@ -924,11 +1002,11 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
 #pragma unroll
             for (int r = 0; r < RC; ++r) {
                 cj[r] = 0xffffffffu;
-                cL[r] = cT[r] = 0.f;
+                cL[r] = cU[r] = 0.f;
                 if (glane + r * GROUP < n) {
                     cj[r] = __ldcs(vp + r * GROUP);
                     cL[r] = __ldcs(lp + r * GROUP);
-                    cT[r] = __ldcs(tp + r * GROUP);
+                    cU[r] = __ldcs(tp + r * GROUP);
                 }
             }
         }
@@ -946,21 +1024,19 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
         }
 #pragma unroll
         for (int r = 0; r < RC; ++r) {
-            cl[r] = 0.f;
-            if (cj[r] < V) cl[r] = ld_keep(a.lam + cj[r], keep);
+            cw[r] = 0.f;
+            if (cj[r] < V) cw[r] = ld_keep(a.lam + cj[r], keep);
         }
-        float c0 = 0.f, c1 = 0.f, c2 = 0.f;
-        auto add = [&](float l, float L, float T) {
-            float u, q;
-            pair_factors(L, T, u, q);
-            const float lL = l * L;
-            c0 += lL;
-            c1 = fmaf(lL, u, c1);
-            c2 = fmaf(lL, q, c2);
-        };
 #pragma unroll
-        for (int r = 0; r < RC; ++r) add(cl[r], cL[r], cT[r]);
-        // pairs beyond the held ones: read again below, from L1 or L2
+        for (int r = 0; r < RC; ++r) {
+            cU[r] = fmaf(0.5f, cL[r], cU[r]);
+            cw[r] *= cL[r];
+        }
+        float c0, c1, c2, at;
+        first_sums(cw, cU, c0, at);
+        // pairs beyond the held ones: read again below, from L1 or L2; their lambda is
+        // gathered once, so they are counted from centres of their own at first
+        Moments more{0.f, 0.f, 0.f, 0.f};
         for (uint32_t k0 = glane + GROUP * RC; k0 < n; k0 += GROUP * U) {
             uint32_t jj[U];
             float ll[U], tt[U], lv[U];
@@ -980,27 +1056,51 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
                 if (jj[u] < V) lv[u] = ld_keep(a.lam + jj[u], keep);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) add(lv[u], ll[u], tt[u]);
+            for (int u = 0; u < U; ++u) {
+                tt[u] = fmaf(0.5f, ll[u], tt[u]);
+                lv[u] *= ll[u];
+            }
+            Moments four;
+            first_sums(lv, tt, four.a, four.r);
+            c0 += four.a;
+            at += four.r;
+            four.r = centre(four.r, four.a, e.reach);
+            sums_about(four.r, lv, ll, tt, four.b1, four.b2);
+            more = both(more, four);
         }
         __syncwarp();
 #pragma unroll
         for (int o = GROUP / 2; o > 0; o >>= 1) {
             c0 += __shfl_xor_sync(kFull, c0, o);
+            at += __shfl_xor_sync(kFull, at, o);
+        }
+        const float R = centre(at, c0, e.reach);  // (the sums are the same on every lane of the group)
+        sums_about(R, cw, cL, cU, c1, c2);
+        if (n > GROUP * RC) {
+            float b1, b2;
+            count_from(R, more, b1, b2);
+            c1 += b1;
+            c2 += b2;
+        }
+#pragma unroll
+        for (int o = GROUP / 2; o > 0; o >>= 1) {
             c1 += __shfl_xor_sync(kFull, c1, o);
             c2 += __shfl_xor_sync(kFull, c2, o);
         }
         OnceCoef o{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         unsigned sing = 0;
-        if (m < a.N && !once_coefficients(c0, c1, c2, pr2, v, e, o, sing)) {
+        v = deviations_from(R, v);
+        if (m < a.N && !once_coefficients(c0, c1, c2, pr2, v, errors_from(R, e), o, sing)) {
             // rare: the terms added here from the lists, and nothing below
             float k0, k1, k2;
             unsigned long long s64 = 0;
             double cost = 0.0;
-            muon_coefficients<float>(c0, c1, c2, pr2, v, a.E00, a.E01, a.E11, false, k0, k1, k2, cost, s64);
+            muon_coefficients<float>(c0, c1, c2, pr2, v, a.E00, e01_from(R, a.E00, a.E01), e11_from(R, a.E00, a.E01, a.E11),
+                                     false, k0, k1, k2, cost, s64);
             sing = static_cast<unsigned>(s64);
             for (uint32_t k = glane; k < n; k += GROUP) {
                 const uint32_t j = a.vidx[pb + k];
-                if (j < V) red_add(a.G + j, g_term(k0, k1, k2, a.L[pb + k], a.T[pb + k]), keep);
+                if (j < V) red_add(a.G + j, g_term(k0, k1, k2, a.L[pb + k], a.T[pb + k] - R), keep);
             }
             n = 0;
 #pragma unroll
@@ -1008,10 +1108,10 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
         }
         if (glane == 0) {
             singular += sing;
-            if (sums && m < a.N) sums[m] = make_float4(c0, c1, c2, 0.f);
+            if (sums && m < a.N) sums[m] = make_float4(c0, c1, c2, R);
         }
-        auto put = [&](uint32_t j, float L, float T) {
-            if (j < V) red_add(a.G + j, once_g(o, L, T), keep);
+        auto put = [&](uint32_t j, float L, float u) {
+            if (j < V) red_add(a.G + j, once_g(o, L, u), keep);
         };
         for (uint32_t k0p = glane + GROUP * RC; k0p < n; k0p += GROUP * U) {
             uint32_t jj[U];
@@ -1027,10 +1127,10 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
                 }
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) put(jj[u], ll[u], tt[u]);
+            for (int u = 0; u < U; ++u) put(jj[u], ll[u], fmaf(0.5f, ll[u], tt[u]) - R);
         }
 #pragma unroll
-        for (int r = 0; r < RC; ++r) put(cj[r], cL[r], cT[r]);
+        for (int r = 0; r < RC; ++r) put(cj[r], cL[r], cU[r]);
         m = mn;
         pb = pbn;
         n = static_cast<uint32_t>(pen - pbn);
@@ -1064,11 +1164,12 @@ __global__ void __launch_bounds__(kCostThreads) k_once_cost(FusedArgs<float> a, 
     for (int u = 0; u < kCostMuons; ++u) {
         if (m0 + u * kCostThreads >= a.N) continue;
         const float4 c = cs[u], v = vs[u];
-        const double p2 = ps[u];
-        const double S00 = p2 * c.x + a.E00, S01 = p2 * c.y + a.E01, S11 = p2 * c.z + a.E11;
+        const double p2 = ps[u], R = c.w;  // the sums, and so all of this, counted from R
+        const double S00 = p2 * c.x + a.E00, S01 = p2 * c.y + e01_from(R, a.E00, a.E01),
+                     S11 = p2 * c.z + e11_from(R, a.E00, a.E01, a.E11);
         const double det = S00 * S11 - S01 * S01;
         if (!(det > 1e-12)) continue;  // cost 0; counted by k_em_once
-        const double sx = v.x, dx = v.y, sy = v.z, dy = v.w;
+        const double sx = v.x, dx = v.y - R * sx, sy = v.z, dy = v.w - R * sy;
         cost += ((sx * sx + sy * sy) * S11 + (dx * dx + dy * dy) * S00 - (sx * dx + sy * dy) * 2.0 * S01) / det;
         if (det > 1.0e300) {
             cost += 2.0 * log(det);
@@ -1092,7 +1193,8 @@ Df df_of(double x) {
 }
 template <int GROUP, int RC, int MB>
 void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t s) {
-    const DfE e{df_of(a.E00), df_of(a.E01), df_of(a.E11)};
+    const double at = a.E00 > 0.0 ? a.E01 / a.E00 : 0.0;
+    const OnceErrors e{df_of(a.E00), df_of(a.E11 - at * a.E01), static_cast<float>(at), a.reach};
     const uint64_t need = (static_cast<uint64_t>(a.N) * GROUP + kOnceThreads - 1) / kOnceThreads;
     const uint64_t most = static_cast<uint64_t>(MB) * num_sms;
     k_em_once<GROUP, RC, MB><<<static_cast<unsigned>(need < most ? need : most), kOnceThreads, 0, s>>>(a, e, sums);
@@ -1102,9 +1204,10 @@ void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t
 
 void launch_em_once(const FusedArgs<float>& a, int group, float4* sums, int num_sms, cudaStream_t s) {
     if (a.N == 0) return;
-    // blocks per SM: what the registers allow
-    if (group <= 16) run_once<16, kOnceHeld, 6>(a, sums, num_sms, s);
-    else run_once<32, kOnceHeld, 7>(a, sums, num_sms, s);
+    // blocks per SM: what the registers allow (32 lanes with 8 held pairs: six, or seven
+    // with spills; 1.71 and 1.79 ms where seven with 7 held pairs take 1.68)
+    if (group <= 16) run_once<16, once_held(16), 6>(a, sums, num_sms, s);
+    else run_once<32, once_held(32), 7>(a, sums, num_sms, s);
     if (sums) {
         constexpr uint64_t per = kCostMuons * kCostThreads;
         k_once_cost<<<static_cast<unsigned>((static_cast<uint64_t>(a.N) + per - 1) / per), kCostThreads, 0, s>>>(a, sums);

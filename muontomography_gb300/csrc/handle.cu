@@ -1583,6 +1583,10 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
     a.E00 = 4.0 * exy * exy / (ezo * ezo);
     a.E11 = 2.0 * exy * exy * (1.0 + (ezi / ezo + 1.0) * ezi / ezo);
     a.E01 = 2.0 * exy * exy * ezi / (ezo * ezo);
+    double reach = 0.0;  // two straight halves
+    for (const auto& sc : h->scans)
+        reach = std::max(reach, 2.0 * (sc.grid.nx * sc.grid.dx + sc.grid.ny * sc.grid.dy + sc.grid.nz * sc.grid.dz));
+    a.reach = static_cast<float>(reach);
     a.compute_cost = cost ? 1 : 0;
     a.prefetch = P.fused_prefetch ? 1 : 0;
     a.ctr = h->ctr();
@@ -2451,7 +2455,7 @@ int muto_get_status(const muto_handle* hc, muto_status* out) {
     } else if (h->method != kPoca && h->lists == kListsMuonMajor && h->fused_variant == kFusedOnce) {
         out->muon_pass = 3;
         out->muon_group = h->once_group;
-        out->tile_pairs = h->once_group * kOnceHeld;
+        out->tile_pairs = h->once_group * once_held(h->once_group);
         out->tile_muons = 32 / h->once_group;
     } else if (h->method != kPoca && h->lists == kListsMuonMajor) {
         const bool staged = h->fused_variant == kFusedStaged;
