@@ -173,7 +173,12 @@ int muto_set_initial_image(muto_handle* h, const double* img, const muto_grid* g
 int muto_reconstruct(muto_handle* h, const muto_ray* rays, uint64_t n, double* out_img, uint64_t out_len);
 
 /* Staged form of the same work.  on_device != 0: rays is a device pointer
- * (it is copied; the caller keeps ownership). */
+ * (it is copied; the caller keeps ownership).  The copy runs behind all work
+ * queued before the call on the legacy default stream, and on the streams
+ * that this one waits for (those not created non-blocking); what writes the
+ * tracks on a non-blocking stream, or on a per-thread default stream, must be
+ * complete, or the legacy stream made to wait for it, before the call.  The
+ * copy is complete when the call returns. */
 int muto_load_tracks(muto_handle* h, const muto_ray* rays, uint64_t n, int on_device);
 /* PoCA: runs the whole method.  MLSD/MAP: gatherInformation + paths + W
  * setup (src/MutoMLSD.cpp:99-152) and the initial image. */

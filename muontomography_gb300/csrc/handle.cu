@@ -2491,6 +2491,20 @@ int muto_set_initial_image(muto_handle* h, const double* img, const muto_grid* g
     });
 }
 
+// n tracks to dst, complete on return.  Device tracks are read behind what the caller
+// has queued on the legacy default stream, which the handle's own stream does not wait
+// for by itself.
+static void copy_tracks(muto_handle* h, void* dst, const muto_ray* rays, uint64_t n, int on_device) {
+    if (n > 0 && on_device) {
+        CK(cudaEventRecord(h->fan.fork, cudaStreamLegacy));
+        CK(cudaStreamWaitEvent(h->stream, h->fan.fork, 0));
+    }
+    if (n > 0)
+        CK(cudaMemcpyAsync(dst, rays, n * sizeof(muto_ray), on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                           h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+}
+
 int muto_load_tracks(muto_handle* h, const muto_ray* rays, uint64_t n, int on_device) {
     if (!h) return MUTO_ERR_ARG;
     return guarded(h, [&] {
@@ -2504,10 +2518,7 @@ int muto_load_tracks(muto_handle* h, const muto_ray* rays, uint64_t n, int on_de
             h->rays.alloc(std::max<uint64_t>(n, 1) * sizeof(muto_ray), &h->dev_bytes);
         }
         HostPhase ph(h, "load_copy");
-        if (n > 0)
-            CK(cudaMemcpyAsync(h->rays.as<void>(), rays, n * sizeof(muto_ray),
-                               on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        copy_tracks(h, h->rays.as<void>(), rays, n, on_device);
     });
 }
 
@@ -2896,10 +2907,7 @@ int muto_batch_load_tracks(muto_handle* h, uint32_t scan, const muto_ray* rays, 
         auto& slot = h->batch_rays[scan - 1];
         slot.reset(new DevMem());
         slot->alloc(std::max<uint64_t>(n, 1) * sizeof(muto_ray), &h->dev_bytes);
-        if (n > 0)
-            CK(cudaMemcpyAsync(slot->as<void>(), rays, n * sizeof(muto_ray),
-                               on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
+        copy_tracks(h, slot->as<void>(), rays, n, on_device);
         h->scans[scan].n_rays = n;
     });
 }
