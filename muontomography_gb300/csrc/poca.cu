@@ -25,7 +25,7 @@ struct WeightSink {
     int skip_scat;  // out-half, not length weighted: skip the scattering voxel (:166-168)
     uint32_t sx, sy, sz;
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
-        if (x >= nx || y >= ny || z >= nz) return;  // never for an in-grid walk
+        if (x >= nx || y >= ny || z >= nz) return;  // (nx or ny just below an upper face, see slr.cu)
         if (skip_scat && x == sx && y == sy && z == sz) return;
         const uint64_t j = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * (y + static_cast<uint64_t>(ny) * z);
         atomicAdd(weight + j, length_weighted ? l : dz);

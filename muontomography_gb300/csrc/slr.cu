@@ -40,6 +40,14 @@ __device__ __forceinline__ SlrRay slr_ray(const muto_ray& r, const DevGrid& g, d
     return o;
 }
 
+// A nearly upright line (at most 1e-6 mm to the side, growing) that starts within 1e-6
+// of a voxel below a grid's upper face is walked with index nx (or ny) there: the
+// start's voxel is rounded up by that much (src/MutoSiddon.cpp:62-81).  Such voxels
+// are outside the image: they count for the equal shares and for nothing else.
+__device__ __forceinline__ bool outside(uint32_t x, uint32_t y, uint32_t z, uint32_t nx, uint32_t ny, uint32_t nz) {
+    return x >= nx || y >= ny || z >= nz;
+}
+
 struct CountSink {
     uint32_t n = 0;
     __device__ void operator()(uint32_t, uint32_t, uint32_t, double) { ++n; }
@@ -52,7 +60,7 @@ struct SlrSink {
     double dz, a2, l_total, share, e2;  // share: a2 / 2 / n^2 (equal shares)
     int length_weighted, has_energy;
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
-        if (x >= nx || y >= ny || z >= nz) return;  // never for a walk inside the grid
+        if (outside(x, y, z, nx, ny, nz)) return;
         const uint64_t j = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * (y + static_cast<uint64_t>(ny) * z);
         double iv;
         if (length_weighted) {  // :80-83
@@ -87,14 +95,15 @@ __global__ void k_slr(SlrArgs a, DevGrid g) {
     siddon_walk(g, s.p_in, s.p_out, sink);
 }
 
-// The walked straight lines, for the in-place passes: per ray its voxel
-// count (first call) or its voxels and lengths at off[i] (second call).
+// The walked straight lines, for the in-place passes: per ray the count of its
+// voxels in the image (first call) or these voxels and lengths at off[i] (second call).
 struct PathSink {
     uint32_t* vox;
     double* len;
-    uint32_t nx, ny;
+    uint32_t nx, ny, nz;
     uint32_t k = 0;
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
+        if (outside(x, y, z, nx, ny, nz)) return;
         if (vox) {
             vox[k] = x + nx * (y + ny * z);
             len[k] = l;
@@ -110,7 +119,7 @@ __global__ void k_slr_paths(SlrArgs a, DevGrid g, const uint64_t* __restrict__ o
     const double z_lo = a.g.z_min;
     const double z_hi = dadd(a.g.z_min, dmul(a.g.dz, static_cast<double>(a.g.nz)));
     const SlrRay s = slr_ray(a.rays[i], g, z_lo, z_hi, a.mag);
-    PathSink p{off ? vox + off[i] : nullptr, off ? len + off[i] : nullptr, g.n[0], g.n[1]};
+    PathSink p{off ? vox + off[i] : nullptr, off ? len + off[i] : nullptr, g.n[0], g.n[1], g.n[2]};
     siddon_walk(g, s.p_in, s.p_out, p);
     if (!off) counts[i] = p.k;
 }
@@ -129,7 +138,12 @@ __global__ void k_slr_pair_terms(SlrArgs a, DevGrid g, SlrPass p) {
     const SlrRay s = slr_ray(r, g, z_lo, z_hi, a.mag);
     const uint64_t p0 = p.off[i];
     const uint32_t n = static_cast<uint32_t>(p.off[i + 1] - p0);
-    const double share = ddiv(dmul(s.a2, 0.5), static_cast<double>(static_cast<uint64_t>(n) * n));
+    double share = 0.0;
+    if (!a.length_weighted) {
+        CountSink c;
+        siddon_walk(g, s.p_in, s.p_out, c);
+        share = ddiv(dmul(s.a2, 0.5), static_cast<double>(static_cast<uint64_t>(c.n) * c.n));
+    }
     for (uint32_t k = 0; k < n; ++k) {
         const double l = p.len[p0 + k];
         if (a.length_weighted) {
