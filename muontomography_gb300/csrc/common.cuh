@@ -211,16 +211,17 @@ struct SlrPass {
 void launch_slr_pair_terms(const SlrArgs& a, const SlrPass& p, cudaStream_t s);
 // one later pass, muon after muon
 void launch_slr_iter_pass(const SlrArgs& a, const SlrPass& p, cudaStream_t s);
-// the same pairs (fewer than 2^32) in level order: muon q of the level order
-// (order[q]) has its pairs at fo[q] .. fo[q+1]
+// the same pairs in level order: muon q of the level order (order[q]) has its
+// pairs at fo[q] .. fo[q+1]
 struct SlrFlat {
-    const uint32_t* fo;
+    const uint64_t* fo;
     uint32_t* vox;
     double* iv0;      // times ein^2 with has_energy
     double* winc;
     uint8_t* place;   // the pair's muon in its step (0 .. kSlrStep-1)
 };
 constexpr int kSlrStep = 24;  // muons of a step at most (a group of 16 of a block's 384 threads each)
+constexpr uint64_t kSlrStepPairs = uint64_t(1) << 31;  // pairs of a step at most (a thread's numbers run past them)
 void launch_slr_flatten(const SlrArgs& a, const SlrPass& p, const uint32_t* order, const uint8_t* place, uint64_t nt,
                         const SlrFlat& f, cudaStream_t s);
 // the same pass level by level, in steps of one level or part of one: step s's

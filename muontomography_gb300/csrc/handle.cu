@@ -720,28 +720,21 @@ uint32_t slr_level_schedule(muto_handle* h, const DevMem& off, const DevMem& vox
     std::vector<uint32_t> cur(start.begin(), start.end());
     for (uint64_t i = 0; i < nt; ++i) order_h[cur[level[i]]++] = static_cast<uint32_t>(i);
     start.push_back(static_cast<uint32_t>(nt));
-    std::vector<uint32_t> steps_h;
-    std::vector<uint8_t> place_h(nt);
-    for (uint32_t l = 1; l <= levels; ++l)
-        for (uint32_t q = start[l]; q < start[l + 1]; ++q) {
-            const uint32_t in = (q - start[l]) % kSlrStep;
-            if (in == 0) steps_h.push_back(q);
-            place_h[q] = static_cast<uint8_t>(in);
-        }
-    const uint32_t steps = static_cast<uint32_t>(steps_h.size());
-    steps_h.push_back(static_cast<uint32_t>(nt));
     // where each muon's pairs go in level order
-    std::vector<uint32_t> fo_h(nt + 1, 0);
-    for (uint64_t q = 0; q < nt; ++q) fo_h[q + 1] = fo_h[q] + static_cast<uint32_t>(off_h[order_h[q] + 1] - off_h[order_h[q]]);
+    std::vector<uint64_t> fo_h(nt + 1, 0);
+    for (uint64_t q = 0; q < nt; ++q) fo_h[q + 1] = fo_h[q] + (off_h[order_h[q] + 1] - off_h[order_h[q]]);
+    std::vector<uint32_t> steps_h;
+    std::vector<uint8_t> place_h;
+    const uint32_t steps = slr_steps(start, levels, fo_h.data(), kSlrStep, kSlrStepPairs, steps_h, place_h);
     order.alloc(std::max<uint64_t>(nt, 1) * sizeof(uint32_t), &h->dev_bytes);
     place.alloc(std::max<uint64_t>(nt, 1), &h->dev_bytes);
     sstart.alloc(steps_h.size() * sizeof(uint32_t), &h->dev_bytes);
-    fo.alloc((nt + 1) * sizeof(uint32_t), &h->dev_bytes);
+    fo.alloc((nt + 1) * sizeof(uint64_t), &h->dev_bytes);
     CK(cudaMemcpyAsync(order.as<uint32_t>(), order_h.data(), nt * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(place.as<uint8_t>(), place_h.data(), nt, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(sstart.as<uint32_t>(), steps_h.data(), steps_h.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
                        s));
-    CK(cudaMemcpyAsync(fo.as<uint32_t>(), fo_h.data(), (nt + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(fo.as<uint64_t>(), fo_h.data(), (nt + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));  // the host vectors go out of scope
     h->slr_levels = levels;
     return steps;
@@ -789,8 +782,9 @@ void prepare_slr(muto_handle* h, uint64_t nt) {
         DevMem order, place, sstart, fo, fvox, fiv0, fwinc, fplace;
         SlrFlat fl{};
         uint32_t steps = 0;
-        // (2^32 pairs and more: muon after muon, the level order's offsets have 32 bits)
-        const bool by_level = !h->P.slr_sequential && np < 0xffffffffull;
+        // (a step counts its pairs in 32 bits, and a path has at most nx + ny + nz)
+        const bool by_level = !h->P.slr_sequential &&
+                              static_cast<uint64_t>(h->grid.nx) + h->grid.ny + h->grid.nz < kSlrStepPairs;
         if (by_level) {
             {
                 HostPhase ph(h, "slr_levels");
@@ -801,7 +795,7 @@ void prepare_slr(muto_handle* h, uint64_t nt) {
             fiv0.alloc(std::max<uint64_t>(np, 1) * sizeof(double), &h->dev_bytes);
             fwinc.alloc(std::max<uint64_t>(np, 1) * sizeof(double), &h->dev_bytes);
             fplace.alloc(std::max<uint64_t>(np, 1), &h->dev_bytes);
-            fl = SlrFlat{fo.as<uint32_t>(), fvox.as<uint32_t>(), fiv0.as<double>(), fwinc.as<double>(), fplace.as<uint8_t>()};
+            fl = SlrFlat{fo.as<uint64_t>(), fvox.as<uint32_t>(), fiv0.as<double>(), fwinc.as<double>(), fplace.as<uint8_t>()};
             run(h, "slr_paths", [&] { launch_slr_flatten(a, sp, order.as<uint32_t>(), place.as<uint8_t>(), nt, fl, s); });
         }
         for (int p = 1; p < passes; ++p)

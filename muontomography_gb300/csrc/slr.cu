@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
     extern __shared__ double slr_smem[];
     __shared__ double s_rec[kSlrStep];
     constexpr int H = 32 / kSlrLanes;  // pairs of a muon's sum held per lane
-    const int tid = threadIdx.x, l8 = tid % kSlrLanes, slot = tid / kSlrLanes;
+    const uint32_t tid = threadIdx.x, l8 = tid % kSlrLanes, slot = tid / kSlrLanes;
     const uint32_t V = a.g.nx * a.g.ny * a.g.nz;
     double* img = a.img;
     double* weight = a.weight;
@@ -269,20 +269,22 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
         }
         __syncthreads();
     }
-    // a step's offsets: this lane group's muon [b, e), the step's pairs [p, q)
+    // a step's offsets: its first pair, and counted from there this lane group's muon
+    // [b, e) and the step's end q
     struct Offsets {
-        uint32_t b, e, p, q;
+        uint64_t p;
+        uint32_t b, e, q;
     };
     auto offsets = [&](uint32_t q0, uint32_t q1) -> Offsets {  // of the step with muons [q0, q1)
         Offsets o{0, 0, 0, 0};
         const uint32_t m = q0 + slot;
         if (q0 < q1) {
             o.p = f.fo[q0];
-            o.q = f.fo[q1];
+            o.q = static_cast<uint32_t>(f.fo[q1] - o.p);
         }
         if (m < q1) {
-            o.b = f.fo[m];
-            o.e = f.fo[m + 1];
+            o.b = static_cast<uint32_t>(f.fo[m] - o.p);
+            o.e = static_cast<uint32_t>(f.fo[m + 1] - o.p);
         }
         return o;
     };
@@ -294,11 +296,12 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
     };
     auto pairs = [&](const Offsets& o) -> Pairs {
         Pairs r{};
+        const uint32_t* vox = f.vox + o.p;
 #pragma unroll
         for (int h = 0; h < H; ++h)
-            if (o.b + l8 + h * kSlrLanes < o.e) r.v[h] = f.vox[o.b + l8 + h * kSlrLanes];
-        if (o.p + tid < o.q) {
-            r.j = f.vox[o.p + tid];
+            if (o.b + l8 + h * kSlrLanes < o.e) r.v[h] = vox[o.b + l8 + h * kSlrLanes];
+        if (tid < o.q) {
+            r.j = vox[tid];
             r.place = f.place[o.p + tid];
             r.iv0 = f.iv0[o.p + tid];
             r.winc = f.winc[o.p + tid];
@@ -319,13 +322,13 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
 #pragma unroll
                 for (int h = 0; h < d; ++h) w[h] = dadd(w[h], w[h + d]);
             double part = w[0];
-            for (uint32_t k = o.b + l8 + H * kSlrLanes; k < o.e; k += kSlrLanes) part = dadd(part, img[f.vox[k]]);
+            for (uint32_t k = o.b + l8 + H * kSlrLanes; k < o.e; k += kSlrLanes) part = dadd(part, img[f.vox[o.p + k]]);
             __syncwarp();
 #pragma unroll
             for (int d = kSlrLanes / 2; d > 0; d >>= 1) part = dadd(part, __shfl_xor_sync(kFull, part, d));
             if (l8 == 0 && o.b < o.e) s_rec[slot] = slr_reciprocal(part);
         }
-        const bool mine = o.p + tid < o.q;
+        const bool mine = tid < o.q;
         double x = 0.0, inc = 0.0;
         if (mine) {
             x = img[c.j];
@@ -339,11 +342,11 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
         q4 = first(s + 5);
         __syncthreads();
         if (mine) img[c.j] = fma(inc, s_rec[c.place], x);
-        for (uint32_t k = o.p + tid + kSlrThreads; k < o.q; k += kSlrThreads) {  // more pairs than threads
-            const uint32_t j = f.vox[k];
+        for (uint32_t k = tid + kSlrThreads; k < o.q; k += kSlrThreads) {  // more pairs than threads
+            const uint32_t j = f.vox[o.p + k];
             const double xk = img[j];
-            weight[j] = dadd(weight[j], f.winc[k]);
-            img[j] = fma(dmul(f.iv0[k], xk), s_rec[f.place[k]], xk);
+            weight[j] = dadd(weight[j], f.winc[o.p + k]);
+            img[j] = fma(dmul(f.iv0[o.p + k], xk), s_rec[f.place[o.p + k]], xk);
         }
         __syncthreads();
         o = o1;
