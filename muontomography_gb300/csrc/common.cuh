@@ -218,17 +218,20 @@ struct SlrFlat {
     uint32_t* vox;
     double* iv0;      // times ein^2 with has_energy
     double* winc;
-    uint8_t* place;   // the pair's muon in its step (0 .. kSlrStep-1)
+    uint8_t* place;   // the pair's muon in its step
 };
-constexpr int kSlrStep = 24;  // muons of a step at most (a group of 16 of a block's 384 threads each)
+constexpr int kSlrLanes = 16;     // of the one block's threads a muon of a step has
+constexpr int kSlrStep = 24;      // muons of a step at most, the image in shared memory ...
+constexpr int kSlrWideStep = 64;  // ... and in global memory
 constexpr uint64_t kSlrStepPairs = uint64_t(1) << 31;  // pairs of a step at most (a thread's numbers run past them)
 void launch_slr_flatten(const SlrArgs& a, const SlrPass& p, const uint32_t* order, const uint8_t* place, uint64_t nt,
                         const SlrFlat& f, cudaStream_t s);
 // the same pass level by level, in steps of one level or part of one: step s's
-// muons are q = sstart[s] .. sstart[s+1] of the level order; the image and
-// weight sums are kept in shared memory when 2 V doubles fit in smem_optin bytes
-void launch_slr_iter_steps(const SlrArgs& a, const SlrFlat& f, const uint32_t* sstart, uint32_t steps,
-                           size_t smem_optin, cudaStream_t s);
+// muons are q = sstart[s] .. sstart[s+1] of the level order; the image and weight
+// sums are kept in shared memory unless wide (2 V doubles do not fit)
+bool slr_wide(const muto_grid& g, size_t smem_optin);
+void launch_slr_iter_steps(const SlrArgs& a, const SlrFlat& f, const uint32_t* sstart, uint32_t steps, bool wide,
+                           cudaStream_t s);
 
 // PoCut's per-voxel step (src/MutoPoCut.cpp:113-118), after launch_poca:
 // the kept values grouped by voxel (counts, then offsets, then a scatter of

@@ -694,8 +694,8 @@ void alloc_counters(muto_handle* h) {
 // The level schedule of SLRIter's later passes (slr_levels.h), made once
 // from the walked paths, which do not change between passes; the muons are
 // then grouped by level (index order inside a level) for the device.
-// sstart: the steps' first muons in level order (a level, or kSlrStep muons of a
-// longer one, a step); returns the number of steps.
+// sstart: the steps' first muons in level order (a step: a level, or kSlrStep or
+// kSlrWideStep muons of a longer one); returns the number of steps.
 uint32_t slr_level_schedule(muto_handle* h, const DevMem& off, const DevMem& vox, uint64_t nt, uint64_t np,
                             DevMem& order, DevMem& place, DevMem& sstart, DevMem& fo) {
     const uint64_t V = h->V();
@@ -725,7 +725,8 @@ uint32_t slr_level_schedule(muto_handle* h, const DevMem& off, const DevMem& vox
     for (uint64_t q = 0; q < nt; ++q) fo_h[q + 1] = fo_h[q] + (off_h[order_h[q] + 1] - off_h[order_h[q]]);
     std::vector<uint32_t> steps_h;
     std::vector<uint8_t> place_h;
-    const uint32_t steps = slr_steps(start, levels, fo_h.data(), kSlrStep, kSlrStepPairs, steps_h, place_h);
+    const uint32_t steps = slr_steps(start, levels, fo_h.data(), slr_wide(h->grid, h->smem_optin) ? kSlrWideStep : kSlrStep,
+                                     kSlrStepPairs, steps_h, place_h);
     order.alloc(std::max<uint64_t>(nt, 1) * sizeof(uint32_t), &h->dev_bytes);
     place.alloc(std::max<uint64_t>(nt, 1), &h->dev_bytes);
     sstart.alloc(steps_h.size() * sizeof(uint32_t), &h->dev_bytes);
@@ -803,7 +804,7 @@ void prepare_slr(muto_handle* h, uint64_t nt) {
                 if (!by_level)
                     launch_slr_iter_pass(a, sp, s);
                 else
-                    launch_slr_iter_steps(a, fl, sstart.as<uint32_t>(), steps, h->smem_optin, s);
+                    launch_slr_iter_steps(a, fl, sstart.as<uint32_t>(), steps, slr_wide(h->grid, h->smem_optin), s);
             });
         CK(cudaStreamSynchronize(s));  // the path arrays go out of scope
     }

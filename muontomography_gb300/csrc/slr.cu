@@ -229,7 +229,7 @@ __device__ __forceinline__ double slr_reciprocal(double x) {
 // one level share no voxel, and every voxel meets its muons in index order:
 // each muon reads and writes the image state it would see in the sequential
 // loop, whatever the order inside a level.  One block; a step is a level, or at
-// most kSlrStep muons of a longer one.  In a step
+// most THREADS / 16 muons of a longer one.  In a step
 //   sum     sixteen lanes a muon add up the image on its path (:49-52) and take
 //           the sum's reciprocal;
 //   pairs   a thread per pair adds its weight increment and multiplies its
@@ -241,20 +241,21 @@ __device__ __forceinline__ double slr_reciprocal(double x) {
 // part's two FP64 lanes a clock per SM, two barriers) and by that pipe.  20^3
 // voxels, 30 k muons, 2 449 levels: 1.29 us a step; 2.82 us with a warp a muon
 // (a division a pair, a 32-lane sum a muon).  8 and 4 lanes a muon, 512 and 640
-// threads took 1.29 to 1.51 us, 32 lanes 1.95.
+// threads took 1.29 to 1.51 us, 32 lanes 1.95.  Where the image is in global memory
+// its latency bounds a step, and grids are larger and paths longer: 1 024 threads, 64
+// muons a step (slr_wide).  A pass, in ms, with 384 / 768 / 1 024 threads: 32^3 with
+// 50 k muons 11.7 / 9.7 / 8.9, 48^3 with 100 k 34.1 / 24.5 / 22.4, 100^3 with 100 k
+// 59.6 / 38.4 / 35.0, 200^3 with 50 k 57.4 / 35.3 / 32.7 (1 024 threads with 32 lanes
+// a muon: 9.2, 24.7, 41.7, 35.0); in shared memory, 20^3 with 30 k: 3.1 / 4.2 / 4.9.
 // With SMEM the image and weight sums (2 V doubles) are copied into shared
 // memory for the pass and back after it.  Nothing that a step loads from the
 // lists depends on the image: a step's bounds are loaded five steps ahead,
 // its offsets three, its pairs two.
-constexpr int kSlrThreads = 384;  // a step of the 20^3 grid has about 12 muons and 300 pairs
-constexpr int kSlrLanes = 16;     // of a muon's sum
-static_assert(kSlrThreads / kSlrLanes >= kSlrStep, "a lane group for every muon of a step");
-
-template <bool SMEM>
-__global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFlat f,
-                                                                const uint32_t* __restrict__ sstart, uint32_t steps) {
+template <bool SMEM, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_slr_iter_steps(SlrArgs a, SlrFlat f,
+                                                            const uint32_t* __restrict__ sstart, uint32_t steps) {
     extern __shared__ double slr_smem[];
-    __shared__ double s_rec[kSlrStep];
+    __shared__ double s_rec[THREADS / kSlrLanes];
     constexpr int H = 32 / kSlrLanes;  // pairs of a muon's sum held per lane
     const uint32_t tid = threadIdx.x, l8 = tid % kSlrLanes, slot = tid / kSlrLanes;
     const uint32_t V = a.g.nx * a.g.ny * a.g.nz;
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kSlrThreads) k_slr_iter_steps(SlrArgs a, SlrFl
         q4 = first(s + 5);
         __syncthreads();
         if (mine) img[c.j] = fma(inc, s_rec[c.place], x);
-        for (uint32_t k = tid + kSlrThreads; k < o.q; k += kSlrThreads) {  // more pairs than threads
+        for (uint32_t k = tid + THREADS; k < o.q; k += THREADS) {  // more pairs than threads
             const uint32_t j = f.vox[o.p + k];
             const double xk = img[j];
             weight[j] = dadd(weight[j], f.winc[o.p + k]);
@@ -397,17 +398,26 @@ void launch_slr_flatten(const SlrArgs& a, const SlrPass& p, const uint32_t* orde
     count_launches(1);
 }
 
-void launch_slr_iter_steps(const SlrArgs& a, const SlrFlat& f, const uint32_t* sstart, uint32_t steps,
-                           size_t smem_optin, cudaStream_t s) {
+static size_t slr_shared_bytes(const muto_grid& g) {
+    return 2 * sizeof(double) * static_cast<size_t>(g.nx) * g.ny * g.nz;
+}
+
+bool slr_wide(const muto_grid& g, size_t smem_optin) {
+    return slr_shared_bytes(g) + kSlrStep * sizeof(double) + 1024 > smem_optin;
+}
+
+void launch_slr_iter_steps(const SlrArgs& a, const SlrFlat& f, const uint32_t* sstart, uint32_t steps, bool wide,
+                           cudaStream_t s) {
     if (a.n == 0 || steps == 0) return;
-    const size_t bytes = 2 * sizeof(double) * static_cast<size_t>(a.g.nx) * a.g.ny * a.g.nz;
-    if (bytes + kSlrStep * sizeof(double) + 1024 <= smem_optin &&
-        cudaFuncSetAttribute(k_slr_iter_steps<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(bytes)) == cudaSuccess) {
-        k_slr_iter_steps<true><<<1, kSlrThreads, bytes, s>>>(a, f, sstart, steps);
+    const size_t bytes = slr_shared_bytes(a.g);
+    if (wide) {
+        k_slr_iter_steps<false, kSlrWideStep * kSlrLanes><<<1, kSlrWideStep * kSlrLanes, 0, s>>>(a, f, sstart, steps);
+    } else if (cudaFuncSetAttribute(k_slr_iter_steps<true, kSlrStep * kSlrLanes>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)) == cudaSuccess) {
+        k_slr_iter_steps<true, kSlrStep * kSlrLanes><<<1, kSlrStep * kSlrLanes, bytes, s>>>(a, f, sstart, steps);
     } else {
         (void)cudaGetLastError();  // a refused attribute: the pass stays in global memory
-        k_slr_iter_steps<false><<<1, kSlrThreads, 0, s>>>(a, f, sstart, steps);
+        k_slr_iter_steps<false, kSlrStep * kSlrLanes><<<1, kSlrStep * kSlrLanes, 0, s>>>(a, f, sstart, steps);
     }
     count_launches(1);
 }
