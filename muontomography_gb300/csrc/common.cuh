@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstddef>
 #include "geometry.cuh"
+#include "streams.h"
 
 namespace muto {
 
@@ -342,15 +343,6 @@ __host__ __device__ constexpr int vox_class_of(uint32_t M) {
 struct alignas(16) VoxDesc {
     uint32_t j, M;
     unsigned long long start;
-};
-// Side streams the class kernels of a voxel pass are spread over (they touch
-// disjoint voxels), with the events that fork them from the launching stream
-// and join them back; inside stream capture they become parallel branches.
-struct ClassFan {
-    static constexpr int kSide = 3;
-    cudaStream_t side[kSide];
-    cudaEvent_t fork, join[kSide];
-    int n = 0;  // side streams in use (0: every class on the launching stream)
 };
 // The key pass over a.P pairs, then the class kernels.  lists[c], counts[c]:
 // the descriptors of class c; resident_blocks[c] and [kVoxClasses + c]:

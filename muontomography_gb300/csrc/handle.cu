@@ -128,85 +128,6 @@ private:
     std::atomic<uint64_t>* tally_ = nullptr;
 };
 
-// The streams and events of one handle (or call), from a small pool per device: creating
-// and destroying them takes longer than a small scan's iterations.  A set goes
-// back to the pool idle (the handle's destructor waits for its stream); the pool
-// keeps at most kKept sets a device and destroys the rest.
-struct HandleStreams {
-    static constexpr int kOverlap = 5;
-    int device = 0;
-    cudaStream_t stream = nullptr;
-    ClassFan fan{};
-    cudaEvent_t ov_ev[kOverlap] = {};
-
-    void create(int dev) {
-        device = dev;
-        CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&fan.fork, cudaEventDisableTiming));
-        for (int k = 0; k < ClassFan::kSide; ++k) {
-            CK(cudaStreamCreateWithFlags(&fan.side[k], cudaStreamNonBlocking));
-            CK(cudaEventCreateWithFlags(&fan.join[k], cudaEventDisableTiming));
-            fan.n = k + 1;
-        }
-        for (cudaEvent_t& e : ov_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    void destroy() {
-        for (int k = 0; k < ClassFan::kSide; ++k) {
-            if (fan.side[k]) cudaStreamDestroy(fan.side[k]);
-            if (fan.join[k]) cudaEventDestroy(fan.join[k]);
-        }
-        if (fan.fork) cudaEventDestroy(fan.fork);
-        for (cudaEvent_t e : ov_ev)
-            if (e) cudaEventDestroy(e);
-        if (stream) cudaStreamDestroy(stream);
-        *this = HandleStreams{};
-    }
-    static constexpr size_t kKept = 8;
-    // (never destroyed: a handle of a program's own static object may outlive them)
-    static std::mutex& mutex() {
-        static std::mutex* m = new std::mutex;
-        return *m;
-    }
-    static std::map<int, std::vector<HandleStreams>>& kept() {
-        static auto* k = new std::map<int, std::vector<HandleStreams>>;
-        return *k;
-    }
-    // the device's streams for a new handle
-    static HandleStreams take(int dev) {
-        {
-            std::lock_guard<std::mutex> lock(mutex());
-            auto& k = kept()[dev];
-            if (!k.empty()) {
-                HandleStreams h = k.back();
-                k.pop_back();
-                return h;
-            }
-        }
-        HandleStreams h;
-        try {
-            h.create(dev);
-        } catch (...) {
-            h.destroy();
-            throw;
-        }
-        return h;
-    }
-    // back to the pool, its work done
-    void give() {
-        if (!stream) return;
-        if (cudaStreamSynchronize(stream) == cudaSuccess) {
-            std::lock_guard<std::mutex> lock(mutex());
-            auto& k = kept()[device];
-            if (k.size() < kKept) {
-                k.push_back(*this);
-                *this = HandleStreams{};
-                return;
-            }
-        }
-        destroy();
-    }
-};
-
 // A stream owned by one call, from the same pool and back to it, idle, on every way
 // out; the call's allocations are ordered on it.
 struct OwnedStream {
@@ -216,11 +137,11 @@ struct OwnedStream {
     OwnedStream() {
         int dev = 0;
         CK(cudaGetDevice(&dev));
-        set = HandleStreams::take(dev);
+        CK(HandleStreams::take(dev, &set));
         s = set.stream;
         scope.reset(new AllocScope(s));
     }
-    ~OwnedStream() { set.give(); }
+    ~OwnedStream() { set.give(false); }
     OwnedStream(const OwnedStream&) = delete;
     OwnedStream& operator=(const OwnedStream&) = delete;
 };
@@ -936,23 +857,20 @@ template <class F>
 void fan_scans(muto_handle* h, F&& f) {
     const size_t S = h->scans.size();
     const int side = S > 1 && !h->prof.on ? h->fan.n : 0;
+    Forked forked(h->fan, side);
     if (side) {
         CK(cudaEventRecord(h->fan.fork, h->stream));
         for (int q = 0; q < side; ++q) CK(cudaStreamWaitEvent(h->fan.side[q], h->fan.fork, 0));
     }
-    try {
-        for (size_t k = 0; k < S; ++k) {
-            const size_t q = k % static_cast<size_t>(side + 1);
-            f(k, q == 0 ? h->stream : h->fan.side[q - 1]);
-        }
-    } catch (...) {  // nothing is freed under the launches that were made
-        for (int q = 0; q < side; ++q) cudaStreamSynchronize(h->fan.side[q]);
-        throw;
+    for (size_t k = 0; k < S; ++k) {
+        const size_t q = k % static_cast<size_t>(side + 1);
+        f(k, q == 0 ? h->stream : h->fan.side[q - 1]);
     }
     for (int q = 0; q < side; ++q) {
         CK(cudaEventRecord(h->fan.join[q], h->fan.side[q]));
         CK(cudaStreamWaitEvent(h->stream, h->fan.join[q], 0));
     }
+    forked.joined = true;
 }
 
 // src[at[k]] of every k on the host, in one copy; waits for the handle's stream
@@ -1614,6 +1532,7 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
             mb.V = static_cast<uint32_t>(h->vb);
         }
         cudaStream_t side = h->fan.side[0];
+        Forked forked(h->fan, 1);
         constexpr int C = muto_handle::kOverlapChunks;
         for (int c = 0; c < C; ++c) {
             const uint64_t m0 = h->N * c / C, m1 = h->N * (c + 1) / C;
@@ -1633,6 +1552,7 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
         }
         CK(cudaEventRecord(h->ov_ev[C], side));
         CK(cudaStreamWaitEvent(s, h->ov_ev[C], 0));
+        forked.joined = true;
         return;
     }
     if (h->lists == kListsRecompute) {
@@ -2382,7 +2302,7 @@ int muto_create(const char* method, const char* config_json, muto_handle** out) 
         int optin = 0;
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
         h->smem_optin = static_cast<size_t>(optin);
-        static_cast<HandleStreams&>(h->streams) = HandleStreams::take(h->device);
+        CK(HandleStreams::take(h->device, &h->streams));
         h->stream = h->streams.stream;
         h->fan = h->streams.fan;
         static_assert(HandleStreams::kOverlap == muto_handle::kOverlapChunks + 1, "one event a chunk and one more");
