@@ -12,7 +12,8 @@
 // (G is L2-resident), and a small voxel kernel finishes the update.
 //
 // One-pass form of the mixed precision (k_em_once, below): what "auto" runs
-// there.  The forms that follow serve FP64 and the forced variants.
+// there.  FP64 takes the split form.  Neither is timed against the others, which run
+// when a config asks for them (fused_variant, fused_prefetch).
 //
 // Stored-list pass (k_em_fused_lists).  A CTA takes 32 consecutive muons at a
 // time, GROUP lanes per muon.  Each lane loads its share of the muon's pairs
@@ -31,8 +32,8 @@
 // (em_muon.cu: warp-batched, no block barriers, its FP64 2x2 algebra a muon
 // per lane) writes every muon's coefficients; a second pass streams the lists
 // again and only adds g_ij to G_j, 4 or 8 pairs in flight per lane.  Twice
-// the list traffic from HBM, but neither pass waits at a block barrier; the
-// autotuner times it beside the one-pass variants (FP64).
+// the list traffic from HBM, but neither pass waits at a block barrier.  In FP64 its
+// two passes spend the fewest FP64 operations on a pair.
 //
 // Recompute pass (k_em_fused_walk).  The same sums without stored lists: a
 // thread per muon (one muon each, so that a warp's lanes walk in step; the
@@ -1282,7 +1283,6 @@ int scatter_blocks_per_sm() {
 
 template <typename Real>
 int em_scatter_blocks(int group, int depth) {
-    if (group <= 4) return scatter_blocks_per_sm<Real, 4, 4, true>();
     if (depth > 4) {
         if (group <= 8) return scatter_blocks_per_sm<Real, 8, 8, true>();
         if (group <= 16) return scatter_blocks_per_sm<Real, 16, 8, true>();
@@ -1303,15 +1303,12 @@ void launch_em_scatter(const FusedArgs<Real>& a, const typename Vec4<Real>::type
     const unsigned nb = static_cast<unsigned>(need < static_cast<uint64_t>(blocks) ? need : blocks);
     if constexpr (sizeof(Real) == 8) {
         if (a.W11) {  // (the grid was sized for the plain form, which keeps fewer values per pair)
-            if (group <= 4) k_em_scatter<Real, 4, 4, true, true><<<nb, 256, 0, s>>>(a, kvec);
-            else k_em_scatter<Real, 8, 8, true, true><<<nb, 256, 0, s>>>(a, kvec);
+            k_em_scatter<Real, 8, 8, true, true><<<nb, 256, 0, s>>>(a, kvec);
             count_launches(1);
             return;
         }
     }
-    if (group <= 4) {
-        k_em_scatter<Real, 4, 4, true><<<nb, 256, 0, s>>>(a, kvec);
-    } else if (depth > 4) {
+    if (depth > 4) {
         if (group <= 8) k_em_scatter<Real, 8, 8, true><<<nb, 256, 0, s>>>(a, kvec);
         else if (group <= 16) k_em_scatter<Real, 16, 8, true><<<nb, 256, 0, s>>>(a, kvec);
         else k_em_scatter<Real, 32, 8, true><<<nb, 256, 0, s>>>(a, kvec);

@@ -476,7 +476,8 @@ template <typename Real, bool WEIGHTS>
 static int warp_blocks(int group) {
     int n = 0;
     cudaError_t e;
-    if (group <= 4) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 4, WEIGHTS>, kThreads, 0);
+    if (sizeof(Real) == 8 && group <= 4)  // (4 lanes a muon: FP64 alone)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<double, 4, WEIGHTS>, kThreads, 0);
     else if (group <= 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 8, WEIGHTS>, kThreads, 0);
     else if (group <= 16) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 16, WEIGHTS>, kThreads, 0);
     else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 32, WEIGHTS>, kThreads, 0);
@@ -497,8 +498,13 @@ void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int bloc
     const unsigned nb = static_cast<unsigned>(need < static_cast<uint64_t>(blocks) ? need : blocks);
     auto go = [&](auto w) {
         constexpr bool W = decltype(w)::value;
-        if (group <= 4) k_em_muon_warp<Real, 4, W><<<nb, kThreads, 0, s>>>(a, n_muons);
-        else if (group <= 8) k_em_muon_warp<Real, 8, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+        if constexpr (sizeof(Real) == 8) {
+            if (group <= 4) {
+                k_em_muon_warp<Real, 4, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+                return;
+            }
+        }
+        if (group <= 8) k_em_muon_warp<Real, 8, W><<<nb, kThreads, 0, s>>>(a, n_muons);
         else if (group <= 16) k_em_muon_warp<Real, 16, W><<<nb, kThreads, 0, s>>>(a, n_muons);
         else k_em_muon_warp<Real, 32, W><<<nb, kThreads, 0, s>>>(a, n_muons);
     };
