@@ -387,7 +387,7 @@ __host__ __device__ inline uint32_t unbrick(uint32_t jb, const BrickDims& b) {
     const uint32_t z = bz * 8 + (((in >> 1) & 3u) | ((in >> 2) & 4u));
     return x + b.nx * (y + b.ny * z);
 }
-// voxel indices to bricked ones in place (indices >= V are left alone)
+// voxel indices to bricked ones in place (indices >= V to ones >= brick_volume)
 void launch_brick_indices(uint32_t* vidx, uint64_t n, BrickDims b, uint32_t V, cudaStream_t s);
 // bricked indices back to voxel indices
 void launch_unbrick_indices(const uint32_t* in, uint32_t* out, uint64_t n, BrickDims b, cudaStream_t s);

@@ -563,11 +563,14 @@ __global__ void k_class_scatter(const uint32_t* __restrict__ mult, const uint64_
     }
 }
 
+// (An index past the grid, as a path just below the upper x face has in the last row
+// and plane, goes past the bricks, whose padding it would fall into otherwise.)
 __global__ void k_brick_indices(uint32_t* __restrict__ vidx, uint64_t n, BrickDims b, uint32_t V) {
     const uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k < n) {
         const uint32_t j = vidx[k];
-        if (j < V) vidx[k] = brick_of(j, b);
+        const uint64_t past = brick_volume(b) + (static_cast<uint64_t>(j) - V);
+        vidx[k] = j < V ? brick_of(j, b) : past < 0xffffffffull ? static_cast<uint32_t>(past) : 0xffffffffu;
     }
 }
 
@@ -576,7 +579,8 @@ __global__ void k_unbrick_indices(const uint32_t* __restrict__ in, uint32_t* __r
     const uint64_t k = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k < n) {
         const uint32_t jb = in[k];
-        out[k] = jb == 0xffffffffu ? jb : unbrick(jb, b);
+        const uint64_t vb = brick_volume(b), V = static_cast<uint64_t>(b.nx) * b.ny * b.nz;
+        out[k] = jb == 0xffffffffu ? jb : jb < vb ? unbrick(jb, b) : static_cast<uint32_t>(jb - vb + V);
     }
 }
 
