@@ -428,6 +428,7 @@ struct muto_handle {
     uint64_t N = 0, npairs = 0;
     DevMem kept, sd, pr2, scat, pr64, off;
     DevMem vidx, L, T;            // muon-major pair lists
+    uint64_t vm_pairs = 0;        // pairs of the voxel-major copy: those of voxels in the image
     DevMem vm_mu, vm_LT;          // voxel-major copy (muon, (L, T))
     DevMem vclass;                // VoxDesc of every voxel, by segment-length class
     uint32_t vclass_n[kVoxClasses] = {};
@@ -1248,6 +1249,8 @@ void prepare_em(muto_handle* h) {
                 launch_segment_starts(h->mult.as<uint32_t>(), static_cast<uint32_t>(V), h->batch ? nullptr : &h->grid,
                                       mcol.as<uint32_t>(), scol.as<uint64_t>(), scratch.as<void>(), h->start.as<uint64_t>(), s);
             });
+            // (paths may hold pairs past the image, which have no place in a segment)
+            CK(cudaMemcpyAsync(&h->vm_pairs, h->start.as<uint64_t>() + V, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
         }
         {
@@ -1281,7 +1284,7 @@ void prepare_em(muto_handle* h) {
             run(h, "voxel_major", [&] {
                 launch_build_voxel_major<Real>(h->off.as<uint64_t>(), N, h->vidx.as<uint32_t>(), h->L.as<Real>(),
                                                h->T.as<Real>(), static_cast<uint32_t>(V), h->start.as<uint64_t>(),
-                                               cursor.as<uint32_t>(), Pn, staging.as<R4>(), h->vm_mu.as<uint32_t>(),
+                                               cursor.as<uint32_t>(), h->vm_pairs, staging.as<R4>(), h->vm_mu.as<uint32_t>(),
                                                h->vm_LT.as<typename Vec2<Real>::type>(),
                                                h->kslot.empty() ? nullptr : h->kslot.as<uint32_t>(), s);
             });
@@ -1943,7 +1946,7 @@ VoxelPassArgs<Real, OutT> voxel_args(muto_handle* h, const Real* lam, int mode, 
     v.grad = nullptr;
     v.lam64 = nullptr;
     v.keys = h->keys.as<typename KeyOf<Real>::type>();
-    v.P = h->npairs;
+    v.P = h->vm_pairs;
     v.win = (mode == kVoxMedian || mode == kVoxPercentile) && !h->win.empty() ? h->win.as<Real>() : nullptr;
     return v;
 }

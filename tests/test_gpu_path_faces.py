@@ -5,7 +5,7 @@ the second for nothing (src/MutoMLSD.cpp reads past its vector).  In every form 
 lists, with grids that fill whole bricks and grids that do not.
 
 Tolerances: FP64 1e-11 (sums of another order, three iterations), mixed 2e-5 (as in the
-other tests of the mixed lists).
+other tests of the mixed lists); medians and percentiles 1e-10 and 1e-4, as in theirs.
 """
 import numpy as np
 import pytest
@@ -56,7 +56,7 @@ def test_such_paths_leave_the_image(oracle, n):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", SIZES)
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("mixed", 2e-5)])
-@pytest.mark.parametrize("lists", ["muon_major"])
+@pytest.mark.parametrize("lists", ["muon_major", "voxel_major"])
 def test_they_count_as_in_the_oracle(gpu, oracle, n, precision, tol, lists):
     wl, rays = scan(n)
     cfg = wl.em_config(update_with_mean=True, mean_percentile=100, precision=precision, num_iteration=3, path_lists=lists)
@@ -68,6 +68,22 @@ def test_they_count_as_in_the_oracle(gpu, oracle, n, precision, tol, lists):
         if lists != "recompute":
             paths, want = rec.export_paths(), ref.export()
             assert np.array_equal(paths["off"], want["off"]) and np.array_equal(paths["idx"], want["idx"])
+    assert np.linalg.norm(img - ref.image()) <= tol * np.linalg.norm(ref.image())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 1e-4)])
+@pytest.mark.parametrize("layout", ["index", "columns"])
+@pytest.mark.parametrize("over", [{}, {"update_with_mean": True, "mean_percentile": 60}, {"muon_pass": "tile"}])
+def test_in_the_voxel_major_copy(gpu, oracle, n, precision, tol, layout, over):
+    wl, rays = scan(n)
+    cfg = wl.em_config(precision=precision, num_iteration=3, muon_layout=layout, **over)
+    ref = oracle.Mlsd(wl.grid, cfg, rays, np.full(wl.grid.nvox, 1e-7))
+    ref.iterate(3)
+    with M.MutoMLSD(cfg) as rec:
+        img = rec.reconstruct(rays).reshape(-1, order="F")
+        assert np.array_equal(rec.multiplicity(), np.bincount(ref.export()["idx"], minlength=wl.grid.nvox)[:wl.grid.nvox])
     assert np.linalg.norm(img - ref.image()) <= tol * np.linalg.norm(ref.image())
 
 
