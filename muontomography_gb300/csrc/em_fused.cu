@@ -522,13 +522,22 @@ __device__ __forceinline__ bool walk_path(const DevGrid& g, const muto_ray& r, c
     return ci >= 0 && co >= 0;
 }
 
+// A walked voxel's entry of lambda and G, kNoVoxel for one past the image.  A path just
+// below the upper x or y face has index nx or ny there: its flat index is the next row's
+// or plane's, as in the stored lists, or past the image.
+constexpr uint32_t kNoVoxel = 0xffffffffu;
+__device__ __forceinline__ uint32_t flat_index(uint32_t x, uint32_t y, uint32_t z, uint32_t nx, uint32_t nxy, uint32_t V) {
+    const uint32_t j = x + y * nx + z * nxy;  // xyz2index, include/MutoMLSD.h:76
+    return j < V ? j : kNoVoxel;
+}
 struct VoxelIndexer {
-    uint32_t nx, nxy;
+    uint32_t nx, ny, nxy, V;
     BrickDims b;
     int brick;
     __device__ __forceinline__ uint32_t operator()(uint32_t x, uint32_t y, uint32_t z) const {
-        if (!brick) return x + y * nx + z * nxy;  // xyz2index, include/MutoMLSD.h:76
-        return brick_xyz(x, y, z, b);
+        if (brick && x < nx && y < ny && z < b.nz) return brick_xyz(x, y, z, b);
+        const uint32_t j = flat_index(x, y, z, nx, nxy, V);
+        return brick && j != kNoVoxel ? brick_of(j, b) : j;
     }
 };
 
@@ -555,7 +564,8 @@ struct SumEmit {
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
         run += l;
         const double t = ltot - run;  // T_ij: the in-grid length after the pair
-        shift_in(ld_keep(lam + ix(x, y, z), keep), static_cast<Real>(l), static_cast<Real>(t > 0.0 ? t : 0.0));
+        const uint32_t j = ix(x, y, z);
+        shift_in(j != kNoVoxel ? ld_keep(lam + j, keep) : Real(0), static_cast<Real>(l), static_cast<Real>(t > 0.0 ? t : 0.0));
     }
     __device__ void drain() {  // the pairs still in flight, oldest first
         for (int k = 0; k < 3; ++k) shift_in(Real(0), Real(0), Real(0));
@@ -571,7 +581,8 @@ struct ScatterEmit {
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
         run += l;
         const double t = ltot - run;
-        red_add(G + ix(x, y, z), g_term(k0, k1, k2, static_cast<Real>(l), static_cast<Real>(t > 0.0 ? t : 0.0)), keep);
+        const uint32_t j = ix(x, y, z);
+        if (j != kNoVoxel) red_add(G + j, g_term(k0, k1, k2, static_cast<Real>(l), static_cast<Real>(t > 0.0 ? t : 0.0)), keep);
     }
 };
 
@@ -580,7 +591,7 @@ __global__ void __launch_bounds__(128) k_em_fused_walk(FusedArgs<Real> a) {
     using R4 = typename Vec4<Real>::type;
     double cost_local = 0.0;
     unsigned long long singular_local = 0;
-    const VoxelIndexer ix{a.g.n[0], a.g.n[0] * a.g.n[1], a.bdims, a.brick};
+    const VoxelIndexer ix{a.g.n[0], a.g.n[1], a.g.n[0] * a.g.n[1], a.g.n[0] * a.g.n[1] * a.g.n[2], a.bdims, a.brick};
     const uint64_t keep = l2_keep_policy();
     // a thread per muon (not a grid-stride loop, whose lanes would drift out
     // of step), the muons in a.order (by decreasing path bound) when given
@@ -610,11 +621,12 @@ __global__ void __launch_bounds__(128) k_em_fused_walk(FusedArgs<Real> a) {
 // drops) and the pairs per voxel M_j.
 struct StatEmit {
     uint32_t* mult;
-    uint32_t nx, nxy;
+    uint32_t nx, nxy, V;
     double run = 0.0;
     __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double l) {
         run += l;
-        atomicAdd(mult + (x + y * nx + z * nxy), 1u);
+        const uint32_t j = flat_index(x, y, z, nx, nxy, V);
+        if (j != kNoVoxel) atomicAdd(mult + j, 1u);
     }
 };
 __global__ void k_path_stats(const muto_ray* __restrict__ rays, const uint32_t* __restrict__ kept,
@@ -625,7 +637,7 @@ __global__ void k_path_stats(const muto_ray* __restrict__ rays, const uint32_t* 
     if (i >= n) return;
     const muto_ray r = rays[kept[i]];
     const double ps[3] = {scat[3 * i], scat[3 * i + 1], scat[3 * i + 2]};
-    StatEmit e{mult, g.n[0], g.n[0] * g.n[1]};
+    StatEmit e{mult, g.n[0], g.n[0] * g.n[1], g.n[0] * g.n[1] * g.n[2]};
     if (!walk_path(g, r, ps, straight, e, lanes)) {
         // dropped like the set-up's fill walk drops it; its voxels were counted
         // as they were walked, so count the same walk again with -1
@@ -638,8 +650,11 @@ __global__ void k_path_stats(const muto_ray* __restrict__ rays, const uint32_t* 
 
 struct UncountEmit {
     uint32_t* mult;
-    uint32_t nx, nxy;
-    __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double) { atomicSub(mult + (x + y * nx + z * nxy), 1u); }
+    uint32_t nx, nxy, V;
+    __device__ void operator()(uint32_t x, uint32_t y, uint32_t z, double) {
+        const uint32_t j = flat_index(x, y, z, nx, nxy, V);
+        if (j != kNoVoxel) atomicSub(mult + j, 1u);
+    }
 };
 __global__ void k_path_uncount(const muto_ray* __restrict__ rays, const uint32_t* __restrict__ kept,
                                const double* __restrict__ scat, uint64_t n, DevGrid g, int straight,
@@ -650,7 +665,7 @@ __global__ void k_path_uncount(const muto_ray* __restrict__ rays, const uint32_t
     if (!again) return;
     const muto_ray r = rays[kept[i]];
     const double ps[3] = {scat[3 * i], scat[3 * i + 1], scat[3 * i + 2]};
-    UncountEmit e{mult, g.n[0], g.n[0] * g.n[1]};
+    UncountEmit e{mult, g.n[0], g.n[0] * g.n[1], g.n[0] * g.n[1] * g.n[2]};
     walk_path(g, r, ps, straight, e, lanes);
 }
 

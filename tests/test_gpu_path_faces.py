@@ -56,7 +56,7 @@ def test_such_paths_leave_the_image(oracle, n):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", SIZES)
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("mixed", 2e-5)])
-@pytest.mark.parametrize("lists", ["muon_major", "voxel_major"])
+@pytest.mark.parametrize("lists", ["muon_major", "voxel_major", "recompute"])
 def test_they_count_as_in_the_oracle(gpu, oracle, n, precision, tol, lists):
     wl, rays = scan(n)
     cfg = wl.em_config(update_with_mean=True, mean_percentile=100, precision=precision, num_iteration=3, path_lists=lists)
