@@ -70,7 +70,8 @@ typedef struct muto_status {
     double cost_prev;           /* mean cost of the iteration before */
     uint64_t device_bytes;      /* device memory held by the handle */
     int32_t muon_pass;          /* muon-pass variant in use: 1 TMA tiles, 2 warp-batched, 3 the mean
-                                   update's one-pass form over stored lists, 4 its pass over recomputed
+                                   update's one-pass form over stored lists (in two passes where lambda
+                                   and its sums fill L2), 4 its pass over recomputed
                                    paths, 5 its split form (warp-batched muon pass, then a scatter pass),
                                    6 its one-pass form with each batch's pairs staged in shared memory */
     int32_t muon_group;         /* lanes per muon in its covariance sums */

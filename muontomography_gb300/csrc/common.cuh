@@ -438,10 +438,11 @@ int em_fused_blocks(int variant);  // resident CTAs per SM
 template <typename Real>
 void launch_em_fused(const FusedArgs<Real>& a, int variant, int blocks, cudaStream_t s);
 // The mixed form's one-pass kernel without block barriers: `group` (16 or 32)
-// lanes per muon; sums (N, or null): also adds every muon's cost to the
-// counters, through a second small kernel over the sums.
+// lanes per muon; two_passes: with 32 lanes, over the lists twice, the sums alone and
+// then the terms; sums: N entries of scratch.  With compute_cost every muon's cost is
+// added to the counters, by a small kernel over the sums.
 constexpr int once_held(int group) { return group <= 16 ? 8 : 7; }  // pairs held per lane
-void launch_em_once(const FusedArgs<float>& a, int group, float4* sums, int num_sms, cudaStream_t s);
+void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s);
 template <typename Real>
 void launch_em_fused_walk(const FusedArgs<Real>& a, int num_sms, cudaStream_t s);
 // split form: g_ij of every pair from the muon pass's coefficients kvec, added to G

@@ -992,7 +992,11 @@ __device__ __forceinline__ float once_g(const OnceCoef& o, float L, float u) {
     return o.c * L * fmaf(x, x, fmaf(y, y, fmaf(-o.f * d, d, fmaf(o.w * L, L, -o.h))));
 }
 
-template <int GROUP, int RC, int MB>
+// PASS: the whole of it; or the sums alone, left in `sums` (c0, c1, c2, R); or the
+// terms alone, from them.  Two passes read the lists twice, but each keeps one of
+// lambda and G in L2, where the two together do not fit (the rule's figures: handle.cu).
+enum OncePass { kOnceBoth, kOnceSums, kOnceTerms };
+template <int GROUP, int RC, int MB, int PASS>
 __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a, OnceErrors e, float4* __restrict__ sums) {
     constexpr int kPer = 32 / GROUP;  // muons of a warp at once
     constexpr int U = 4;              // loads in flight per lane for the pairs beyond the held ones
@@ -1026,11 +1030,12 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
                 }
             }
         }
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f), c = v;
         float pr2 = 0.f;
-        if (m < a.N) {
+        if (PASS != kOnceSums && m < a.N) {
             v = __ldcs(a.sd + m);
             pr2 = __ldcs(a.pr2 + m);
+            if (PASS == kOnceTerms) c = __ldcs(sums + m);
         }
         const uint32_t mn = m + step;
         uint64_t pbn = 0, pen = 0;
@@ -1039,119 +1044,126 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
             pen = a.off[mn + 1];
         }
 #pragma unroll
-        for (int r = 0; r < RC; ++r) {
-            cw[r] = 0.f;
-            if (cj[r] < V) cw[r] = ld_keep(a.lam + cj[r], keep);
-        }
+        for (int r = 0; r < RC; ++r) cU[r] = fmaf(0.5f, cL[r], cU[r]);
+        if constexpr (PASS == kOnceTerms) {
 #pragma unroll
-        for (int r = 0; r < RC; ++r) {
-            cU[r] = fmaf(0.5f, cL[r], cU[r]);
-            cw[r] *= cL[r];
-        }
-        float c0, c1, c2, at;
-        first_sums(cw, cU, c0, at);
-        // pairs beyond the held ones: read again below, from L1 or L2; their lambda is
-        // gathered once, so they are counted from centres of their own at first
-        Moments more{0.f, 0.f, 0.f, 0.f};
-        for (uint32_t k0 = glane + GROUP * RC; k0 < n; k0 += GROUP * U) {
-            uint32_t jj[U];
-            float ll[U], tt[U], lv[U];
+            for (int r = 0; r < RC; ++r) cU[r] -= c.w;
+        } else {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                jj[u] = 0xffffffffu;
-                ll[u] = tt[u] = 0.f;
-                if (k0 + u * GROUP < n) {
-                    jj[u] = __ldg(a.vidx + pb + k0 + u * GROUP);
-                    ll[u] = __ldg(a.L + pb + k0 + u * GROUP);
-                    tt[u] = __ldg(a.T + pb + k0 + u * GROUP);
+            for (int r = 0; r < RC; ++r) {
+                cw[r] = 0.f;
+                if (cj[r] < V) cw[r] = ld_keep(a.lam + cj[r], keep);
+            }
+#pragma unroll
+            for (int r = 0; r < RC; ++r) cw[r] *= cL[r];
+            float c0, c1, c2, at;
+            first_sums(cw, cU, c0, at);
+            // pairs beyond the held ones: read again below, from L1 or L2; their lambda is
+            // gathered once, so they are counted from centres of their own at first
+            Moments more{0.f, 0.f, 0.f, 0.f};
+            for (uint32_t k0 = glane + GROUP * RC; k0 < n; k0 += GROUP * U) {
+                uint32_t jj[U];
+                float ll[U], tt[U], lv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    jj[u] = 0xffffffffu;
+                    ll[u] = tt[u] = 0.f;
+                    if (k0 + u * GROUP < n) {
+                        jj[u] = __ldg(a.vidx + pb + k0 + u * GROUP);
+                        ll[u] = __ldg(a.L + pb + k0 + u * GROUP);
+                        tt[u] = __ldg(a.T + pb + k0 + u * GROUP);
+                    }
                 }
-            }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                lv[u] = 0.f;
-                if (jj[u] < V) lv[u] = ld_keep(a.lam + jj[u], keep);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                tt[u] = fmaf(0.5f, ll[u], tt[u]);
-                lv[u] *= ll[u];
-            }
-            Moments four;
-            first_sums(lv, tt, four.a, four.r);
-            c0 += four.a;
-            at += four.r;
-            four.r = centre(four.r, four.a, e.reach);
-            sums_about(four.r, lv, ll, tt, four.b1, four.b2);
-            more = both(more, four);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int o = GROUP / 2; o > 0; o >>= 1) {
-            c0 += __shfl_xor_sync(kFull, c0, o);
-            at += __shfl_xor_sync(kFull, at, o);
-        }
-        const float R = centre(at, c0, e.reach);  // (the sums are the same on every lane of the group)
-        sums_about(R, cw, cL, cU, c1, c2);
-        if (n > GROUP * RC) {
-            float b1, b2;
-            count_from(R, more, b1, b2);
-            c1 += b1;
-            c2 += b2;
-        }
-#pragma unroll
-        for (int o = GROUP / 2; o > 0; o >>= 1) {
-            c1 += __shfl_xor_sync(kFull, c1, o);
-            c2 += __shfl_xor_sync(kFull, c2, o);
-        }
-        OnceCoef o{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        unsigned sing = 0;
-        v = deviations_from(R, v);
-        if (m < a.N && !once_coefficients(c0, c1, c2, pr2, v, errors_from(R, e), o, sing)) {
-            // rare: the terms added here from the lists, and nothing below
-            float k0, k1, k2;
-            unsigned long long s64 = 0;
-            double cost = 0.0;
-            muon_coefficients<float>(c0, c1, c2, pr2, v, a.E00, e01_from(R, a.E00, a.E01), e11_from(R, a.E00, a.E01, a.E11),
-                                     false, k0, k1, k2, cost, s64);
-            sing = static_cast<unsigned>(s64);
-            for (uint32_t k = glane; k < n; k += GROUP) {
-                const uint32_t j = a.vidx[pb + k];
-                if (j < V) red_add(a.G + j, g_term(k0, k1, k2, a.L[pb + k], a.T[pb + k] - R), keep);
-            }
-            n = 0;
-#pragma unroll
-            for (int r = 0; r < RC; ++r) cj[r] = 0xffffffffu;
-        }
-        if (glane == 0) {
-            singular += sing;
-            if (sums && m < a.N) sums[m] = make_float4(c0, c1, c2, R);
-        }
-        auto put = [&](uint32_t j, float L, float u) {
-            if (j < V) red_add(a.G + j, once_g(o, L, u), keep);
-        };
-        for (uint32_t k0p = glane + GROUP * RC; k0p < n; k0p += GROUP * U) {
-            uint32_t jj[U];
-            float ll[U], tt[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                jj[u] = 0xffffffffu;
-                ll[u] = tt[u] = 0.f;
-                if (k0p + u * GROUP < n) {
-                    jj[u] = __ldcs(a.vidx + pb + k0p + u * GROUP);
-                    ll[u] = __ldcs(a.L + pb + k0p + u * GROUP);
-                    tt[u] = __ldcs(a.T + pb + k0p + u * GROUP);
+                for (int u = 0; u < U; ++u) {
+                    lv[u] = 0.f;
+                    if (jj[u] < V) lv[u] = ld_keep(a.lam + jj[u], keep);
                 }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    tt[u] = fmaf(0.5f, ll[u], tt[u]);
+                    lv[u] *= ll[u];
+                }
+                Moments four;
+                first_sums(lv, tt, four.a, four.r);
+                c0 += four.a;
+                at += four.r;
+                four.r = centre(four.r, four.a, e.reach);
+                sums_about(four.r, lv, ll, tt, four.b1, four.b2);
+                more = both(more, four);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = GROUP / 2; o > 0; o >>= 1) {
+                c0 += __shfl_xor_sync(kFull, c0, o);
+                at += __shfl_xor_sync(kFull, at, o);
+            }
+            const float R = centre(at, c0, e.reach);  // (the sums are the same on every lane of the group)
+            sums_about(R, cw, cL, cU, c1, c2);
+            if (n > GROUP * RC) {
+                float b1, b2;
+                count_from(R, more, b1, b2);
+                c1 += b1;
+                c2 += b2;
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) put(jj[u], ll[u], fmaf(0.5f, ll[u], tt[u]) - R);
+            for (int o = GROUP / 2; o > 0; o >>= 1) {
+                c1 += __shfl_xor_sync(kFull, c1, o);
+                c2 += __shfl_xor_sync(kFull, c2, o);
+            }
+            c = make_float4(c0, c1, c2, R);
         }
+        if (PASS != kOnceTerms && sums && glane == 0 && m < a.N) sums[m] = c;
+        if constexpr (PASS != kOnceSums) {
+            const float R = c.w;
+            OnceCoef o{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            unsigned sing = 0;
+            v = deviations_from(R, v);
+            if (m < a.N && !once_coefficients(c.x, c.y, c.z, pr2, v, errors_from(R, e), o, sing)) {
+                // rare: the terms added here from the lists, and nothing below
+                float k0, k1, k2;
+                unsigned long long s64 = 0;
+                double cost = 0.0;
+                muon_coefficients<float>(c.x, c.y, c.z, pr2, v, a.E00, e01_from(R, a.E00, a.E01), e11_from(R, a.E00, a.E01, a.E11),
+                                         false, k0, k1, k2, cost, s64);
+                sing = static_cast<unsigned>(s64);
+                for (uint32_t k = glane; k < n; k += GROUP) {
+                    const uint32_t j = a.vidx[pb + k];
+                    if (j < V) red_add(a.G + j, g_term(k0, k1, k2, a.L[pb + k], a.T[pb + k] - R), keep);
+                }
+                n = 0;
 #pragma unroll
-        for (int r = 0; r < RC; ++r) put(cj[r], cL[r], cU[r]);
+                for (int r = 0; r < RC; ++r) cj[r] = 0xffffffffu;
+            }
+            if (glane == 0) singular += sing;
+            auto put = [&](uint32_t j, float L, float u) {
+                if (j < V) red_add(a.G + j, once_g(o, L, u), keep);
+            };
+            for (uint32_t k0p = glane + GROUP * RC; k0p < n; k0p += GROUP * U) {
+                uint32_t jj[U];
+                float ll[U], tt[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    jj[u] = 0xffffffffu;
+                    ll[u] = tt[u] = 0.f;
+                    if (k0p + u * GROUP < n) {
+                        jj[u] = __ldcs(a.vidx + pb + k0p + u * GROUP);
+                        ll[u] = __ldcs(a.L + pb + k0p + u * GROUP);
+                        tt[u] = __ldcs(a.T + pb + k0p + u * GROUP);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) put(jj[u], ll[u], fmaf(0.5f, ll[u], tt[u]) - R);
+            }
+#pragma unroll
+            for (int r = 0; r < RC; ++r) put(cj[r], cL[r], cU[r]);
+        }
         m = mn;
         pb = pbn;
         n = static_cast<uint32_t>(pen - pbn);
         if (mw + step < mw) break;  // the next muons are past 2^32
     }
+    if (PASS == kOnceSums) return;
     singular = __reduce_add_sync(kFull, singular);
     if (lane == 0 && singular) atomicAdd(&a.ctr->singular, static_cast<unsigned long long>(singular));
 }
@@ -1207,24 +1219,32 @@ Df df_of(double x) {
     const float h = static_cast<float>(x);
     return Df{h, static_cast<float>(x - static_cast<double>(h))};
 }
-template <int GROUP, int RC, int MB>
+template <int GROUP, int MB, int PASS>
 void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t s) {
     const double at = a.E00 > 0.0 ? a.E01 / a.E00 : 0.0;
     const OnceErrors e{df_of(a.E00), df_of(a.E11 - at * a.E01), static_cast<float>(at), a.reach};
     const uint64_t need = (static_cast<uint64_t>(a.N) * GROUP + kOnceThreads - 1) / kOnceThreads;
     const uint64_t most = static_cast<uint64_t>(MB) * num_sms;
-    k_em_once<GROUP, RC, MB><<<static_cast<unsigned>(need < most ? need : most), kOnceThreads, 0, s>>>(a, e, sums);
+    k_em_once<GROUP, once_held(GROUP), MB, PASS>
+        <<<static_cast<unsigned>(need < most ? need : most), kOnceThreads, 0, s>>>(a, e, sums);
     count_launches(1);
 }
 }  // namespace
 
-void launch_em_once(const FusedArgs<float>& a, int group, float4* sums, int num_sms, cudaStream_t s) {
+void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s) {
     if (a.N == 0) return;
+    float4* const kept = a.compute_cost ? sums : nullptr;
     // blocks per SM: what the registers allow (32 lanes with 8 held pairs: six, or seven
     // with spills; 1.71 and 1.79 ms where seven with 7 held pairs take 1.68)
-    if (group <= 16) run_once<16, once_held(16), 6>(a, sums, num_sms, s);
-    else run_once<32, once_held(32), 7>(a, sums, num_sms, s);
-    if (sums) {
+    if (two_passes) {
+        run_once<32, 7, kOnceSums>(a, sums, num_sms, s);
+        run_once<32, 7, kOnceTerms>(a, sums, num_sms, s);
+    } else if (group <= 16) {
+        run_once<16, 6, kOnceBoth>(a, kept, num_sms, s);
+    } else {
+        run_once<32, 7, kOnceBoth>(a, kept, num_sms, s);
+    }
+    if (a.compute_cost) {
         constexpr uint64_t per = kCostMuons * kCostThreads;
         k_once_cost<<<static_cast<unsigned>((static_cast<uint64_t>(a.N) + per - 1) / per), kCostThreads, 0, s>>>(a, sums);
         count_launches(1);

@@ -448,6 +448,7 @@ struct muto_handle {
     DevMem ltot;                      // recompute: in-grid path length per kept muon
     int fused_variant = 1, fused_blocks = 0;  // stored-list fused pass: variant and persistent grid
     int once_group = 32;                         // lanes per muon of the one-pass mixed form
+    bool once_two = false;                       // its sums and its terms in a pass each
     int scatter_group = 32, scatter_blocks = 0;  // split form's scatter pass (fused_variant == kFusedVariants)
     int scatter_depth = 4;                       // its pairs in flight per lane
     // the split form overlapped: muon pass and scatter on chunks of the muons,
@@ -1508,7 +1509,7 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
     a.ctr = h->ctr();
     if constexpr (std::is_same<Real, float>::value) {
         if (h->lists == kListsMuonMajor && h->fused_variant == kFusedOnce) {
-            launch("em_fused", [&] { launch_em_once(a, h->once_group, cost ? h->kvec.as<float4>() : nullptr, h->num_sms, s); });
+            launch("em_fused", [&] { launch_em_once(a, h->once_group, h->once_two, h->kvec.as<float4>(), h->num_sms, s); });
             return;
         }
     }
@@ -1642,14 +1643,19 @@ void autotune_fused(muto_handle* h) {
     const double avg = h->N ? static_cast<double>(h->npairs) / static_cast<double>(h->N) : 0.0;
     const bool forced = h->P.fused_variant >= 0;
     if (!forced && !h->fp64() && !h->P.fused_prefetch) {
-        // Mixed: the one-pass kernel, faster than every other form on cubes of
-        // 16 to 150 voxels a side and on the 256 x 256 x 128 grid (mean paths of
-        // 23 to 221 pairs) and equal below, so nothing is timed here.  16 lanes
-        // a muon up to a mean path of 160 pairs, 32 beyond (0.8 M muons): 247
-        // against 438 us at 46 pairs, 309 against 455 at 91, 493 against 507 at
-        // 142, 759 against 686 at 213.
+        // Mixed: the one-pass kernel, nothing timed.  Lanes a muon: 16 up to a mean
+        // path of 160 pairs, 32 beyond (0.8 M muons: 247 against 438 us at 46 pairs,
+        // 309 against 455 at 91, 493 against 507 at 142, 759 against 686 at 213).
+        const uint64_t entries = h->brick ? h->vb : h->V();
         h->fused_variant = kFusedOnce;
         h->once_group = avg <= 160.0 ? 16 : 32;
+        // Where lambda and G together fill L2: a pass over the lists for each.  One pass /
+        // two, 4 M tracks: 300 x 300 x 128 (92 MB) 2.41 / 2.76 ms, 320 x 320 x 128 (105)
+        // 2.83 / 2.89, 345 x 345 x 128 (122) 3.19 / 3.00, 440 x 440 x 128 4.62 / 4.03,
+        // 320^3 8.87 / 8.02; below 100 pairs a path equal (1 200 x 1 200 x 24: 0.61 /
+        // 0.62).
+        h->once_two = avg > 100.0 && entries * 2 * sizeof(float) > h->l2_bytes / 8 * 7;
+        if (h->once_two) h->once_group = 32;
         h->overlap = false;
         return;
     }
