@@ -134,7 +134,7 @@ typedef struct muto_handle muto_handle;
  * "muon_major" and "recompute" require the mean update),
  * "fused_variant" ("auto": the mean update's pass over muon-major lists
  * is, in the mixed form, the one-pass kernel without block barriers, its
- * lanes per muon by the scan's mean path; in fp64 the split form (the muon
+ * lanes per muon by the scan's mean path, muons and voxels; in fp64 the split form (the muon
  * pass, then a second pass over the lists adding the terms); with
  * "fused_prefetch" the one-pass variants that suit the mean path and the
  * split form are timed at prepare; "4x8", "8x4",

@@ -437,11 +437,12 @@ template <typename Real>
 int em_fused_blocks(int variant);  // resident CTAs per SM
 template <typename Real>
 void launch_em_fused(const FusedArgs<Real>& a, int variant, int blocks, cudaStream_t s);
-// The mixed form's one-pass kernel without block barriers: `group` (16 or 32)
+// The mixed form's one-pass kernel without block barriers: `group` (4, 8, 16 or 32)
 // lanes per muon; two_passes: with 32 lanes, over the lists twice, the sums alone and
 // then the terms; sums: N entries of scratch.  With compute_cost every muon's cost is
 // added to the counters, by a small kernel over the sums.
 constexpr int once_held(int group) { return group <= 16 ? 8 : 7; }  // pairs held per lane
+int em_once_muons16(int num_sms);  // muons worked on at once with 16 lanes each
 void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s);
 template <typename Real>
 void launch_em_fused_walk(const FusedArgs<Real>& a, int num_sms, cudaStream_t s);

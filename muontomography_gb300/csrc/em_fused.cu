@@ -1231,6 +1231,8 @@ void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t
 }
 }  // namespace
 
+int em_once_muons16(int num_sms) { return 6 * (kOnceThreads / 16) * num_sms; }
+
 void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s) {
     if (a.N == 0) return;
     float4* const kept = a.compute_cost ? sums : nullptr;
@@ -1239,6 +1241,10 @@ void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float
     if (two_passes) {
         run_once<32, 7, kOnceSums>(a, sums, num_sms, s);
         run_once<32, 7, kOnceTerms>(a, sums, num_sms, s);
+    } else if (group <= 4) {
+        run_once<4, 6, kOnceBoth>(a, kept, num_sms, s);
+    } else if (group <= 8) {
+        run_once<8, 6, kOnceBoth>(a, kept, num_sms, s);
     } else if (group <= 16) {
         run_once<16, 6, kOnceBoth>(a, kept, num_sms, s);
     } else {

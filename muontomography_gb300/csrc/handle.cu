@@ -1646,9 +1646,20 @@ void autotune_fused(muto_handle* h) {
         // Mixed: the one-pass kernel, nothing timed.  Lanes a muon: 16 up to a mean
         // path of 160 pairs, 32 beyond (0.8 M muons: 247 against 438 us at 46 pairs,
         // 309 against 455 at 91, 493 against 507 at 142, 759 against 686 at 213).
+        // Shorter paths leave 16 lanes idle: 8 up to 48 pairs (16 / 8 lanes: 131 / 78 us
+        // on 64 x 64 x 16 voxels, 30 pairs, 0.4 M muons; 125 / 85 at 38 pairs; 112 / 121
+        // at 51), 4 up to 20 (8 / 4: 109 / 68 us on 100 x 100 x 6, 12 pairs, 0.67 M
+        // muons; 51 / 37 at 16; 15 / 16 at 23).  Not where there are no more muons than
+        // groups of 16 lanes at once, nor where so few voxels take the reductions that
+        // more muons at once only collide (12^3 voxels: 234 / 238 / 262 us with 16 / 8 /
+        // 4 lanes; 32 x 32 x 8, 15 pairs: 211 / 158 / 159).
         const uint64_t entries = h->brick ? h->vb : h->V();
         h->fused_variant = kFusedOnce;
         h->once_group = avg <= 160.0 ? 16 : 32;
+        if (h->N > static_cast<uint64_t>(em_once_muons16(h->num_sms))) {
+            if (avg <= 20.0 && entries >= 32768) h->once_group = 4;
+            else if (avg <= 48.0 && entries >= 4096) h->once_group = 8;
+        }
         // Where lambda and G together fill L2: a pass over the lists for each.  One pass /
         // two, 4 M tracks: 300 x 300 x 128 (92 MB) 2.41 / 2.76 ms, 320 x 320 x 128 (105)
         // 2.83 / 2.89, 345 x 345 x 128 (122) 3.19 / 3.00, 440 x 440 x 128 4.62 / 4.03,

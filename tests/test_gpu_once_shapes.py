@@ -1,6 +1,7 @@
-"""The mixed form's one-pass mean kernel in two passes (grids whose lambda and sums outgrow
-L2): images against the FP64 form, and the sums of g_ij where one layer holds most of
-every muon's sum lambda L.
+"""The mixed form's one-pass mean kernel on short paths (4 and 8 lanes a muon, where there
+are muons enough to fill the GPU) and in two passes (grids whose lambda and sums outgrow
+L2): images against the FP64 oracle or form, and the sums of g_ij where one layer holds
+most of every muon's sum lambda L.  Paths within the held pairs (32 and 64) and beyond.
 
 Tolerances: as in test_gpu_once.py (2e-5 after three iterations) and
 test_gpu_once_moments.py (1e-4 for the sums of a heavy layer).
@@ -28,6 +29,28 @@ def scan(nx, ny, nz, mm, n_muons, seed):
     return W.Workload("scan", g, blocks, n_muons, seed, True, 3)
 
 
+# (voxels, mm, tracks, lanes a muon: 16 where there are few muons or few voxels)
+SHORT = [(70, 66, 8, 20.0, 60_011, 4), (70, 66, 1, 200.0, 90_001, 4), (200, 170, 1, 20.0, 200_003, 16),
+         (97, 101, 12, 15.0, 50_001, 8), (40, 41, 20, 20.0, 40_009, 8), (25, 24, 12, 20.0, 60_007, 8),
+         (64, 60, 19, 20.0, 40_003, 8), (70, 66, 8, 20.0, 9_001, 16), (12, 12, 12, 50.0, 60_000, 16)]
+
+
+@pytest.mark.parametrize("nx,ny,nz,mm,n_muons,group", SHORT)
+def test_short_paths_match_oracle(gpu, oracle, nx, ny, nz, mm, n_muons, group):
+    wl = scan(nx, ny, nz, mm, n_muons, 83)
+    rays = wl.tracks()
+    cfg = wl.em_config(update_with_mean=True, precision="mixed", compute_cost=True)
+    ref = oracle.Mlsd(wl.grid, cfg, rays, np.full(wl.grid.nvox, 1e-7))
+    ref.iterate(3)
+    with M.MutoMLSD(cfg) as rec:
+        img = rec.reconstruct(rays).reshape(-1, order="F")
+        st = rec.status()
+    assert st["muon_pass"] == 3 and st["muon_group"] == group
+    assert st["n_singular"] == ref.counts()["n_singular"]
+    assert rel_l2(img, ref.image()) < 2e-5
+    assert abs(st["cost"] - ref.costs()[-1]) <= 1e-5 * abs(ref.costs()[-1])
+
+
 def g_sums(wl, rays, x, precision):
     with M.MutoMLSD(wl.em_config(update_with_mean=True, precision=precision, num_iteration=0)) as rec:
         rec.load_tracks(rays)
@@ -41,6 +64,17 @@ def heavy_layer(wl, height):
     x = np.full(g.nvox, np.log(1.0e-7))
     x[np.arange(g.nvox) // (g.nx * g.ny) == int(height * g.nz)] = np.log(0.05)
     return x
+
+
+@pytest.mark.parametrize("nx,ny,nz,mm,n_muons,group", [s for s in SHORT if s[5] < 16 and s[2] > 1])
+def test_one_heavy_layer(gpu, nx, ny, nz, mm, n_muons, group):
+    wl = scan(nx, ny, nz, mm, n_muons, 84)
+    rays = wl.tracks()
+    x = heavy_layer(wl, 0.9)
+    v64, g64, _ = g_sums(wl, rays, x, "fp64")
+    v, g, st = g_sums(wl, rays, x, "mixed")
+    assert st["muon_group"] == group
+    assert rel_l2(g, g64) < 1e-4 and abs(v - v64) <= 1e-4 * abs(v64)
 
 
 def images(wl, rays, precision):
