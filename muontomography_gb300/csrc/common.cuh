@@ -295,7 +295,8 @@ template <typename Real>
 int em_muon_blocks(int tile_pairs, int tile_muons, int group);
 // warp-batched variant of the muon pass (no shared memory)
 template <typename Real>
-void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int blocks, int group, cudaStream_t s);
+void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int blocks, int group, int num_sms,
+                         cudaStream_t s);
 template <typename Real>
 int em_muon_warp_blocks(int group);
 

@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_em_muon(MuonPassArgs<Real> a, i
 // WEIGHTS (FP64): the pairs hold W01 and W11 beside L, so a pair costs three
 // FP64 operations instead of eight.
 template <typename Real, int GROUP, bool WEIGHTS>
-__global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a, uint32_t n_muons) {
+__global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a, uint32_t n_muons, int batch) {
     using R4 = typename Vec4<Real>::type;
     constexpr int U = 5;                    // pair loads in flight per lane per round
     constexpr int kPer = 32 / GROUP;        // muons summed at once per warp
@@ -307,14 +307,14 @@ __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a,
     const uint32_t V = a.V;
     const uint64_t warp = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    const uint64_t nbatch = (static_cast<uint64_t>(n_muons) + 31) / 32;
+    const uint64_t nbatch = (static_cast<uint64_t>(n_muons) + batch - 1) / batch;
     double cost_local = 0.0;
     unsigned long long singular_local = 0;
 
     for (uint64_t bt = warp; bt < nbatch; bt += nwarps) {
-        const uint64_t m0 = bt * 32;
+        const uint64_t m0 = bt * batch;
         Real my0 = 0, my1 = 0, my2 = 0;  // the sums of muon m0 + lane
-        for (int q = 0; q < 32; q += kPer) {
+        for (int q = 0; q < batch; q += kPer) {
             const uint64_t mi = m0 + q + sub;
             Real c0 = 0, c1 = 0, c2 = 0;
             if (mi < n_muons) {
@@ -376,8 +376,8 @@ __global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a,
                 my2 = v2;
             }
         }
-        // ---- FP64 2x2 algebra of the warp's 32 muons, one per lane ----------
-        if (m0 + lane < n_muons) {
+        // ---- FP64 2x2 algebra of the warp's muons, one per lane ----------
+        if (lane < batch && m0 + lane < n_muons) {
             const uint64_t m = a.order ? a.order[m0 + lane] : m0 + lane;
             const Real pr2 = a.pr2[m];
             const double p2 = static_cast<double>(pr2);
@@ -491,22 +491,33 @@ template int em_muon_warp_blocks<float>(int);
 template int em_muon_warp_blocks<double>(int);
 
 template <typename Real>
-void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int blocks, int group, cudaStream_t s) {
+void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int blocks, int group, int num_sms, cudaStream_t s) {
     if (n_muons == 0) return;
-    const uint64_t batches = (static_cast<uint64_t>(n_muons) + 31) / 32;
-    const uint64_t need = (batches + kThreads / 32 - 1) / (kThreads / 32);
+    // Muons a batch: 32, so that the FP64 algebra runs on full warps; fewer of few muons,
+    // whose time is a warp's rounds one after another, down to one round, as long as an
+    // SM has no more than eight batches (an iteration of the FP64 mean update on 40^3
+    // voxels: 11.7 k muons 66 -> 47 us; on 12^3: 2.1 k 34 -> 23, 10.7 k 37 -> 32).
+    const int per = 32 / (group <= 4 ? 4 : group <= 8 ? 8 : group <= 16 ? 16 : 32);
+    int batch = 32;
+    while (batch / 2 >= per && n_muons <= 8ull * num_sms * (batch / 2)) batch /= 2;
+    const uint64_t batches = (static_cast<uint64_t>(n_muons) + batch - 1) / batch;
+    // (nothing is shared in a block: with fewer batches than warps of a block on each SM
+    // the blocks are smaller)
+    int threads = kThreads;
+    while (threads > 32 && batches <= static_cast<uint64_t>(num_sms) * (threads / 64)) threads /= 2;
+    const uint64_t need = (batches + threads / 32 - 1) / (threads / 32);
     const unsigned nb = static_cast<unsigned>(need < static_cast<uint64_t>(blocks) ? need : blocks);
     auto go = [&](auto w) {
         constexpr bool W = decltype(w)::value;
         if constexpr (sizeof(Real) == 8) {
             if (group <= 4) {
-                k_em_muon_warp<Real, 4, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+                k_em_muon_warp<Real, 4, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
                 return;
             }
         }
-        if (group <= 8) k_em_muon_warp<Real, 8, W><<<nb, kThreads, 0, s>>>(a, n_muons);
-        else if (group <= 16) k_em_muon_warp<Real, 16, W><<<nb, kThreads, 0, s>>>(a, n_muons);
-        else k_em_muon_warp<Real, 32, W><<<nb, kThreads, 0, s>>>(a, n_muons);
+        if (group <= 8) k_em_muon_warp<Real, 8, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
+        else if (group <= 16) k_em_muon_warp<Real, 16, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
+        else k_em_muon_warp<Real, 32, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
     };
     if constexpr (sizeof(Real) == 8) {
         if (a.W11) go(std::true_type{});
@@ -516,7 +527,7 @@ void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int bloc
     }
     count_launches(1);
 }
-template void launch_em_muon_warp<float>(const MuonPassArgs<float>&, uint32_t, int, int, cudaStream_t);
-template void launch_em_muon_warp<double>(const MuonPassArgs<double>&, uint32_t, int, int, cudaStream_t);
+template void launch_em_muon_warp<float>(const MuonPassArgs<float>&, uint32_t, int, int, int, cudaStream_t);
+template void launch_em_muon_warp<double>(const MuonPassArgs<double>&, uint32_t, int, int, int, cudaStream_t);
 
 }  // namespace muto

@@ -1418,7 +1418,7 @@ void launch_muon_pass(muto_handle* h, const MuonPassArgs<Real>& a_in, cudaStream
         a.V = static_cast<uint32_t>(h->vb);
     }
     if (h->muon_kind == 2)
-        launch_em_muon_warp<Real>(a, static_cast<uint32_t>(h->N), h->warp_blocks, h->muon_group, s);
+        launch_em_muon_warp<Real>(a, static_cast<uint32_t>(h->N), h->warp_blocks, h->muon_group, h->num_sms, s);
     else
         launch_em_muon<Real>(a, h->tile_pairs, h->tile_muons, h->tile_blocks, h->group, s);
 }
@@ -1545,7 +1545,7 @@ void launch_fused_pass(muto_handle* h, const Real* lam, bool cost, cudaStream_t 
             mc.sd += m0;
             mc.pr2 += m0;
             mc.kout += m0;
-            launch_em_muon_warp<Real>(mc, static_cast<uint32_t>(m1 - m0), h->warp_blocks_ov, h->muon_group, s);
+            launch_em_muon_warp<Real>(mc, static_cast<uint32_t>(m1 - m0), h->warp_blocks_ov, h->muon_group, h->num_sms, s);
             CK(cudaEventRecord(h->ov_ev[c], s));
             CK(cudaStreamWaitEvent(side, h->ov_ev[c], 0));
             FusedArgs<Real> ac = a;
