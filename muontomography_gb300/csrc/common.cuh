@@ -63,6 +63,16 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// 1 / x: one third-order step in FP64 from the FP32 reciprocal (an error of 2^-23
+// becomes 2^-66), three dependent operations instead of a division's dozen; outside
+// the FP32 range (and for 0, infinities and NaN) the division.
+__device__ __forceinline__ double reciprocal(double x) {
+    const float f = static_cast<float>(x);
+    if (!(f > 1.0e-30f && f < 1.0e30f)) return __ddiv_rn(1.0, x);
+    const double r = static_cast<double>(1.0f / f), e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // Warp-aggregated increment of a global counter by the number of lanes with pred.
 __device__ __forceinline__ void warp_count(unsigned long long* ctr, bool pred) {
     const unsigned b = __ballot_sync(__activemask(), pred);
@@ -440,8 +450,8 @@ template <typename Real>
 void launch_em_fused(const FusedArgs<Real>& a, int variant, int blocks, cudaStream_t s);
 // The mixed form's one-pass kernel without block barriers: `group` (4, 8, 16 or 32)
 // lanes per muon; two_passes: with 32 lanes, over the lists twice, the sums alone and
-// then the terms; sums: N entries of scratch.  With compute_cost every muon's cost is
-// added to the counters, by a small kernel over the sums.
+// then the terms, with N entries of scratch (sums).  With compute_cost every muon's
+// cost is added to the counters.
 constexpr int once_held(int group) { return group <= 16 ? 8 : 7; }  // pairs held per lane
 int em_once_muons16(int num_sms);  // muons worked on at once with 16 lanes each
 void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s);

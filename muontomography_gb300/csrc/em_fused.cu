@@ -992,11 +992,87 @@ __device__ __forceinline__ float once_g(const OnceCoef& o, float L, float u) {
     return o.c * L * fmaf(x, x, fmaf(y, y, fmaf(-o.f * d, d, fmaf(o.w * L, L, -o.h))));
 }
 
+// The cost of muons (src/MutoMLSD.cpp:465-468) in FP64: the sum of their quadratic forms
+// and one product of their determinants' mantissas, whose exponent is moved to an
+// integer after each (exact), so that a block takes one logarithm.  A warp of k_em_once
+// puts its muons' sums aside in shared memory and works out 32 of them at a time, a
+// muon a lane: an FP64 instruction takes the SM's pipe for 16 cycles however few lanes
+// are active, and here it runs beside the other warps' loads.  100 x 100 x 6 voxels,
+// 0.33 M muons: an iteration 56 us with the cost, 39 without; 83 with a kernel of its
+// own for the cost over the muons' sums (50 k muons: 25, 17 and 31).
+struct CostSum {
+    double forms = 0.0, prod = 1.0;  // prod in [1, 2)
+    int ex = 0;
+    __device__ __forceinline__ void add(const FusedArgs<float>& a, const float4& c, const float4& v, float pr2) {
+        const double p2 = pr2, R = c.w;  // the sums, and so all of this, counted from R
+        const double S00 = p2 * c.x + a.E00, S01 = p2 * c.y + e01_from(R, a.E00, a.E01),
+                     S11 = p2 * c.z + e11_from(R, a.E00, a.E01, a.E11);
+        double det = S00 * S11 - S01 * S01;
+        if (!(det > 1e-12)) return;  // cost 0; counted with the terms
+        const double sx = v.x, dx = v.y - R * sx, sy = v.z, dy = v.w - R * sy;
+        forms = fma((sx * sx + sy * sy) * S11 + (dx * dx + dy * dy) * S00 - (sx * dx + sy * dy) * 2.0 * S01,
+                    reciprocal(det), forms);
+        if (det > 1.0e300) {
+            if (isinf(det)) {
+                forms += det;
+                return;
+            }
+            det *= 0x1p-64;
+            ex += 64;
+        }
+        const double q = prod * det;  // a normal number: 1e-12 < q < 2e300
+        const int hi = __double2hiint(q), e = (hi >> 20) - 1023;
+        ex += e;
+        prod = __hiloint2double(hi - (e << 20), __double2loint(q));
+    }
+};
+struct CostHeld {  // a warp's muons put aside: (c0, c1, c2, R), (S, D), pr^2 (-1: none)
+    float4 c[32], v[32];
+    float pr2[32];
+};
+// The block's muons to the counters: those that its warps still have aside (`kept` each)
+// on as few warps as they fill, then one sum and one logarithm a block.
+template <int WARPS>
+__device__ __forceinline__ void finish_cost(const FusedArgs<float>& a, const CostHeld* held, int kept, CostSum t, bool used) {
+    __shared__ double forms[WARPS], prods[WARPS];
+    __shared__ int exs[WARPS], left[WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) left[warp] = kept;
+    __syncthreads();
+    int k = threadIdx.x, w = 0;
+    while (w < WARPS && k >= left[w]) k -= left[w++];
+    if (w < WARPS && held[w].pr2[k] >= 0.f) t.add(a, held[w].c[k], held[w].v[k], held[w].pr2[k]);
+    used = used || __any_sync(kFull, w < WARPS);
+    double f = 0.0, p = 1.0;
+    int ex = 0;
+    if (used) {  // (a warp without muons spends no FP64 operations)
+        f = warp_sum(t.forms);
+        p = t.prod;  // below 2^32 for a warp, 2^(32 WARPS) for a block
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) p *= __shfl_xor_sync(kFull, p, o);
+        ex = __reduce_add_sync(kFull, t.ex);
+    }
+    if (lane == 0) forms[warp] = f, prods[warp] = p, exs[warp] = ex;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double sum = 0.0, prod = 1.0;
+        long long e = 0;
+        for (int q = 0; q < WARPS; ++q) {
+            sum += forms[q];
+            prod *= prods[q];
+            e += exs[q];
+        }
+        sum = 0.5 * sum + log(prod) + static_cast<double>(e) * 0.69314718055994530942;  // ln 2
+        if (sum != 0.0) atomicAdd(&a.ctr->cost_sum, sum);
+    }
+}
+
 // PASS: the whole of it; or the sums alone, left in `sums` (c0, c1, c2, R); or the
 // terms alone, from them.  Two passes read the lists twice, but each keeps one of
 // lambda and G in L2, where the two together do not fit (the rule's figures: handle.cu).
 enum OncePass { kOnceBoth, kOnceSums, kOnceTerms };
-template <int GROUP, int RC, int MB, int PASS>
+// COST: also adds the muons' cost to the counters.
+template <int GROUP, int RC, int MB, int PASS, bool COST>
 __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a, OnceErrors e, float4* __restrict__ sums) {
     constexpr int kPer = 32 / GROUP;  // muons of a warp at once
     constexpr int U = 4;              // loads in flight per lane for the pairs beyond the held ones
@@ -1005,6 +1081,11 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
     const uint64_t keep = l2_keep_policy();
     const uint32_t step = ((gridDim.x * blockDim.x) >> 5) * kPer;
     unsigned singular = 0;
+    [[maybe_unused]] __shared__ CostHeld held[COST ? kOnceThreads / 32 : 1];
+    [[maybe_unused]] CostHeld& aside = held[COST ? threadIdx.x >> 5 : 0];
+    [[maybe_unused]] CostSum cost;
+    [[maybe_unused]] int kept = 0;  // of the warp's muons in `aside`
+    [[maybe_unused]] bool used = false;
     uint32_t m = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kPer + sub;
     uint64_t pb = 0;
     uint32_t n = 0;
@@ -1113,8 +1194,13 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
             }
             c = make_float4(c0, c1, c2, R);
         }
-        if (PASS != kOnceTerms && sums && glane == 0 && m < a.N) sums[m] = c;
+        if (PASS == kOnceSums && glane == 0 && m < a.N) sums[m] = c;
         if constexpr (PASS != kOnceSums) {
+            if (COST && glane == 0) {
+                aside.c[kept + sub] = c;
+                aside.v[kept + sub] = v;
+                aside.pr2[kept + sub] = m < a.N ? pr2 : -1.f;
+            }
             const float R = c.w;
             OnceCoef o{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             unsigned sing = 0;
@@ -1157,6 +1243,16 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
             }
 #pragma unroll
             for (int r = 0; r < RC; ++r) put(cj[r], cL[r], cU[r]);
+            if constexpr (COST) {
+                kept += kPer;
+                if (kept == 32) {
+                    __syncwarp();
+                    if (aside.pr2[lane] >= 0.f) cost.add(a, aside.c[lane], aside.v[lane], aside.pr2[lane]);
+                    __syncwarp();
+                    kept = 0;
+                    used = true;
+                }
+            }
         }
         m = mn;
         pb = pbn;
@@ -1166,50 +1262,7 @@ __global__ void __launch_bounds__(kOnceThreads, MB) k_em_once(FusedArgs<float> a
     if (PASS == kOnceSums) return;
     singular = __reduce_add_sync(kFull, singular);
     if (lane == 0 && singular) atomicAdd(&a.ctr->singular, static_cast<unsigned long long>(singular));
-}
-
-// The cost of every muon (src/MutoMLSD.cpp:465-468) from the sums that k_em_once
-// left, in FP64.  Bound by FP64 work, most of it the logarithm and the division: a
-// thread takes kCostMuons muons with one logarithm of the product of their
-// determinants' mantissas (each product's exponent is moved to an integer, which
-// is exact), and their divisions' latencies overlap.  897 k muons: 81 us;
-// 122 us with a logarithm a muon.
-constexpr int kCostMuons = 4, kCostThreads = 256;
-__global__ void __launch_bounds__(kCostThreads) k_once_cost(FusedArgs<float> a, const float4* __restrict__ sums) {
-    const uint64_t m0 = static_cast<uint64_t>(blockIdx.x) * (kCostMuons * kCostThreads) + threadIdx.x;
-    float4 cs[kCostMuons], vs[kCostMuons];
-    float ps[kCostMuons];
-#pragma unroll
-    for (int u = 0; u < kCostMuons; ++u) {  // (a muon past the end repeats the last one's loads)
-        const uint64_t m = m0 + u * kCostThreads < a.N ? m0 + u * kCostThreads : a.N - 1;
-        cs[u] = sums[m];
-        vs[u] = a.sd[m];
-        ps[u] = a.pr2[m];
-    }
-    double cost = 0.0, prod = 1.0;
-    int ex = 0;
-#pragma unroll
-    for (int u = 0; u < kCostMuons; ++u) {
-        if (m0 + u * kCostThreads >= a.N) continue;
-        const float4 c = cs[u], v = vs[u];
-        const double p2 = ps[u], R = c.w;  // the sums, and so all of this, counted from R
-        const double S00 = p2 * c.x + a.E00, S01 = p2 * c.y + e01_from(R, a.E00, a.E01),
-                     S11 = p2 * c.z + e11_from(R, a.E00, a.E01, a.E11);
-        const double det = S00 * S11 - S01 * S01;
-        if (!(det > 1e-12)) continue;  // cost 0; counted by k_em_once
-        const double sx = v.x, dx = v.y - R * sx, sy = v.z, dy = v.w - R * sy;
-        cost += ((sx * sx + sy * sy) * S11 + (dx * dx + dy * dy) * S00 - (sx * dx + sy * dy) * 2.0 * S01) / det;
-        if (det > 1.0e300) {
-            cost += 2.0 * log(det);
-            continue;
-        }
-        const double q = prod * det;  // a normal number: 1e-12 < q < 2e300
-        const int hi = __double2hiint(q), e = (hi >> 20) - 1023;
-        ex += e;
-        prod = __hiloint2double(hi - (e << 20), __double2loint(q));  // [1, 2)
-    }
-    cost = 0.5 * cost + log(prod) + ex * 0.69314718055994530942;  // ln 2
-    flush_counters<kCostThreads>(cost, 0ull, 1, a.ctr);
+    if constexpr (COST) finish_cost<kOnceThreads / 32>(a, held, kept, cost, used);
 }
 
 }  // namespace
@@ -1219,13 +1272,13 @@ Df df_of(double x) {
     const float h = static_cast<float>(x);
     return Df{h, static_cast<float>(x - static_cast<double>(h))};
 }
-template <int GROUP, int MB, int PASS>
+template <int GROUP, int MB, int PASS, bool COST>
 void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t s) {
     const double at = a.E00 > 0.0 ? a.E01 / a.E00 : 0.0;
     const OnceErrors e{df_of(a.E00), df_of(a.E11 - at * a.E01), static_cast<float>(at), a.reach};
     const uint64_t need = (static_cast<uint64_t>(a.N) * GROUP + kOnceThreads - 1) / kOnceThreads;
     const uint64_t most = static_cast<uint64_t>(MB) * num_sms;
-    k_em_once<GROUP, once_held(GROUP), MB, PASS>
+    k_em_once<GROUP, once_held(GROUP), MB, PASS, COST>
         <<<static_cast<unsigned>(need < most ? need : most), kOnceThreads, 0, s>>>(a, e, sums);
     count_launches(1);
 }
@@ -1233,28 +1286,30 @@ void run_once(const FusedArgs<float>& a, float4* sums, int num_sms, cudaStream_t
 
 int em_once_muons16(int num_sms) { return 6 * (kOnceThreads / 16) * num_sms; }
 
-void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s) {
-    if (a.N == 0) return;
-    float4* const kept = a.compute_cost ? sums : nullptr;
+namespace {
+template <bool COST>
+void run_once_as(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s) {
     // blocks per SM: what the registers allow (32 lanes with 8 held pairs: six, or seven
     // with spills; 1.71 and 1.79 ms where seven with 7 held pairs take 1.68)
     if (two_passes) {
-        run_once<32, 7, kOnceSums>(a, sums, num_sms, s);
-        run_once<32, 7, kOnceTerms>(a, sums, num_sms, s);
+        run_once<32, 7, kOnceSums, false>(a, sums, num_sms, s);
+        run_once<32, 7, kOnceTerms, COST>(a, sums, num_sms, s);
     } else if (group <= 4) {
-        run_once<4, 6, kOnceBoth>(a, kept, num_sms, s);
+        run_once<4, 6, kOnceBoth, COST>(a, sums, num_sms, s);
     } else if (group <= 8) {
-        run_once<8, 6, kOnceBoth>(a, kept, num_sms, s);
+        run_once<8, 6, kOnceBoth, COST>(a, sums, num_sms, s);
     } else if (group <= 16) {
-        run_once<16, 6, kOnceBoth>(a, kept, num_sms, s);
+        run_once<16, 6, kOnceBoth, COST>(a, sums, num_sms, s);
     } else {
-        run_once<32, 7, kOnceBoth>(a, kept, num_sms, s);
+        run_once<32, 7, kOnceBoth, COST>(a, sums, num_sms, s);
     }
-    if (a.compute_cost) {
-        constexpr uint64_t per = kCostMuons * kCostThreads;
-        k_once_cost<<<static_cast<unsigned>((static_cast<uint64_t>(a.N) + per - 1) / per), kCostThreads, 0, s>>>(a, sums);
-        count_launches(1);
-    }
+}
+}  // namespace
+
+void launch_em_once(const FusedArgs<float>& a, int group, bool two_passes, float4* sums, int num_sms, cudaStream_t s) {
+    if (a.N == 0) return;
+    if (a.compute_cost) run_once_as<true>(a, group, two_passes, sums, num_sms, s);
+    else run_once_as<false>(a, group, two_passes, sums, num_sms, s);
 }
 
 // (GROUP, RC) of each stored-list variant; the last is the staged one (GROUP

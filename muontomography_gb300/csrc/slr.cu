@@ -213,17 +213,6 @@ __global__ void k_slr_flatten(SlrPass p, const uint32_t* __restrict__ order, con
     }
 }
 
-// 1 / x for the paths' sums: one third-order step in FP64 from the FP32
-// reciprocal (an error of 2^-23 becomes 2^-66), three dependent operations
-// instead of a division's dozen; outside the FP32 range (and for 0, infinities
-// and NaN) the division.
-__device__ __forceinline__ double slr_reciprocal(double x) {
-    const float f = static_cast<float>(x);
-    if (!(f > 1.0e-30f && f < 1.0e30f)) return ddiv(1.0, x);
-    const double r = static_cast<double>(1.0f / f), e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 // A later pass level by level.  A muon's level is one more than the highest
 // level among the earlier muons that share a voxel with it, so two muons of
 // one level share no voxel, and every voxel meets its muons in index order:
@@ -327,7 +316,7 @@ __global__ void __launch_bounds__(THREADS) k_slr_iter_steps(SlrArgs a, SlrFlat f
             __syncwarp();
 #pragma unroll
             for (int d = kSlrLanes / 2; d > 0; d >>= 1) part = dadd(part, __shfl_xor_sync(kFull, part, d));
-            if (l8 == 0 && o.b < o.e) s_rec[slot] = slr_reciprocal(part);
+            if (l8 == 0 && o.b < o.e) s_rec[slot] = reciprocal(part);
         }
         const bool mine = tid < o.q;
         double x = 0.0, inc = 0.0;
