@@ -398,6 +398,51 @@ __host__ __device__ inline uint32_t unbrick(uint32_t jb, const BrickDims& b) {
     const uint32_t z = bz * 8 + (((in >> 1) & 3u) | ((in >> 2) & 4u));
     return x + b.nx * (y + b.ny * z);
 }
+// Voxel order and bricked order side by side: a thread has one x and y and four layers
+// from z on; the pair of threads of an even x and the next has one sector, half each.
+// So both orders are read and written in whole sectors (a thread a voxel moves a sector
+// in four pieces of two entries).  A warp has 16 x and two y: 64 bytes together in
+// either order.
+struct BrickQuad {
+    uint32_t x, y, z, own;  // own: the entry of this thread's half of the sector
+    bool in;
+    __device__ __forceinline__ BrickQuad(uint64_t t, const BrickDims& b) {
+        const uint32_t nbx = (b.nx + 15) / 16, nby = (b.ny + 1) / 2;
+        const uint32_t w = static_cast<uint32_t>(t >> 5), lane = static_cast<uint32_t>(t) & 31u, r = w / nbx;
+        x = w % nbx * 16 + (lane & 15u);
+        y = r % nby * 2 + (lane >> 4);
+        z = r / nby * 4;
+        in = (x & ~1u) < b.nx && y < b.ny && z < b.nz;
+        own = in ? brick_xyz(x & ~1u, y, z, b) + (x & 1u) * 4 : 0u;
+    }
+    __device__ __forceinline__ bool voxel(int u, const BrickDims& b) const { return in && x < b.nx && z + u < b.nz; }
+    __device__ __forceinline__ uint32_t index(int u, const BrickDims& b) const { return x + b.nx * (y + b.ny * (z + u)); }
+};
+inline uint64_t brick_quads(const BrickDims& b) {  // threads, 32 a warp
+    return static_cast<uint64_t>((b.nx + 15) / 16) * ((b.ny + 1) / 2) * ((b.nz + 3) / 4) * 32;
+}
+// The halves of a pair's sector (x0 z0, x1 z0, x0 z1, x1 z1; the same of z2 and z3) to
+// each thread's four layers, and back.  Every thread of the warp takes part.
+template <typename R4, typename Real>
+__device__ __forceinline__ void quad_to_layers(const R4& half, Real (&v)[4]) {
+    const bool odd = threadIdx.x & 1u;
+    const Real a = __shfl_xor_sync(kFull, odd ? half.x : half.y, 1), b = __shfl_xor_sync(kFull, odd ? half.z : half.w, 1);
+    v[0] = odd ? a : half.x;
+    v[1] = odd ? b : half.z;
+    v[2] = odd ? half.y : a;
+    v[3] = odd ? half.w : b;
+}
+template <typename R4, typename Real>
+__device__ __forceinline__ R4 layers_to_quad(const Real (&v)[4]) {
+    const bool odd = threadIdx.x & 1u;
+    const Real a = __shfl_xor_sync(kFull, odd ? v[0] : v[2], 1), b = __shfl_xor_sync(kFull, odd ? v[1] : v[3], 1);
+    R4 half;
+    half.x = odd ? a : v[0];
+    half.y = odd ? v[2] : a;
+    half.z = odd ? b : v[1];
+    half.w = odd ? v[3] : b;
+    return half;
+}
 // voxel indices to bricked ones in place (indices >= V to ones >= brick_volume)
 void launch_brick_indices(uint32_t* vidx, uint64_t n, BrickDims b, uint32_t V, cudaStream_t s);
 // bricked indices back to voxel indices

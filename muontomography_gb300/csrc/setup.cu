@@ -585,9 +585,14 @@ __global__ void k_unbrick_indices(const uint32_t* __restrict__ in, uint32_t* __r
 }
 
 template <typename Real>
-__global__ void k_brick_lambda(const Real* __restrict__ lam, uint32_t V, BrickDims b, Real* __restrict__ lam_b) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < V) lam_b[brick_of(j, b)] = lam[j];
+__global__ void k_brick_lambda(const Real* __restrict__ lam, BrickDims b, Real* __restrict__ lam_b) {
+    using R4 = typename Vec4<Real>::type;
+    const BrickQuad q(static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x, b);
+    Real v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = q.voxel(u, b) ? lam[q.index(u, b)] : Real(0);
+    const R4 half = layers_to_quad<R4>(v);
+    if (q.in) *reinterpret_cast<R4*>(lam_b + q.own) = half;
 }
 
 }  // namespace
@@ -809,7 +814,7 @@ void launch_unbrick_indices(const uint32_t* in, uint32_t* out, uint64_t n, Brick
 template <typename Real>
 void launch_brick_lambda(const Real* lam, uint32_t V, BrickDims b, Real* lam_b, cudaStream_t s) {
     if (V == 0) return;
-    k_brick_lambda<Real><<<blocks_for(V), kThreads, 0, s>>>(lam, V, b, lam_b);
+    k_brick_lambda<Real><<<blocks_for(brick_quads(b)), kThreads, 0, s>>>(lam, b, lam_b);
     count_launches(1);
 }
 template void launch_brick_lambda<float>(const float*, uint32_t, BrickDims, float*, cudaStream_t);
