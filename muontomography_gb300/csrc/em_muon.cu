@@ -296,11 +296,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_em_muon(MuonPassArgs<Real> a, i
 // ---------------------------------------------------------------------------
 // WEIGHTS (FP64): the pairs hold W01 and W11 beside L, so a pair costs three
 // FP64 operations instead of eight.
-template <typename Real, int GROUP, bool WEIGHTS>
-__global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a, uint32_t n_muons, int batch) {
+// FULL: batches of 32 muons, a constant (with a variable, 580 us where it takes 526).
+template <typename Real, int GROUP, bool WEIGHTS, bool FULL>
+__global__ void __launch_bounds__(kThreads) k_em_muon_warp(MuonPassArgs<Real> a, uint32_t n_muons, int some) {
     using R4 = typename Vec4<Real>::type;
     constexpr int U = 5;                    // pair loads in flight per lane per round
     constexpr int kPer = 32 / GROUP;        // muons summed at once per warp
+    const int batch = FULL ? 32 : some;
     const int lane = threadIdx.x & 31;
     const int sub = lane / GROUP, glane = lane % GROUP;
     const unsigned gmask = GROUP == 32 ? kFull : (((1u << GROUP) - 1u) << (lane & ~(GROUP - 1)));
@@ -477,10 +479,10 @@ static int warp_blocks(int group) {
     int n = 0;
     cudaError_t e;
     if (sizeof(Real) == 8 && group <= 4)  // (4 lanes a muon: FP64 alone)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<double, 4, WEIGHTS>, kThreads, 0);
-    else if (group <= 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 8, WEIGHTS>, kThreads, 0);
-    else if (group <= 16) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 16, WEIGHTS>, kThreads, 0);
-    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 32, WEIGHTS>, kThreads, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<double, 4, WEIGHTS, true>, kThreads, 0);
+    else if (group <= 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 8, WEIGHTS, true>, kThreads, 0);
+    else if (group <= 16) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 16, WEIGHTS, true>, kThreads, 0);
+    else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_em_muon_warp<Real, 32, WEIGHTS, true>, kThreads, 0);
     return (e == cudaSuccess && n > 0) ? n : 1;
 }
 template <typename Real>
@@ -507,23 +509,27 @@ void launch_em_muon_warp(const MuonPassArgs<Real>& a, uint32_t n_muons, int bloc
     while (threads > 32 && batches <= static_cast<uint64_t>(num_sms) * (threads / 64)) threads /= 2;
     const uint64_t need = (batches + threads / 32 - 1) / (threads / 32);
     const unsigned nb = static_cast<unsigned>(need < static_cast<uint64_t>(blocks) ? need : blocks);
-    auto go = [&](auto w) {
-        constexpr bool W = decltype(w)::value;
+    auto go = [&](auto w, auto full) {
+        constexpr bool W = decltype(w)::value, F = decltype(full)::value;
         if constexpr (sizeof(Real) == 8) {
             if (group <= 4) {
-                k_em_muon_warp<Real, 4, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
+                k_em_muon_warp<Real, 4, W, F><<<nb, threads, 0, s>>>(a, n_muons, batch);
                 return;
             }
         }
-        if (group <= 8) k_em_muon_warp<Real, 8, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
-        else if (group <= 16) k_em_muon_warp<Real, 16, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
-        else k_em_muon_warp<Real, 32, W><<<nb, threads, 0, s>>>(a, n_muons, batch);
+        if (group <= 8) k_em_muon_warp<Real, 8, W, F><<<nb, threads, 0, s>>>(a, n_muons, batch);
+        else if (group <= 16) k_em_muon_warp<Real, 16, W, F><<<nb, threads, 0, s>>>(a, n_muons, batch);
+        else k_em_muon_warp<Real, 32, W, F><<<nb, threads, 0, s>>>(a, n_muons, batch);
+    };
+    auto choose = [&](auto w) {
+        if (batch == 32) go(w, std::true_type{});
+        else go(w, std::false_type{});
     };
     if constexpr (sizeof(Real) == 8) {
-        if (a.W11) go(std::true_type{});
-        else go(std::false_type{});
+        if (a.W11) choose(std::true_type{});
+        else choose(std::false_type{});
     } else {
-        go(std::false_type{});
+        choose(std::false_type{});
     }
     count_launches(1);
 }
