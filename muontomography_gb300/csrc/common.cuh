@@ -372,30 +372,33 @@ void launch_em_voxel(const VoxelPassArgs<Real, OutT>& a, const VoxDesc* const* l
 // 128 steps in z and 93 in x and y, so sectors and lines are longest in z.  A
 // warp instruction over 32 consecutive pairs of a path then touches 10.2 lines
 // and 15.9 sectors; with 4x4x2 lines of 2x2x2 sectors it was 12.8 and 16.5
-// (counted by ncu on the reductions of the 256 x 256 x 128 grid).
+// (counted by ncu on the reductions of the 256 x 256 x 128 grid).  Grids of up to four
+// layers have bricks half as high, 4x4x4: the others' upper halves would be padding.
 struct BrickDims {
-    uint32_t nx, ny, nz, nbx, nby, nbz;
+    uint32_t nx, ny, nz, nbx, nby, nbz, zb;  // a brick's layers: 2^zb
 };
 __host__ __device__ inline BrickDims brick_dims(const muto_grid& g) {
-    return BrickDims{g.nx, g.ny, g.nz, (g.nx + 3) / 4, (g.ny + 3) / 4, (g.nz + 7) / 8};
+    const uint32_t zb = g.nz > 4 ? 3 : 2;
+    return BrickDims{g.nx, g.ny, g.nz, (g.nx + 3) / 4, (g.ny + 3) / 4, (g.nz + 7) / 8, zb};
 }
 __host__ __device__ inline uint64_t brick_volume(const BrickDims& b) {
-    return static_cast<uint64_t>(b.nbx) * b.nby * b.nbz * 128;
+    return (static_cast<uint64_t>(b.nbx) * b.nby * b.nbz) << (4 + b.zb);
 }
 __host__ __device__ inline uint32_t brick_xyz(uint32_t x, uint32_t y, uint32_t z, const BrickDims& b) {
-    const uint32_t in = (x & 1u) | ((z & 3u) << 1) | ((y & 1u) << 3) | ((z & 4u) << 2) | ((x & 2u) << 4) | ((y & 2u) << 5);
-    return (((z >> 3) * b.nby + (y >> 2)) * b.nbx + (x >> 2)) * 128u + in;
+    const uint32_t in = (x & 1u) | ((z & 3u) << 1) | ((y & 1u) << 3) | ((z & 4u) << 2) |
+                        (((x & 2u) | ((y & 2u) << 1)) << (b.zb + 1));
+    return ((((z >> 3) * b.nby + (y >> 2)) * b.nbx + (x >> 2)) << (4 + b.zb)) + in;
 }
 __host__ __device__ inline uint32_t brick_of(uint32_t j, const BrickDims& b) {
     const uint32_t x = j % b.nx, t = j / b.nx, y = t % b.ny, z = t / b.ny;
     return brick_xyz(x, y, z, b);
 }
 __host__ __device__ inline uint32_t unbrick(uint32_t jb, const BrickDims& b) {
-    const uint32_t in = jb & 127u, blk = jb >> 7;
+    const uint32_t in = jb & ((16u << b.zb) - 1u), blk = jb >> (4 + b.zb), top = in >> (b.zb + 1);
     const uint32_t bx = blk % b.nbx, t = blk / b.nbx, by = t % b.nby, bz = t / b.nby;
-    const uint32_t x = bx * 4 + ((in & 1u) | ((in >> 4) & 2u));
-    const uint32_t y = by * 4 + (((in >> 3) & 1u) | ((in >> 5) & 2u));
-    const uint32_t z = bz * 8 + (((in >> 1) & 3u) | ((in >> 2) & 4u));
+    const uint32_t x = bx * 4 + ((in & 1u) | (top & 2u));
+    const uint32_t y = by * 4 + (((in >> 3) & 1u) | ((top >> 1) & 2u));
+    const uint32_t z = bz * 8 + (((in >> 1) & 3u) | (b.zb == 3 ? (in >> 2) & 4u : 0u));
     return x + b.nx * (y + b.ny * z);
 }
 // Voxel order and bricked order side by side: a thread has one x and y and four layers

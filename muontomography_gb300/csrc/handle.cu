@@ -1652,12 +1652,12 @@ void autotune_fused(muto_handle* h) {
         // muons; 51 / 37 at 16; 15 / 16 at 23).  Not where there are no more muons than
         // groups of 16 lanes at once, nor where so few voxels take the reductions that
         // more muons at once only collide (12^3 voxels: 234 / 238 / 262 us with 16 / 8 /
-        // 4 lanes; 32 x 32 x 8, 15 pairs: 211 / 158 / 159).
+        // 4 lanes; 32 x 32 x 8, 15 pairs: 211 / 158 / 159; 48 x 48 x 8: 210 / 146 / 144).
         const uint64_t entries = h->brick ? h->vb : h->V();
         h->fused_variant = kFusedOnce;
         h->once_group = avg <= 160.0 ? 16 : 32;
         if (h->N > static_cast<uint64_t>(em_once_muons16(h->num_sms))) {
-            if (avg <= 20.0 && entries >= 32768) h->once_group = 4;
+            if (avg <= 20.0 && entries >= 16384) h->once_group = 4;
             else if (avg <= 48.0 && entries >= 4096) h->once_group = 8;
         }
         // Where lambda and G together fill L2: a pass over the lists for each.  One pass /
