@@ -689,7 +689,11 @@ def run_ours(args) -> int:
             "config": {"workload": wl.name, "method": method_of(args), "grid": list(wl.grid.shape),
                        "voxel_mm": wl.grid.dx, "muons": n,
                        "kept_muons": kept, "pairs_per_iteration": pairs, "mode": args.mode,
-                       "precision": args.precision, "per_muon_2x2": "f64", "graph": True,
+                       "precision": args.precision,
+                       # (the mixed form's one-pass kernel, with fewer than 32 muons a warp's batch)
+                       "per_muon_2x2": ("double-float, 48 bits" if args.precision == "mixed" and st["muon_pass"] == 3
+                                        and st["tile_muons"] < 32 else "f64"),
+                       "graph": True,
                        "path_lists": {1: "voxel_major", 2: "muon_major", 3: "recompute"}.get(st["path_lists"]),
                        "parallelism": f"replicas x{world} (one scan per GPU)",
                        "l2": "inputs larger than L2: the pair lists read every iteration far exceed 126 MB, no flush",

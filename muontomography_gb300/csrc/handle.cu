@@ -1595,6 +1595,8 @@ std::map<TuneShape, int> g_fused_choice;  // the tuner's pick per scan shape (gu
 // together; and W01 (in place of T) and W11 of every pair, when W11's 8 bytes
 // beside the lists' 20 are at most a quarter of the memory that is left.  A pair
 // then costs three FP64 operations in either pass, not eight and seven.
+// (Without them a pair's weights are rounded otherwise: beside other work on the GPU
+// the same scan may come out a few units of the last place away.)
 // The FP64 passes a config may name (the TMA tile pass, a one-pass variant or
 // its prefetch) keep the lists as they are.
 bool fp64_passes(const muto_handle* h) {
