@@ -42,7 +42,10 @@ __global__ void k_exp_lambda(const double* __restrict__ loglam, const uint32_t* 
 // voxel's terms are gathered, not scattered with an FP64 reduction each, and a block
 // adds its value once.  96 x 96 x 48 voxels, 26 neighbours,
 // p = 2: 86 us (its FP64 operations alone take 75); 295 us with the terms scattered.
-constexpr int kPriorThreads = 256;
+// Blocks are as small as it takes for every SM to have one (down to a warp): a few
+// large ones leave the FP64 pipes of most SMs idle (16^3 voxels, p = 1.5: the objective
+// takes 184 us, 261 with 256 threads).
+constexpr int kPriorThreads = 256;  // at most
 template <int POWER>
 __global__ void __launch_bounds__(kPriorThreads) k_prior(const double* __restrict__ lam64,
                                                          const uint32_t* __restrict__ mult, DevGrid g, MapParams mp,
@@ -53,8 +56,8 @@ __global__ void __launch_bounds__(kPriorThreads) k_prior(const double* __restric
     const double w2 = 0.70710678118654752440, w3 = 0.57735026918962576451;  // 1/sqrt(2), 1/sqrt(3)
     const double scale = POWER == kMapTwo ? unit : 1.0;                     // of the differences summed below
     double v = 0.0;
-    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * kPriorThreads + threadIdx.x; i < V;
-         i += static_cast<uint64_t>(gridDim.x) * kPriorThreads) {
+    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < V;
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint32_t j = static_cast<uint32_t>(i);
         const uint32_t x = j % nxy % nx, y = j % nxy / nx, z = j / nxy;
         const uint32_t xs[3] = {0 < x ? x - 1 : 0, x, x < nx - 1 ? x + 1 : nx - 1};
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(kPriorThreads) k_prior(const double* __restric
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x < 32) {
-        v = warp_sum(threadIdx.x < kPriorThreads / 32 ? part[threadIdx.x] : 0.0);
+        v = warp_sum(threadIdx.x < blockDim.x / 32 ? part[threadIdx.x] : 0.0);
         if (threadIdx.x == 0) atomicAdd(value, v);
     }
 }
@@ -112,11 +115,14 @@ template void launch_exp_lambda<double>(const double*, const uint32_t*, uint32_t
 void launch_prior(const double* lam64, const uint32_t* mult, DevGrid g, MapParams mp, int num_sms, double* grad,
                   double* value, cudaStream_t s) {
     // blocks that loop, so that few add to the one value
-    const unsigned need = blocks_for(static_cast<uint64_t>(g.n[0]) * g.n[1] * g.n[2], kPriorThreads);
+    const uint64_t V = static_cast<uint64_t>(g.n[0]) * g.n[1] * g.n[2];
+    int threads = kPriorThreads;
+    while (threads > 32 && V < static_cast<uint64_t>(threads) * num_sms) threads /= 2;
+    const unsigned need = blocks_for(V, threads);
     const unsigned nb = need < 4u * num_sms ? need : 4u * num_sms;
-    if (mp.p == 2.0) k_prior<kMapTwo><<<nb, kPriorThreads, 0, s>>>(lam64, mult, g, mp, grad, value);
-    else if (mp.p == 1.0) k_prior<kMapOne><<<nb, kPriorThreads, 0, s>>>(lam64, mult, g, mp, grad, value);
-    else k_prior<kMapAny><<<nb, kPriorThreads, 0, s>>>(lam64, mult, g, mp, grad, value);
+    if (mp.p == 2.0) k_prior<kMapTwo><<<nb, threads, 0, s>>>(lam64, mult, g, mp, grad, value);
+    else if (mp.p == 1.0) k_prior<kMapOne><<<nb, threads, 0, s>>>(lam64, mult, g, mp, grad, value);
+    else k_prior<kMapAny><<<nb, threads, 0, s>>>(lam64, mult, g, mp, grad, value);
     count_launches(1);
 }
 
