@@ -387,7 +387,8 @@ using namespace muto;
 struct muto_handle {
     // first: the allocations below are freed on its stream
     struct Streams : HandleStreams {
-        ~Streams() { give(); }
+        bool forks = true;  // the one-shot methods never leave the main stream
+        ~Streams() { give(forks); }
     } streams;
     Method method = kMlsd;
     Params P;
@@ -2339,6 +2340,7 @@ int muto_create(const char* method, const char* config_json, muto_handle** out) 
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
         h->smem_optin = static_cast<size_t>(optin);
         CK(HandleStreams::take(h->device, &h->streams));
+        h->streams.forks = h->method != kPoca;
         h->stream = h->streams.stream;
         h->fan = h->streams.fan;
         static_assert(HandleStreams::kOverlap == muto_handle::kOverlapChunks + 1, "one event a chunk and one more");
